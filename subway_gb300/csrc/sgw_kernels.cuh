@@ -1504,9 +1504,97 @@ __global__ void __launch_bounds__(kRelaxThreads) k_relax_tile(RelaxArgs a) {
   relax_tile_phase<ALGO, ASYNC, W>(a, sm);
 }
 
+// Expansion of up to 32 sources by one warp, shared by the warp kernels.  Lane
+// i owns `d` edges that start at edge `boff` of the device buffer and carries
+// `val`.  The sources that have edges are packed by rank into shared memory,
+// and a bit per edge position marks where each one starts, kExpandSeg
+// positions at a time; lane i of a 32-edge window then finds its edge's owner
+// as (owners before the window) + (start bits up to its own) - 1: a broadcast
+// word, a popcount and one 8-byte shared load.  f(position in the buffer,
+// owner's value) is called for kRelaxUnroll edges of a lane at a time.
+//
+// What bounds the relaxation of a large frontier is instructions, not memory:
+// the earlier owner search (warp votes, __fns and three shuffles per window)
+// took most of them.  Relaxation per run, before and after: SSWP-async on
+// R-MAT of 1.3 M vertices and 16 M 8-byte records in memory 1.37 and 0.98 ms,
+// SSSP-async on R-MAT 2^25 (0.53 G edges, learned schedule) 14.9 and 12.4 ms.
+constexpr uint32_t kExpandSeg = 2048;
+template <class V>
+struct WarpExpand {
+  struct Own { uint32_t delta; V val; };
+  uint32_t bits[kExpandSeg / 32];
+  Own own[32];
+};
+
+template <class V, class F>
+__device__ __forceinline__ uint32_t warp_expand(WarpExpand<V> &s, int lane, uint32_t d, uint32_t boff, V val, F f) {
+  const uint32_t incl = warp_incl_scan(d, lane);
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+  if (total == 0) return 0;
+  const uint32_t excl = incl - d;
+  const bool own = d > 0;
+  const uint32_t owners = __ballot_sync(0xffffffffu, own);
+  const uint32_t le = lanemask_lt() | (1u << lane);
+  if (own) {
+    typename WarpExpand<V>::Own o;
+    o.delta = boff - excl;  // buffer position of edge j of the tile: delta + j (mod 2^32)
+    o.val = val;
+    s.own[__popc(owners & (le >> 1))] = o;
+  }
+  uint32_t base = 0xffffffffu;  // owners that start before the window, minus one
+  for (uint32_t seg = 0; seg < total; seg += kExpandSeg) {
+    __syncwarp();
+#pragma unroll
+    for (uint32_t w = 0; w < kExpandSeg / 32; w += 32) s.bits[w + lane] = 0;
+    __syncwarp();
+    if (own && excl - seg < kExpandSeg) atomicOr(&s.bits[(excl - seg) >> 5], 1u << ((excl - seg) & 31u));
+    __syncwarp();
+    const uint32_t end = min(total - seg, kExpandSeg);
+    for (uint32_t w0 = 0; w0 < end; w0 += 32u * kRelaxUnroll) {
+      uint32_t pos[kRelaxUnroll];
+      V sv[kRelaxUnroll];
+      bool ok[kRelaxUnroll];
+#pragma unroll
+      for (int q = 0; q < kRelaxUnroll; ++q) {
+        const uint32_t word = s.bits[w0 / 32u + q];
+        const uint32_t j = w0 + 32u * q + lane;
+        ok[q] = j < end;
+        const uint32_t r = base + __popc(word & le);
+        base += __popc(word);
+        if (ok[q]) {
+          const typename WarpExpand<V>::Own o = s.own[r];
+          pos[q] = o.delta + seg + j;
+          sv[q] = o.val;
+        }
+      }
+      f(pos, sv, ok);
+    }
+  }
+  __syncwarp();  // the tables are rewritten by the next tile
+  return total;
+}
+
+// Relaxes the kRelaxUnroll edges of a lane: all record loads, then all
+// destination values, then the compares and reductions.
+template <int ALGO, int W>
+__device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&pos)[kRelaxUnroll],
+                                           const uint32_t (&sv)[kRelaxUnroll], const bool (&ok)[kRelaxUnroll]) {
+  uint32_t dst[kRelaxUnroll], w[kRelaxUnroll], cur[kRelaxUnroll];
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w[q], a.wbuf);
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) cur[q] = a.value[dst[q]];
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) any |= relax_edge_seen<ALGO>(sv[q], dst[q], w[q], cur[q], a.value, a.nxt);
+  return any;
+}
+
 // Warp-tile form of k_relax_tile: each warp takes 32 partition sources at a
-// time and expands their edges on its own (warp scan of the degrees, each
-// edge's owner found with warp votes and shuffles, no shared memory), so
+// time and expands their edges on its own (warp_expand), so
 // warps never wait on each other: a warp that runs out of tiles adds its counters
 // to the CTA's in shared memory and leaves, and the last warp of the CTA to
 // leave publishes them.  Sources above tile_degree_max go to the chunk list
@@ -1517,21 +1605,26 @@ constexpr int kWarpsPerCta = kRelaxThreads / 32;
 #ifndef SGW_RELAX_MIN_BLOCKS
 #define SGW_RELAX_MIN_BLOCKS 4
 #endif
-template <int ALGO, bool ASYNC, int W>
-__global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_warp(RelaxArgs a) {
-  __shared__ int s_skip;
-  __shared__ unsigned long long s_edges, s_srcs;
-  __shared__ uint32_t s_any, s_done;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const uint32_t slot = a.iter & 3u;
-  if (tid == 0) {
+
+// Counters of a CTA whose warps finish independently.
+struct CtaTally {
+  unsigned long long edges, srcs;
+  uint32_t any, done;
+  int skip;
+};
+
+// Start of inner iteration a.iter: whether it runs at all, the next
+// iteration's counters cleared, the run counted.
+template <bool ASYNC, class Args>
+__device__ __forceinline__ bool iter_begin(const Args &a, CtaTally &t) {
+  if (threadIdx.x == 0) {
     int skip = 0;
     if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.iter - 1) & 3u]) == 0) skip = 1;
-    s_skip = skip;
-    s_edges = 0;
-    s_srcs = 0;
-    s_any = 0;
-    s_done = 0;
+    t.skip = skip;
+    t.edges = 0;
+    t.srcs = 0;
+    t.any = 0;
+    t.done = 0;
     if (blockIdx.x == 0) {
       a.ctl->upd[(a.iter + 1) & 3u] = 0;
       a.ctl->wl_count[(a.iter + 1) & 3u] = 0;
@@ -1542,7 +1635,34 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_w
     }
   }
   __syncthreads();
-  if (s_skip) return;
+  return !t.skip;
+}
+
+// End of a warp's share; the CTA's last warp publishes.
+__device__ __forceinline__ void warp_publish(CtaTally &t, Ctl *ctl, uint32_t slot, int lane, bool any,
+                                             unsigned long long edges, unsigned long long srcs) {
+  const bool warp_any = __any_sync(0xffffffffu, any);
+  if (lane == 0) {
+    if (edges) atomicAdd(&t.edges, edges);
+    if (srcs) atomicAdd(&t.srcs, srcs);
+    if (warp_any) atomicOr(&t.any, 1u);
+    __threadfence_block();
+    if (atomicAdd(&t.done, 1u) == kWarpsPerCta - 1) {
+      __threadfence_block();
+      if (t.any) atomicAdd(&ctl->upd[slot], 1u);
+      if (t.edges) atomicAdd(&ctl->relaxed_edges, t.edges);
+      if (t.srcs) atomicAdd(&ctl->relaxed_sources, t.srcs);
+    }
+  }
+}
+
+template <int ALGO, bool ASYNC, int W>
+__global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_warp(RelaxArgs a) {
+  __shared__ CtaTally s_tally;
+  __shared__ WarpExpand<uint32_t> s_exp[kWarpsPerCta];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const uint32_t slot = a.iter & 3u;
+  if (!iter_begin<ASYNC>(a, s_tally)) return;
   bool any_update = false;
   unsigned long long my_edges = 0, my_srcs = 0;
   const uint32_t ntiles = (a.size + 31u) / 32u;
@@ -1595,58 +1715,11 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_w
       my_edges += hd;
     }
     if (d > a.tile_degree_max) d = 0;
-    const uint32_t incl = warp_incl_scan(d, lane);
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    const uint32_t excl = incl - d;
-    const uint32_t owners = __ballot_sync(0xffffffffu, d > 0);  // lanes owning edges, in edge order
-    my_edges += total;
-    for (uint32_t w0 = 0; w0 < total; w0 += 32u * kRelaxUnroll) {
-      uint32_t dst[kRelaxUnroll], w[kRelaxUnroll], sv[kRelaxUnroll], cur[kRelaxUnroll];
-      bool ok[kRelaxUnroll];
-#pragma unroll
-      for (int q = 0; q < kRelaxUnroll; ++q) {
-        // window of 32 edges [wb, wb + 32), lane i takes edge wb + i; its
-        // owner is found with votes instead of a search: the owners whose
-        // range starts at or before wb, plus those starting inside the
-        // window up to edge wb + i, count the owner's rank among `owners`
-        const uint32_t wb = w0 + 32u * q;
-        const uint32_t j = wb + lane;
-        ok[q] = j < total;
-        const bool own = d > 0;
-        const uint32_t starts =
-            __reduce_or_sync(0xffffffffu, (own && excl > wb && excl < wb + 32u) ? (1u << (excl - wb)) : 0u);
-        const uint32_t before = __popc(__ballot_sync(0xffffffffu, own && excl <= wb));
-        const uint32_t rank = before + __popc(starts & ((2u << lane) - 1u)) - 1u;
-        const int k = __fns(owners, 0, (int)rank + 1);
-        const uint32_t kb = __shfl_sync(0xffffffffu, boff, k & 31);
-        const uint32_t ke = __shfl_sync(0xffffffffu, excl, k & 31);
-        const uint32_t kv = __shfl_sync(0xffffffffu, val, k & 31);
-        if (ok[q]) {
-          load_edge<W>(a.buf, kb + (j - ke), a.pbits, dst[q], w[q], a.wbuf);
-          sv[q] = kv;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kRelaxUnroll; ++q)
-        if (ok[q]) cur[q] = a.value[dst[q]];
-#pragma unroll
-      for (int q = 0; q < kRelaxUnroll; ++q)
-        if (ok[q]) any_update |= relax_edge_seen<ALGO>(sv[q], dst[q], w[q], cur[q], a.value, a.nxt);
-    }
+    my_edges += warp_expand(s_exp[wid], lane, d, boff, val,
+                            [&](const uint32_t (&pos)[kRelaxUnroll], const uint32_t (&sv)[kRelaxUnroll],
+                                const bool (&ok)[kRelaxUnroll]) { any_update |= relax_lane<ALGO, W>(a, pos, sv, ok); });
   }
-  const bool warp_any = __any_sync(0xffffffffu, any_update);
-  if (lane == 0) {
-    if (my_edges) atomicAdd(&s_edges, my_edges);
-    if (my_srcs) atomicAdd(&s_srcs, my_srcs);
-    if (warp_any) atomicOr(&s_any, 1u);
-    __threadfence_block();
-    if (atomicAdd(&s_done, 1u) == kWarpsPerCta - 1) {  // the CTA's last warp publishes
-      __threadfence_block();
-      if (s_any) atomicAdd(&a.ctl->upd[slot], 1u);
-      if (s_edges) atomicAdd(&a.ctl->relaxed_edges, s_edges);
-      if (s_srcs) atomicAdd(&a.ctl->relaxed_sources, s_srcs);
-    }
-  }
+  warp_publish(s_tally, a.ctl, slot, lane, any_update, my_edges, my_srcs);
 }
 
 // Chunk list of inner iteration `iter`: one warp per item.
