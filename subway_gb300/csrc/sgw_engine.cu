@@ -138,8 +138,15 @@ struct sgw_engine {
   bool initialized = false;
   uint32_t num_active = 0;
   uint64_t num_active_edges = 0;
+  uint32_t max_degree = 0;                 // largest degree in the queue
   uint32_t num_parts = 0;
   bool parts_valid = false;
+  // Async labels of the queued vertices (integer algorithms).  partial: only
+  // some queued vertices are labelled (the first generate queues every
+  // vertex, then only the source keeps its label); taken: the last generate
+  // cleared the labels of what it queued, so a partition processed before any
+  // other of its global iteration has none left to clear.
+  bool labels_partial = false, labels_taken = false;
   uint32_t gitr = 0;  // current global iteration (1-based once processing)
   sgw_run_stats stats{};
   bool trace_on = false;
@@ -609,7 +616,7 @@ int launch_generate(sgw_engine *e, int consume) {
       TRY(launch_select(e));
     }
   }
-  CK(cudaMemsetAsync(&e->d_ctl->num_seen, 0, sizeof(uint32_t), e->s_comp));
+  CK(cudaMemsetAsync(&e->d_ctl->max_degree, 0, sizeof(uint32_t), e->s_comp));
   size_t slot = 0;
   TRY(prof_begin(e, K_GENERATE, e->s_comp, &slot));
   if (e->fam == FAM_PR) k_generate_count<true><<<e->num_tiles, kGenThreads, 0, e->s_comp>>>(a);
@@ -624,6 +631,8 @@ int launch_generate(sgw_engine *e, int consume) {
   TRY(prof_end(e, e->s_comp, slot));
   e->stats.generate_launches += 1;
   e->parts_valid = false;
+  e->labels_partial = false;
+  e->labels_taken = consume != 0;
   return SGW_OK;
 }
 
@@ -647,6 +656,7 @@ int generate_and_plan(sgw_engine *e, int consume) {
   TRY(check_ctl_error(e));
   e->num_active = e->h_ctl->num_active;
   e->num_active_edges = e->h_ctl->num_active_edges;
+  e->max_degree = e->h_ctl->max_degree;
   e->num_parts = e->h_ctl->num_parts;
   if (e->num_parts > 0) {
     CK(cudaMemcpyAsync(e->h_parts, e->d_parts, sizeof(Part) * e->num_parts,
@@ -754,9 +764,12 @@ int gather_into(sgw_engine *e, const Part &q, uint32_t b, cudaStream_t s) {
   return SGW_OK;
 }
 
+// One inner iteration: with `all` (every queued source active, the first
+// pass) one launch cut by edges, else the label-driven warp kernel and, when
+// the queue holds a source above tile_degree_max, its chunk list.
 template <int ALGO, bool ASYNC, int W>
-int launch_relax_pair(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, uint8_t *cur,
-                      uint8_t *nxt) {
+int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, uint8_t *cur,
+                      uint8_t *nxt, bool all) {
   RelaxArgs a;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
@@ -778,29 +791,45 @@ int launch_relax_pair(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   a.stream_base = (uint32_t)e->cur_stream_base;  // with the low words of off: offsets mod 2^32
   a.off = e->d_off;
   a.wbuf = e->use_w ? e->d_wbuf[b] : nullptr;
+  if (all) {
+    const unsigned long long units = q.edge_count + (unsigned long long)kRelaxHeader * q.size;
+    const unsigned long long max_warps = (unsigned long long)e->num_sms * 8 * kWarpsPerCta;
+    const unsigned long long per = std::max<unsigned long long>(kRelaxMinUnits, (units + max_warps - 1) / max_warps);
+    const unsigned long long warps = (units + per - 1) / per;
+    k_relax_all<ALGO, W><<<(uint32_t)((warps + kWarpsPerCta - 1) / kWarpsPerCta), kRelaxThreads, 0, e->s_comp>>>(
+        a, units, per);
+    CK(cudaGetLastError());
+    e->stats.launches += 1;
+    e->stats.relax_launches += 1;
+    return SGW_OK;
+  }
   const uint32_t g1 = grid_for(e, q.size, kRelaxThreads);
   if (e->opts.flags & SGW_OPT_CTA_TILES) k_relax_tile<ALGO, ASYNC, W><<<g1, kRelaxThreads, 0, e->s_comp>>>(a);
   else k_relax_warp<ALGO, ASYNC, W><<<g1, kRelaxThreads, 0, e->s_comp>>>(a);
   CK(cudaGetLastError());
-  k_relax_chunks<ALGO, ASYNC, W><<<e->num_sms * 4, kRelaxThreads, 0, e->s_comp>>>(a);
-  CK(cudaGetLastError());
-  e->stats.launches += 2;
-  e->stats.relax_launches += 2;
+  e->stats.launches += 1;
+  e->stats.relax_launches += 1;
+  if (e->max_degree > e->opts.tile_degree_max) {
+    k_relax_chunks<ALGO, ASYNC, W><<<e->num_sms * 4, kRelaxThreads, 0, e->s_comp>>>(a);
+    CK(cudaGetLastError());
+    e->stats.launches += 1;
+    e->stats.relax_launches += 1;
+  }
   return SGW_OK;
 }
 
 template <int ALGO, int W>
 int relax_dispatch_w(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async,
-                     uint8_t *cur, uint8_t *nxt) {
-  if (async) return launch_relax_pair<ALGO, true, W>(e, q, b, iter, cur, nxt);
-  return launch_relax_pair<ALGO, false, W>(e, q, b, iter, cur, nxt);
+                     uint8_t *cur, uint8_t *nxt, bool all) {
+  if (async) return launch_relax_pass<ALGO, true, W>(e, q, b, iter, cur, nxt, all);
+  return launch_relax_pass<ALGO, false, W>(e, q, b, iter, cur, nxt, all);
 }
 
 template <int ALGO>
 int relax_dispatch(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async,
-                   uint8_t *cur, uint8_t *nxt) {
-  if (e->W == 1) return relax_dispatch_w<ALGO, 1>(e, q, b, iter, async, cur, nxt);
-  return relax_dispatch_w<ALGO, 2>(e, q, b, iter, async, cur, nxt);
+                   uint8_t *cur, uint8_t *nxt, bool all) {
+  if (e->W == 1) return relax_dispatch_w<ALGO, 1>(e, q, b, iter, async, cur, nxt, all);
+  return relax_dispatch_w<ALGO, 2>(e, q, b, iter, async, cur, nxt, all);
 }
 
 template <bool ASYNC, int W>
@@ -836,7 +865,7 @@ int launch_pr_pair(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   return SGW_OK;
 }
 
-int launch_relax(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async) {
+int launch_relax(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async, bool all) {
   if (e->params.algo == SGW_PR) {
     if (e->W == 1) return async ? launch_pr_pair<true, 1>(e, q, b, iter) : launch_pr_pair<false, 1>(e, q, b, iter);
     return async ? launch_pr_pair<true, 2>(e, q, b, iter) : launch_pr_pair<false, 2>(e, q, b, iter);
@@ -844,10 +873,10 @@ int launch_relax(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool a
   uint8_t *cur = e->d_l1, *nxt = e->d_l2;
   if (async && (iter % 2 == 0)) std::swap(cur, nxt);  // ping-pong (sssp-async.cu:108-109)
   switch (e->params.algo) {
-    case SGW_BFS: return relax_dispatch<SGW_BFS>(e, q, b, iter, async, cur, nxt);
-    case SGW_SSSP: return relax_dispatch<SGW_SSSP>(e, q, b, iter, async, cur, nxt);
-    case SGW_SSWP: return relax_dispatch<SGW_SSWP>(e, q, b, iter, async, cur, nxt);
-    case SGW_CC: return relax_dispatch<SGW_CC>(e, q, b, iter, async, cur, nxt);
+    case SGW_BFS: return relax_dispatch<SGW_BFS>(e, q, b, iter, async, cur, nxt, all);
+    case SGW_SSSP: return relax_dispatch<SGW_SSSP>(e, q, b, iter, async, cur, nxt, all);
+    case SGW_SSWP: return relax_dispatch<SGW_SSWP>(e, q, b, iter, async, cur, nxt, all);
+    case SGW_CC: return relax_dispatch<SGW_CC>(e, q, b, iter, async, cur, nxt, all);
     default: return fail(SGW_EINVAL, "algorithm %d not supported", e->params.algo);
   }
 }
@@ -871,8 +900,8 @@ int process_hub(sgw_engine *e, const Part &q, uint32_t b) {
   const bool pr = e->params.algo == SGW_PR;
   const uint32_t u = q.first_vertex;
   if (pr) k_pr_hub_claim<<<1, 1, 0, e->s_comp>>>(q.from, e->d_qpush, e->d_ctl);
-  else if (async) k_hub_claim<true><<<1, 1, 0, e->s_comp>>>(u, e->d_value, e->d_l1, e->d_l2, e->d_ctl);
-  else k_hub_claim<false><<<1, 1, 0, e->s_comp>>>(u, e->d_value, e->d_l1, e->d_l2, e->d_ctl);
+  else k_hub_claim<<<1, 1, 0, e->s_comp>>>(u, e->d_value, e->d_l1, e->d_l2, e->d_ctl,
+                                          !async ? 0 : e->labels_partial ? 1 : 2);
   CK(cudaGetLastError());
   const uint64_t deg = q.edge_count;
   const uint64_t hoff = np_at(e->g, u);
@@ -921,22 +950,32 @@ int process_hub(sgw_engine *e, const Part &q, uint32_t b) {
 // keeps the wait: letting the host run ahead put more gathers beside each
 // relaxation and made both slower (RMAT-24 SSSP-async: 12.2 against 17.0
 // GTEPS).
-int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool sync_always = true) {
+// first: no partition of this global iteration has been relaxed before.
+int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool first,
+                     bool sync_always = true) {
   const bool async = e->params.mode == SGW_ASYNC;
+  const bool tiles = (e->opts.flags & SGW_OPT_CTA_TILES) != 0;
+  const bool all = !tiles && !(async && e->labels_partial);  // the first pass relaxes every queued source
   // upd, wl_count, iters_run
   CK(cudaMemsetAsync(&e->d_ctl->upd[0], 0, sizeof(uint32_t) * 9, e->s_comp));
   if (!async) {
     size_t slot = 0;
     TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
-    TRY(launch_relax(e, q, b, 1, false));
+    TRY(launch_relax(e, q, b, 1, false, all));
     TRY(prof_end(e, e->s_comp, slot));
     if (iters_out) *iters_out = 1;
     return SGW_OK;
   }
   if (e->params.algo != SGW_PR) {  // PR carries no labels
-    k_mix<<<grid_for(e, q.size, 256), 256, 0, e->s_comp>>>(e->d_queue, q.from, q.size, e->d_l1, e->d_l2);
-    CK(cudaGetLastError());
-    e->stats.launches += 1;
+    if (!all) {
+      k_mix<<<grid_for(e, q.size, 256), 256, 0, e->s_comp>>>(e->d_queue, q.from, q.size, e->d_l1, e->d_l2);
+      CK(cudaGetLastError());
+      e->stats.launches += 1;
+    } else if (!(first && e->labels_taken)) {
+      k_claim<<<grid_for(e, q.size, 256), 256, 0, e->s_comp>>>(e->d_queue, q.from, q.size, e->d_l1, e->d_l2);
+      CK(cudaGetLastError());
+      e->stats.launches += 1;
+    }
   }
   uint32_t max_inner = e->params.max_inner ? e->params.max_inner : 0xffffffffu;
   if (e->range_inner_cap) max_inner = std::min(max_inner, e->range_inner_cap);
@@ -946,7 +985,7 @@ int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_o
     const uint32_t nb = std::min<uint32_t>(batch, max_inner - (iter - 1));
     size_t slot = 0;
     TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
-    for (uint32_t k = 0; k < nb; ++k, ++iter) TRY(launch_relax(e, q, b, iter, true));
+    for (uint32_t k = 0; k < nb; ++k, ++iter) TRY(launch_relax(e, q, b, iter, true, all && iter == 1));
     TRY(prof_end(e, e->s_comp, slot));
     const uint32_t last = iter - 1;
     if (!sync_always && last >= max_inner) {  // capped: nothing to decide on the host
@@ -976,7 +1015,9 @@ int validate_params(const sgw_engine *e, const sgw_run_params *p) {
   return SGW_OK;
 }
 
-int state_init(sgw_engine *e, const sgw_run_params *p) {
+// take_labels: every generate clears the labels of what it queues (the run
+// loop, which relaxes all of it); the step API's async generates keep them.
+int state_init(sgw_engine *e, const sgw_run_params *p, bool take_labels) {
   TRY(validate_params(e, p));
   CK(cudaSetDevice(e->device));
   e->params = *p;
@@ -1003,11 +1044,14 @@ int state_init(sgw_engine *e, const sgw_run_params *p) {
   CK(cudaMemsetAsync(e->d_ctl, 0, sizeof(Ctl), e->s_comp));
   e->stats.launches += 1;
   const bool async = p->mode == SGW_ASYNC;
-  if (e->policy == SGW_POLICY_LEARNED) TRY(generate_and_stats(e, async ? 0 : 1));
-  else TRY(generate_and_plan(e, async ? 0 : 1));
+  const int consume = !async || take_labels ? 1 : 0;
+  if (e->policy == SGW_POLICY_LEARNED) TRY(generate_and_stats(e, consume));
+  else TRY(generate_and_plan(e, consume));
   if (async && p->algo != SGW_CC && p->algo != SGW_PR) {
     k_async_reset<<<grid_for(e, e->n, 256), 256, 0, e->s_comp>>>(e->n, p->source, e->d_l1);
     CK(cudaGetLastError());
+    e->labels_taken = false;  // the source's label is set again
+    e->labels_partial = e->policy != SGW_POLICY_LEARNED || (e->opts.sched_flags & SGW_SCHED_KEEP_IDLE);
     e->stats.launches += 1;
   }
   e->initialized = true;
@@ -1029,7 +1073,7 @@ int process_iteration(sgw_engine *e) {
       TRY(process_hub(e, q, b));
     } else {
       CK(cudaStreamWaitEvent(e->s_comp, e->ev_ready[b], 0));
-      TRY(process_resident(e, q, b, &inner));
+      TRY(process_resident(e, q, b, &inner, p == 0));
     }
     CK(cudaEventRecord(e->ev_free[b], e->s_comp));
     trace_partition(e, p, inner);
@@ -1059,6 +1103,7 @@ int generate_and_stats(sgw_engine *e, int consume) {
   TRY(check_ctl_error(e));
   e->num_active = e->h_ctl->num_active;
   e->num_active_edges = e->h_ctl->num_active_edges;
+  e->max_degree = e->h_ctl->max_degree;
   e->stats.d2h_bytes += sizeof(Ctl) + sizeof(RangeStat) * S;
   e->parts_valid = false;
   return SGW_OK;
@@ -1243,7 +1288,7 @@ int process_iteration_ranges(sgw_engine *e) {
       for (uint32_t s = j.s; s < j.s_end; ++s) pred = std::max(pred, e->h_rstat[s].pred);
       const bool cappable = kept || (e->opts.sched_flags & SGW_SCHED_CAP_COMPACT);
       e->range_inner_cap = cappable && (double)pred >= thr ? (e->opts.sched_inner ? e->opts.sched_inner : 3u) : 0u;
-      const int st = process_resident(e, q, (uint32_t)j.buf, &inner);
+      const int st = process_resident(e, q, (uint32_t)j.buf, &inner, k == 0);
       e->cur_streamed = 0;
       e->range_inner_cap = 0;
       TRY(st);
@@ -1659,7 +1704,7 @@ int sgw_engine_device_bytes(const sgw_engine *e, uint64_t *bytes) {
 int sgw_state_init(sgw_engine *e, const sgw_run_params *p) {
   clear_error();
   if (!e) return fail(SGW_EINVAL, "null engine");
-  return state_init(e, p);
+  return state_init(e, p, false);
 }
 
 int sgw_generate(sgw_engine *e, uint32_t *num_active_nodes, uint64_t *num_active_edges) {
@@ -1670,6 +1715,7 @@ int sgw_generate(sgw_engine *e, uint32_t *num_active_nodes, uint64_t *num_active
   TRY(read_ctl(e));
   e->num_active = e->h_ctl->num_active;
   e->num_active_edges = e->h_ctl->num_active_edges;
+  e->max_degree = e->h_ctl->max_degree;
   if (num_active_nodes) *num_active_nodes = e->num_active;
   if (num_active_edges) *num_active_edges = e->num_active_edges;
   return SGW_OK;
@@ -1714,7 +1760,7 @@ int sgw_process_partition(sgw_engine *e, uint32_t i, uint32_t *inner_iterations)
     TRY(process_hub(e, q, 0));
   } else {
     TRY(enqueue_gather(e, i, e->s_comp));
-    TRY(process_resident(e, q, i % e->nbuf, &iters));
+    TRY(process_resident(e, q, i % e->nbuf, &iters, false));
   }
   CK(cudaStreamSynchronize(e->s_comp));
   TRY(read_ctl(e));
@@ -1853,8 +1899,9 @@ int sgw_get_stats(const sgw_engine *e, sgw_run_stats *stats) {
 int sgw_run(sgw_engine *e, const sgw_run_params *p, void *out_values, sgw_run_stats *stats) {
   clear_error();
   if (!e) return fail(SGW_EINVAL, "null engine");
-  TRY(state_init(e, p));
-  const bool async = p->mode == SGW_ASYNC;
+  // the label-driven CTA-tile form needs the labels of an async queue
+  const bool take = !p || p->mode == SGW_SYNC || !(e->opts.flags & SGW_OPT_CTA_TILES);
+  TRY(state_init(e, p, take));
   CK(cudaEventRecord(e->ev_t0, e->s_comp));  // "timer.Start()" after the first generate
   uint32_t gitr = 0;
   while (e->num_active > 0) {
@@ -1864,10 +1911,10 @@ int sgw_run(sgw_engine *e, const sgw_run_params *p, void *out_values, sgw_run_st
     e->stats.active_edges += e->num_active_edges;
     if (e->policy == SGW_POLICY_LEARNED) {
       TRY(process_iteration_ranges(e));
-      TRY(generate_and_stats(e, async ? 0 : 1));
+      TRY(generate_and_stats(e, take ? 1 : 0));
     } else {
       TRY(process_iteration(e));
-      TRY(generate_and_plan(e, async ? 0 : 1));
+      TRY(generate_and_plan(e, take ? 1 : 0));
     }
   }
   CK(cudaEventRecord(e->ev_t1, e->s_comp));
