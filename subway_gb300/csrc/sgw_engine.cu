@@ -441,7 +441,7 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
   L.parts = take(sizeof(Part) * (size_t)L.max_parts);
   L.ranges = take(sizeof(RangeInfo) * (size_t)L.max_parts);
   L.rstat = take(sizeof(RangeStat) * (size_t)L.max_parts);
-  L.wl = take(16ull * (size_t)L.wl_cap);  // WorkItem and PrItem are 16 B
+  L.wl = take(sizeof(WorkItem) * (size_t)L.wl_cap);
   for (uint32_t b = 0; b < kMaxBuf; ++b) L.buf[b] = b < nbuf ? take(cap * esz) : L.buf[0];
   L.total = p;
   return L;
@@ -764,6 +764,21 @@ int gather_into(sgw_engine *e, const Part &q, uint32_t b, cudaStream_t s) {
   return SGW_OK;
 }
 
+// Equal shares of a partition's edges for the warps of a first pass.
+struct WarpCut {
+  unsigned long long units, per_warp;
+  uint32_t grid;
+};
+WarpCut cut_warps(const sgw_engine *e, const Part &q) {
+  WarpCut c;
+  c.units = q.edge_count + (unsigned long long)kRelaxHeader * q.size;
+  const unsigned long long max_warps = (unsigned long long)e->num_sms * 8 * kWarpsPerCta;
+  c.per_warp = std::max<unsigned long long>(kRelaxMinUnits, (c.units + max_warps - 1) / max_warps);
+  const unsigned long long warps = (c.units + c.per_warp - 1) / c.per_warp;
+  c.grid = (uint32_t)((warps + kWarpsPerCta - 1) / kWarpsPerCta);
+  return c;
+}
+
 // One inner iteration: with `all` (every queued source active, the first
 // pass) one launch cut by edges, else the label-driven warp kernel and, when
 // the queue holds a source above tile_degree_max, its chunk list.
@@ -792,12 +807,8 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   a.off = e->d_off;
   a.wbuf = e->use_w ? e->d_wbuf[b] : nullptr;
   if (all) {
-    const unsigned long long units = q.edge_count + (unsigned long long)kRelaxHeader * q.size;
-    const unsigned long long max_warps = (unsigned long long)e->num_sms * 8 * kWarpsPerCta;
-    const unsigned long long per = std::max<unsigned long long>(kRelaxMinUnits, (units + max_warps - 1) / max_warps);
-    const unsigned long long warps = (units + per - 1) / per;
-    k_relax_all<ALGO, W><<<(uint32_t)((warps + kWarpsPerCta - 1) / kWarpsPerCta), kRelaxThreads, 0, e->s_comp>>>(
-        a, units, per);
+    const WarpCut c = cut_warps(e, q);
+    k_relax_all<ALGO, W><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
     CK(cudaGetLastError());
     e->stats.launches += 1;
     e->stats.relax_launches += 1;
@@ -832,8 +843,10 @@ int relax_dispatch(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool
   return relax_dispatch_w<ALGO, 2>(e, q, b, iter, async, cur, nxt, all);
 }
 
-template <bool ASYNC, int W>
-int launch_pr_pair(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
+// One PageRank inner iteration: the first pushes the generate step's snapshot
+// (every queued source), later async ones what has grown above acc again.
+template <int W>
+int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   PrArgs a;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
@@ -842,33 +855,33 @@ int launch_pr_pair(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   a.delta = e->d_delta;
   a.qpush = e->d_qpush;
   a.ctl = e->d_ctl;
-  a.wl = reinterpret_cast<PrItem *>(e->d_wl);
-  a.wl_cap = e->wl_cap;
   a.from = q.from;
   a.size = q.size;
   a.edge_from = q.edge_from;
   a.iter = iter;
-  a.tile_degree_max = e->opts.tile_degree_max;
-  a.chunk_edges = e->opts.chunk_edges;
   a.pbits = e->pbits;
   a.streamed = e->cur_streamed;
   a.stream_base = (uint32_t)e->cur_stream_base;  // with the low words of off: offsets mod 2^32
   a.off = e->d_off;
   a.acc = (double)e->params.pr_acc;
   a.damping = (double)e->params.pr_damping;
-  k_pr_tile<ASYNC, W><<<grid_for(e, q.size, kRelaxThreads), kRelaxThreads, 0, e->s_comp>>>(a);
+  if (iter > 1) {
+    k_pr_claim<<<grid_for(e, q.size, kRelaxThreads), kRelaxThreads, 0, e->s_comp>>>(a);
+    CK(cudaGetLastError());
+    e->stats.launches += 1;
+    e->stats.relax_launches += 1;
+  }
+  const WarpCut c = cut_warps(e, q);
+  k_pr_all<W><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
   CK(cudaGetLastError());
-  k_pr_chunks<ASYNC, W><<<e->num_sms * 4, kRelaxThreads, 0, e->s_comp>>>(a);
-  CK(cudaGetLastError());
-  e->stats.launches += 2;
-  e->stats.relax_launches += 2;
+  e->stats.launches += 1;
+  e->stats.relax_launches += 1;
   return SGW_OK;
 }
 
 int launch_relax(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async, bool all) {
   if (e->params.algo == SGW_PR) {
-    if (e->W == 1) return async ? launch_pr_pair<true, 1>(e, q, b, iter) : launch_pr_pair<false, 1>(e, q, b, iter);
-    return async ? launch_pr_pair<true, 2>(e, q, b, iter) : launch_pr_pair<false, 2>(e, q, b, iter);
+    return e->W == 1 ? launch_pr_pass<1>(e, q, b, iter) : launch_pr_pass<2>(e, q, b, iter);
   }
   uint8_t *cur = e->d_l1, *nxt = e->d_l2;
   if (async && (iter % 2 == 0)) std::swap(cur, nxt);  // ping-pong (sssp-async.cu:108-109)

@@ -1944,26 +1944,16 @@ __global__ void k_reached(uint32_t n, int algo, uint32_t source, const uint32_t 
 // ---- PageRank (pr_kernel / pr_async, shared/gpu_kernels.cu:211-254, :459-502) --
 // Ranks and residuals are kept in double precision on the device; the
 // reference's float results are the final cast.
-struct PrItem {              // a chunk of one high-degree source's pushes
-  uint32_t boff;
-  uint32_t count;
-  double push;
-};
-
 struct PrArgs {
   const uint32_t *queue;
   const uint32_t *ptr;
   const uint32_t *buf;       // device edge buffer (W words per edge)
   double *pval;
   double *delta;
-  const double *qpush;       // pushes snapshotted by the generate step
+  double *qpush;             // push of each queued source (0: none this iteration)
   Ctl *ctl;
-  PrItem *wl;
-  uint32_t wl_cap;
   uint32_t from, size, edge_from;
   uint32_t iter;
-  uint32_t tile_degree_max;
-  uint32_t chunk_edges;
   uint32_t pbits;
   uint32_t streamed;
   uint32_t stream_base;
@@ -1978,150 +1968,98 @@ __device__ __forceinline__ double ld_relaxed_f64(const double *p) {
   return v;
 }
 
-// Same tiling as k_relax_tile.  Inner iteration 1 pushes the snapshot taken
-// by the generate step (every queued source is active); async iterations > 1
-// re-activate partition sources whose residual grew above acc
-// (value += delta; delta -= delta, atomically against concurrent pushes).
-template <bool ASYNC, int W>
-__global__ void __launch_bounds__(kRelaxThreads) k_pr_tile(PrArgs a) {
-  __shared__ uint32_t s_scan[kRelaxThreads + 1];
-  __shared__ uint32_t s_boff[kRelaxThreads];
-  __shared__ double s_push[kRelaxThreads];
-  __shared__ uint32_t s_hub[kRelaxThreads];
-  __shared__ uint32_t s_wsum[kRelaxThreads / 32];
-  __shared__ uint32_t s_nhub, s_wbase;
-  __shared__ int s_skip;
-  const int tid = threadIdx.x;
-  const uint32_t slot = a.iter & 3u;
-  if (tid == 0) {
-    int skip = 0;
-    if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.iter - 1) & 3u]) == 0) skip = 1;
-    s_skip = skip;
-    if (blockIdx.x == 0) {
-      a.ctl->upd[(a.iter + 1) & 3u] = 0;
-      a.ctl->wl_count[(a.iter + 1) & 3u] = 0;
-      if (!skip) {
-        atomicAdd(&a.ctl->iters_run, 1u);
-        atomicAdd(&a.ctl->iters_total, 1u);
-      }
-    }
-  }
-  __syncthreads();
-  if (s_skip) return;
-  bool any_push = false;
-  const uint32_t ntiles = (a.size + kRelaxThreads - 1) / kRelaxThreads;
-  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    if (tid == 0) s_nhub = 0;
-    __syncthreads();
-    const uint32_t i = a.from + t * kRelaxThreads + tid;
-    uint32_t d = 0, boff = 0;
-    double push = 0.0;
-    if (i < a.from + a.size) {
-      const uint32_t p0 = a.ptr[i];
-      const uint32_t deg = a.ptr[i + 1] - p0;
-      bool act;
-      if (!ASYNC || a.iter == 1) {
-        push = a.qpush[i];
-        act = true;
-      } else {
-        const uint32_t u = a.queue[i];
-        const double res = ld_relaxed_f64(&a.delta[u]);
-        act = res > a.acc;
-        if (act) {
-          a.pval[u] += res;
-          atomicAdd(&a.delta[u], -res);
-          push = a.damping * res / (double)deg;
-        }
-      }
-      if (act) {
-        any_push = true;
-        d = deg;
-        boff = a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from;
-        if (d > a.tile_degree_max) {
-          s_hub[atomicAdd(&s_nhub, 1u)] = tid;
-          atomicAdd(&a.ctl->relaxed_edges, (unsigned long long)d);
-        }
-      }
-    }
-    s_boff[tid] = boff;
-    s_push[tid] = push;
-    {
-      const int nsrc = __syncthreads_count(d > 0);
-      if (tid == 0 && nsrc) atomicAdd(&a.ctl->relaxed_sources, (unsigned long long)nsrc);
-    }
-    const uint32_t nhub = s_nhub;
-    for (uint32_t h = 0; h < nhub; ++h) {
-      const uint32_t ht = s_hub[h];
-      if (tid == ht) {
-        s_wbase = atomicAdd(&a.ctl->wl_count[slot], (d + a.chunk_edges - 1) / a.chunk_edges);
-        s_scan[kRelaxThreads] = d;
-      }
-      __syncthreads();
-      const uint32_t hd = s_scan[kRelaxThreads];
-      const uint32_t nch = (hd + a.chunk_edges - 1) / a.chunk_edges;
-      const uint32_t wb = s_wbase;
-      for (uint32_t c = tid; c < nch; c += blockDim.x) {
-        if (wb + c < a.wl_cap) {
-          PrItem it;
-          it.boff = s_boff[ht] + c * a.chunk_edges;
-          it.count = min(a.chunk_edges, hd - c * a.chunk_edges);
-          it.push = s_push[ht];
-          a.wl[wb + c] = it;
-        } else {
-          atomicExch(&a.ctl->error, 3u);
-        }
-      }
-      __syncthreads();
-    }
-    if (d > a.tile_degree_max) d = 0;
-    {
-      const int lane = tid & 31, warp = tid >> 5;
-      const uint32_t incl = warp_incl_scan(d, lane);
-      if (lane == 31) s_wsum[warp] = incl;
-      __syncthreads();
-      if (tid == 0) {
-        uint32_t acc = 0;
-        for (int w = 0; w < kRelaxThreads / 32; ++w) { uint32_t x = s_wsum[w]; s_wsum[w] = acc; acc += x; }
-        s_scan[kRelaxThreads] = acc;
-      }
-      __syncthreads();
-      s_scan[tid] = s_wsum[warp] + incl - d;
-      __syncthreads();
-    }
-    const uint32_t total = s_scan[kRelaxThreads];
-    if (tid == 0 && total) atomicAdd(&a.ctl->relaxed_edges, (unsigned long long)total);
-    for (uint32_t j = tid; j < total; j += blockDim.x) {
-      uint32_t lo = 0, hi = kRelaxThreads;
-      while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (s_scan[mid] <= j) lo = mid + 1; else hi = mid;
-      }
-      const uint32_t k = lo - 1;
-      uint32_t dst, w;
-      load_edge<W>(a.buf, s_boff[k] + (j - s_scan[k]), a.pbits, dst, w);
-      atomicAdd(&a.delta[dst], s_push[k]);
-    }
-    __syncthreads();
-  }
-  if (__syncthreads_or(any_push) && tid == 0) atomicAdd(&a.ctl->upd[slot], 1u);
+// Adds each edge's push to its destination's residual: the records of
+// kRelaxUnroll edges of a lane are loaded before their (non-returning) adds.
+template <int W>
+__device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[kRelaxUnroll],
+                                        const double (&push)[kRelaxUnroll], const bool (&ok)[kRelaxUnroll]) {
+  uint32_t dst[kRelaxUnroll], w;
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w);
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) atomicAdd(&a.delta[dst[q]], push[q]);
 }
 
-template <bool ASYNC, int W>
-__global__ void __launch_bounds__(kRelaxThreads) k_pr_chunks(PrArgs a) {
+// Pushes of one inner iteration, the work cut by edges as in k_relax_all:
+// source i pushes qpush[i], which the generate step (first iteration, every
+// queued source) or k_pr_claim (later async ones; 0 for the sources that are
+// not active again) has written.  PageRank's later rounds queue a few tens of
+// thousands of long rows, which left most of the chip idle when each CTA took
+// 256 of them and found its edges' owners by binary search.
+template <int W>
+__global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(PrArgs a, unsigned long long units,
+                                                                               unsigned long long per_warp) {
+  __shared__ CtaTally s_tally;
+  __shared__ WarpExpand<double> s_exp[kWarpsPerCta];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t slot = a.iter & 3u;
-  if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.iter - 1) & 3u]) == 0) return;
-  const uint32_t items = min(ld_acquire_u32(&a.ctl->wl_count[slot]), a.wl_cap);
-  const int lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t it = gw; it < items; it += nw) {
-    const PrItem wi = a.wl[it];
-    for (uint32_t j = lane; j < wi.count; j += 32) {
-      uint32_t dst, w;
-      load_edge<W>(a.buf, wi.boff + j, a.pbits, dst, w);
-      atomicAdd(&a.delta[dst], wi.push);
+  if (a.iter > 1) {  // k_pr_claim began the iteration and counted its sources
+    if (ld_acquire_u32(&a.ctl->upd[slot]) == 0) return;
+    if (threadIdx.x == 0) s_tally = CtaTally{};
+    __syncthreads();
+  } else {
+    iter_begin<false>(a, s_tally);
+  }
+  unsigned long long my_edges = 0, my_srcs = 0;
+  const unsigned long long t0 = per_warp * (blockIdx.x * kWarpsPerCta + wid);
+  const unsigned long long t1 = min(units, t0 + per_warp);
+  if (t0 < t1) {
+    const uint32_t first = warp_find_unit<kRelaxHeader>(a.ptr, a.from, a.size, a.edge_from, t0, lane);
+    for (uint32_t i0 = first; i0 < a.size; i0 += 32) {
+      const uint32_t idx = i0 + lane;
+      uint32_t d = 0, boff = 0;
+      double push = 0.0;
+      bool past = true, head = false;
+      if (idx < a.size) {
+        const uint32_t i = a.from + idx;
+        const uint32_t p0 = a.ptr[i], p1 = a.ptr[i + 1];
+        push = a.qpush[i];
+        const unsigned long long start = (unsigned long long)(p0 - a.edge_from) + (unsigned long long)kRelaxHeader * idx;
+        past = start >= t1;
+        uint32_t lo;
+        d = unit_clip<kRelaxHeader>(start, p1 - p0, t0, t1, &lo, &head);
+        if (push == 0.0) d = 0;
+        if (d) boff = (a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from) + lo;
+      }
+      if (a.iter == 1) my_srcs += __popc(__ballot_sync(0xffffffffu, head));
+      my_edges += warp_expand(s_exp[wid], lane, d, boff, push,
+                              [&](const uint32_t (&pos)[kRelaxUnroll], const double (&pv)[kRelaxUnroll],
+                                  const bool (&ok)[kRelaxUnroll]) { pr_lane<W>(a, pos, pv, ok); });
+      if (__any_sync(0xffffffffu, past)) break;
     }
   }
+  warp_publish(s_tally, a.ctl, slot, lane, my_srcs != 0, my_edges, my_srcs);
+}
+
+// Async inner iterations > 1: the partition's sources whose residual grew
+// above acc are active again (value += delta; delta -= delta, atomically
+// against pushes still to come); their pushes go to qpush.
+__global__ void __launch_bounds__(kRelaxThreads) k_pr_claim(PrArgs a) {
+  __shared__ CtaTally s_tally;
+  const int lane = threadIdx.x & 31;
+  if (!iter_begin<true>(a, s_tally)) return;
+  uint32_t srcs = 0;
+  for (uint32_t i0 = (blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5)) * 32u; i0 < a.size;
+       i0 += gridDim.x * kRelaxThreads) {
+    const uint32_t i = a.from + i0 + lane;
+    bool act = false;
+    if (i0 + lane < a.size) {
+      const uint32_t u = a.queue[i];
+      const double res = ld_relaxed_f64(&a.delta[u]);
+      double push = 0.0;
+      act = res > a.acc;
+      if (act) {
+        a.pval[u] += res;
+        atomicAdd(&a.delta[u], -res);
+        push = a.damping * res / (double)(a.ptr[i + 1] - a.ptr[i]);
+      }
+      a.qpush[i] = push;
+    }
+    srcs += __popc(__ballot_sync(0xffffffffu, act));
+  }
+  warp_publish(s_tally, a.ctl, a.iter & 3u, lane, srcs != 0, 0, srcs);
 }
 
 // Single-vertex PR partition: the generate snapshot of its push.
