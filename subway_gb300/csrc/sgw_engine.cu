@@ -764,6 +764,14 @@ int gather_into(sgw_engine *e, const Part &q, uint32_t b, cudaStream_t s) {
   return SGW_OK;
 }
 
+// In place of an edge buffer: the pass reads the host copy itself.
+constexpr uint32_t kFromHost = 0xffffffffu;
+
+HostEdges host_edges(const sgw_engine *e) {
+  return HostEdges{HostChunks{e->d_hct, e->hs_ends.shift}, HostChunks{e->d_hct + kMaxHostChunks, e->hs_w.shift},
+                   e->use_w ? 1u : 0u};
+}
+
 // Equal shares of a partition's edges for the warps of a first pass.
 struct WarpCut {
   unsigned long long units, per_warp;
@@ -788,7 +796,7 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   RelaxArgs a;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
-  a.buf = e->d_buf[b];
+  a.buf = b == kFromHost ? nullptr : e->d_buf[b];
   a.value = e->d_value;
   a.cur = cur;
   a.nxt = nxt;
@@ -805,10 +813,12 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   a.streamed = e->cur_streamed;
   a.stream_base = (uint32_t)e->cur_stream_base;  // with the low words of off: offsets mod 2^32
   a.off = e->d_off;
-  a.wbuf = e->use_w ? e->d_wbuf[b] : nullptr;
+  a.wbuf = e->use_w && b != kFromHost ? e->d_wbuf[b] : nullptr;
+  a.host = host_edges(e);
   if (all) {
     const WarpCut c = cut_warps(e, q);
-    k_relax_all<ALGO, W><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
+    if (b == kFromHost) k_relax_all<ALGO, W, true><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
+    else k_relax_all<ALGO, W, false><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
     CK(cudaGetLastError());
     e->stats.launches += 1;
     e->stats.relax_launches += 1;
@@ -850,7 +860,7 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   PrArgs a;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
-  a.buf = e->d_buf[b];
+  a.buf = b == kFromHost ? nullptr : e->d_buf[b];
   a.pval = e->d_pval;
   a.delta = e->d_delta;
   a.qpush = e->d_qpush;
@@ -865,6 +875,7 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   a.off = e->d_off;
   a.acc = (double)e->params.pr_acc;
   a.damping = (double)e->params.pr_damping;
+  a.host = host_edges(e);
   if (iter > 1) {
     k_pr_claim<<<grid_for(e, q.size, kRelaxThreads), kRelaxThreads, 0, e->s_comp>>>(a);
     CK(cudaGetLastError());
@@ -872,7 +883,8 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
     e->stats.relax_launches += 1;
   }
   const WarpCut c = cut_warps(e, q);
-  k_pr_all<W><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
+  if (b == kFromHost) k_pr_all<W, true><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
+  else k_pr_all<W, false><<<c.grid, kRelaxThreads, 0, e->s_comp>>>(a, c.units, c.per_warp);
   CK(cudaGetLastError());
   e->stats.launches += 1;
   e->stats.relax_launches += 1;
@@ -1013,6 +1025,26 @@ int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_o
   return SGW_OK;
 }
 
+// Whether a sync pass reads the host copy itself instead of a gathered
+// buffer.  Each partition of a sync iteration is relaxed once, so gathering
+// it first only adds a trip through HBM and, for the first partition, the wait
+// for it.  Host positions are 32-bit there: graphs with u64 node pointers
+// gather, and so do the forms that ask for the gather or for CTA tiles.
+bool sync_from_host(const sgw_engine *e) {
+  return e->params.mode == SGW_SYNC && !e->wide && !e->hs_ends.h.empty() &&
+         !(e->opts.flags & (SGW_OPT_SCALAR_GATHER | SGW_OPT_CTA_TILES | SGW_OPT_NO_OVERLAP));
+}
+
+// One sync pass over partition q, its records read over the host link.
+int process_from_host(sgw_engine *e, const Part &q) {
+  size_t slot = 0;
+  TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
+  TRY(launch_relax(e, q, kFromHost, 1, false, true));
+  TRY(prof_end(e, e->s_comp, slot));
+  e->stats.h2d_bytes += q.edge_count * (4ull * e->W + (e->use_w ? 1 : 0));
+  return SGW_OK;
+}
+
 int validate_params(const sgw_engine *e, const sgw_run_params *p) {
   if (!p) return fail(SGW_EINVAL, "null params");
   if (p->algo < SGW_BFS || p->algo > SGW_PR) return fail(SGW_EINVAL, "bad algorithm %d", p->algo);
@@ -1076,6 +1108,18 @@ int state_init(sgw_engine *e, const sgw_run_params *p, bool take_labels) {
 int process_iteration(sgw_engine *e) {
   const uint32_t P = e->num_parts;
   if (P == 0) return SGW_OK;
+  if (sync_from_host(e)) {
+    // one launch per partition: what the first ones improve reaches the later
+    // ones in the same iteration (one launch for all took CC a fifth round)
+    for (uint32_t p = 0; p < P; ++p) {
+      const Part &q = e->h_parts[p];
+      if (is_hub(e, q)) TRY(process_hub(e, q, 0));
+      else TRY(process_from_host(e, q));
+      trace_partition(e, p, 1);
+      e->stats.partitions += 1;
+    }
+    return SGW_OK;
+  }
   TRY(enqueue_gather(e, 0, e->s_copy));
   for (uint32_t p = 0; p < P; ++p) {
     const Part &q = e->h_parts[p];
@@ -1264,16 +1308,22 @@ int process_iteration_ranges(sgw_engine *e) {
     return best;
   };
   std::vector<uint32_t> inner_of(S, 0);
+  // jobs that need no buffer before they run: split vertices, and compacted
+  // sync jobs, which read the host copy themselves
+  const bool from_host = sync_from_host(e);
+  auto no_buffer = [&](const Job &j) {
+    return j.action == SGW_ACT_SPLIT || (from_host && j.action == SGW_ACT_COMPACT);
+  };
   for (size_t k = 0; k < jobs.size(); ++k) {
     Job &j = jobs[k];
-    if (!j.ready && j.action != SGW_ACT_SPLIT) {
+    if (!j.ready && !no_buffer(j)) {
       const int b = victim(k, -1);
       if (b < 0) return fail(SGW_ESTATE, "no edge buffer free");
       TRY(range_transfer(e, j, b));
     }
     if (k + 1 < jobs.size()) {  // prefetch the next transfer behind this relaxation
       Job &nx = jobs[k + 1];
-      if (!nx.ready && nx.action != SGW_ACT_SPLIT) {
+      if (!nx.ready && !no_buffer(nx)) {
         const int b = victim(k + 1, j.buf);
         if (b >= 0) TRY(range_transfer(e, nx, b));
       }
@@ -1288,6 +1338,8 @@ int process_iteration_ranges(sgw_engine *e) {
       e->buf_range[b] = -1;
       CK(cudaStreamWaitEvent(e->s_comp, e->ev_free[b], 0));
       TRY(process_hub(e, q, (uint32_t)b));
+    } else if (no_buffer(j)) {
+      TRY(process_from_host(e, q));
     } else {
       CK(cudaStreamWaitEvent(e->s_comp, e->ev_ready[j.buf], 0));
       e->cur_streamed = (j.action == SGW_ACT_RESIDENT || j.action == SGW_ACT_STREAM) ? 1u : 0u;
@@ -1306,7 +1358,7 @@ int process_iteration_ranges(sgw_engine *e) {
       e->range_inner_cap = 0;
       TRY(st);
     }
-    CK(cudaEventRecord(e->ev_free[j.buf], e->s_comp));
+    if (j.buf >= 0) CK(cudaEventRecord(e->ev_free[j.buf], e->s_comp));
     for (uint32_t s = j.s; s < j.s_end; ++s) inner_of[s] = inner;
     e->stats.partitions += 1;
   }

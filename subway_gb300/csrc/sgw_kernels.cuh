@@ -1317,6 +1317,26 @@ __device__ __forceinline__ void load_edge(const uint32_t *buf, uint32_t e, uint3
   }
 }
 
+// Reads edge record e of the host transfer copy (or of the graph's records
+// where they are read in place): the same forms, streams of chunks.
+struct HostEdges {
+  HostChunks ends, w;        // edge words, weight bytes (split form)
+  uint32_t split;            // this run reads the weight bytes
+};
+template <int W>
+__device__ __forceinline__ void load_edge_host(const HostEdges &h, uint32_t e, uint32_t pbits, uint32_t &dst,
+                                               uint32_t &w) {
+  if (W == 1) {
+    const uint32_t r = *reinterpret_cast<const uint32_t *>(hc_at(h.ends, (size_t)e * 4));
+    if (pbits) { dst = r & ((1u << pbits) - 1u); w = r >> pbits; }
+    else { dst = r; w = h.split ? (uint32_t)*reinterpret_cast<const uint8_t *>(hc_at(h.w, e)) : 0u; }
+  } else {
+    const uint2 ed = *reinterpret_cast<const uint2 *>(hc_at(h.ends, (size_t)e * 8));
+    dst = ed.x;
+    w = ed.y;
+  }
+}
+
 struct RelaxArgs {
   const uint32_t *queue;
   const uint32_t *ptr;
@@ -1338,6 +1358,7 @@ struct RelaxArgs {
   uint32_t stream_base;
   const uint32_t *off;
   const uint8_t *wbuf;       // split form: the buffer's weight bytes (else null)
+  HostEdges host;            // first passes that read the host copy themselves
 };
 
 constexpr int kRelaxThreads = 256;
@@ -1525,13 +1546,21 @@ struct WarpExpand {
 };
 
 template <class V, class F>
-__device__ __forceinline__ uint32_t warp_expand(WarpExpand<V> &s, int lane, uint32_t d, uint32_t boff, V val, F f) {
-  const uint32_t incl = warp_incl_scan(d, lane);
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+__device__ __forceinline__ uint32_t warp_expand(WarpExpand<V> &s, int lane, uint32_t d, uint32_t boff, V val, F f,
+                                                bool align = false) {
+  uint32_t incl = warp_incl_scan(d, lane);
+  uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
   if (total == 0) return 0;
-  const uint32_t excl = incl - d;
+  const uint32_t edges = total;
   const bool own = d > 0;
   const uint32_t owners = __ballot_sync(0xffffffffu, own);
+  uint32_t skip = 0;  // align: positions before the first edge that put the windows on multiples of 32
+  if (align) {
+    skip = __shfl_sync(0xffffffffu, boff, __ffs(owners) - 1) & 31u;
+    incl += skip;
+    total += skip;
+  }
+  const uint32_t excl = incl - d;
   const uint32_t le = lanemask_lt() | (1u << lane);
   if (own) {
     typename WarpExpand<V>::Own o;
@@ -1556,7 +1585,7 @@ __device__ __forceinline__ uint32_t warp_expand(WarpExpand<V> &s, int lane, uint
       for (int q = 0; q < kRelaxUnroll; ++q) {
         const uint32_t word = s.bits[w0 / 32u + q];
         const uint32_t j = w0 + 32u * q + lane;
-        ok[q] = j < end;
+        ok[q] = j < end && seg + j >= skip;
         const uint32_t r = base + __popc(word & le);
         base += __popc(word);
         if (ok[q]) {
@@ -1569,19 +1598,22 @@ __device__ __forceinline__ uint32_t warp_expand(WarpExpand<V> &s, int lane, uint
     }
   }
   __syncwarp();  // the tables are rewritten by the next tile
-  return total;
+  return edges;
 }
 
 // Relaxes the kRelaxUnroll edges of a lane: all record loads, then all
 // destination values, then the compares and reductions.
-template <int ALGO, int W>
+template <int ALGO, int W, bool HOST = false>
 __device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&pos)[kRelaxUnroll],
                                            const uint32_t (&sv)[kRelaxUnroll], const bool (&ok)[kRelaxUnroll]) {
   uint32_t dst[kRelaxUnroll], w[kRelaxUnroll], cur[kRelaxUnroll];
   bool any = false;
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
-    if (ok[q]) load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w[q], a.wbuf);
+    if (ok[q]) {
+      if (HOST) load_edge_host<W>(a.host, pos[q], a.pbits, dst[q], w[q]);
+      else load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w[q], a.wbuf);
+    }
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
     if (ok[q]) cur[q] = a.value[dst[q]];
@@ -1768,7 +1800,16 @@ __device__ __forceinline__ uint32_t unit_clip(unsigned long long start, uint32_t
   return a < hi ? (uint32_t)(hi - a) : 0u;
 }
 
-template <int ALGO, int W>
+// With HOST the records are read over the host link by the pass itself (a
+// partition that is relaxed once: every sync pass), at edge off[u] + j of the
+// host copy, so nothing is written to an edge buffer and read back, and the
+// relaxation hides behind the link.  Bound by the link (211 GB/s by DMA):
+// CC-sync over 32 M arcs out of memory reads at 193 GB/s (gather and relaxation
+// before: 1.45 + 0.78 ms partly overlapped, now 1.43), PageRank-sync's query on
+// R-MAT 2^20 went from 21.1 to 16.1 ms.  The windows of a tile start on
+// multiples of 32 edges there (warp_expand's align): without it each one
+// touches two 128-byte lines and CC's passes take 1.65 ms.
+template <int ALGO, int W, bool HOST>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_all(RelaxArgs a,
                                                                                   unsigned long long units,
                                                                                   unsigned long long per_warp) {
@@ -1796,13 +1837,13 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_a
         if (d || head) {
           val = a.value[u];
           if (!can_push<ALGO>(val)) { d = 0; head = false; }
-          boff = (a.streamed ? a.off[u] - a.stream_base : p0 - a.edge_from) + lo;
+          boff = (HOST ? a.off[u] : a.streamed ? a.off[u] - a.stream_base : p0 - a.edge_from) + lo;
         }
       }
       my_srcs += __popc(__ballot_sync(0xffffffffu, head));
       my_edges += warp_expand(s_exp[wid], lane, d, boff, val,
                               [&](const uint32_t (&pos)[kRelaxUnroll], const uint32_t (&sv)[kRelaxUnroll],
-                                  const bool (&ok)[kRelaxUnroll]) { any_update |= relax_lane<ALGO, W>(a, pos, sv, ok); });
+                                  const bool (&ok)[kRelaxUnroll]) { any_update |= relax_lane<ALGO, W, HOST>(a, pos, sv, ok); }, HOST);
       if (__any_sync(0xffffffffu, past)) break;
     }
   }
@@ -1960,6 +2001,7 @@ struct PrArgs {
   const uint32_t *off;
   double acc;
   double damping;
+  HostEdges host;
 };
 
 __device__ __forceinline__ double ld_relaxed_f64(const double *p) {
@@ -1970,13 +2012,16 @@ __device__ __forceinline__ double ld_relaxed_f64(const double *p) {
 
 // Adds each edge's push to its destination's residual: the records of
 // kRelaxUnroll edges of a lane are loaded before their (non-returning) adds.
-template <int W>
+template <int W, bool HOST>
 __device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[kRelaxUnroll],
                                         const double (&push)[kRelaxUnroll], const bool (&ok)[kRelaxUnroll]) {
   uint32_t dst[kRelaxUnroll], w;
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
-    if (ok[q]) load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w);
+    if (ok[q]) {
+      if (HOST) load_edge_host<W>(a.host, pos[q], a.pbits, dst[q], w);
+      else load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w);
+    }
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
     if (ok[q]) atomicAdd(&a.delta[dst[q]], push[q]);
@@ -1988,7 +2033,7 @@ __device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[k
 // not active again) has written.  PageRank's later rounds queue a few tens of
 // thousands of long rows, which left most of the chip idle when each CTA took
 // 256 of them and found its edges' owners by binary search.
-template <int W>
+template <int W, bool HOST>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(PrArgs a, unsigned long long units,
                                                                                unsigned long long per_warp) {
   __shared__ CtaTally s_tally;
@@ -2021,12 +2066,12 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(
         uint32_t lo;
         d = unit_clip<kRelaxHeader>(start, p1 - p0, t0, t1, &lo, &head);
         if (push == 0.0) d = 0;
-        if (d) boff = (a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from) + lo;
+        if (d) boff = (HOST ? a.off[a.queue[i]] : a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from) + lo;
       }
       if (a.iter == 1) my_srcs += __popc(__ballot_sync(0xffffffffu, head));
       my_edges += warp_expand(s_exp[wid], lane, d, boff, push,
                               [&](const uint32_t (&pos)[kRelaxUnroll], const double (&pv)[kRelaxUnroll],
-                                  const bool (&ok)[kRelaxUnroll]) { pr_lane<W>(a, pos, pv, ok); });
+                                  const bool (&ok)[kRelaxUnroll]) { pr_lane<W, HOST>(a, pos, pv, ok); }, HOST);
       if (__any_sync(0xffffffffu, past)) break;
     }
   }

@@ -65,3 +65,34 @@ def test_hub_thresholds(gpu, orc, tile_degree_max):
         for mode in ("sync", "async"):
             vals, _ = eng.run(algo, mode, 0)
             assert np.array_equal(vals, ref), (algo, mode)
+
+
+FORMS = [("packed", {}), ("split", {"flags": "OPT_SPLIT_WEIGHTS"}), ("records", {"flags": "OPT_NO_PACK"}),
+         ("in_place", {"flags": "OPT_GRAPH_IN_PLACE"}), ("chunks", {"transfer_chunk_log2": 12})]
+
+
+@pytest.mark.parametrize("policy", ["plain", "learned"])
+@pytest.mark.parametrize("form", [f[0] for f in FORMS])
+def test_sync_reads_every_transfer_form(gpu, orc, form, policy):
+    """Sync passes read the host copy themselves: packed words, the split
+    form's two streams, records, the graph in place, and copies cut into 4 KiB
+    chunks, with rows that start at every alignment.  Integer answers are the
+    oracle's; PageRank's equal the gathering form's to its FP32 rounding."""
+    opts = dict(dict(FORMS)[form])
+    flags = getattr(gpu, opts.pop("flags"), 0) if "flags" in opts else 0
+    g = gpu.Graph.rmat(11, 9, seed=77, weighted=True, wmax=200)
+    budget = 36 * g.n + 96 * 1024 + 3000 * 16
+    eng = gpu.Engine(g, budget_bytes=budget, flags=flags, **opts)
+    ref_eng = gpu.Engine(g, budget_bytes=budget, flags=gpu.OPT_SCALAR_GATHER)
+    if policy == "learned":
+        eng.set_policy("learned")
+    src = int(g.pick_sources(1, seed=5)[0])
+    for algo in ("bfs", "sssp", "sswp", "cc"):
+        e = g.edges if algo in ("sssp", "sswp") else np.ascontiguousarray(g.ends)
+        vals, st = eng.run(algo, "sync", src)
+        assert np.array_equal(vals, orc.run(algo, g.node_pointer, e, src)), algo
+        assert st["partitions"] > 1 and st["gather_launches"] == 0 or policy == "learned"
+    a, _ = eng.run("pr", "sync", pr_acc=0.001)
+    b, _ = ref_eng.run("pr", "sync", pr_acc=0.001)
+    # FP64 sums in another order, cast to FP32: one unit in the last place
+    assert np.max(np.abs(a.astype(np.float64) - b) / b) < 1.2e-7 * 2
