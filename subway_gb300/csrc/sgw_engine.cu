@@ -876,6 +876,15 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   a.acc = (double)e->params.pr_acc;
   a.damping = (double)e->params.pr_damping;
   a.host = host_edges(e);
+  // without a row above tile_degree_max a warp's 32 rows are short enough to
+  // need no cut by edges, and the claim and the pushes fit one launch
+  if (iter > 1 && e->max_degree <= e->opts.tile_degree_max) {
+    k_pr_warp<W><<<grid_for(e, q.size, kRelaxThreads), kRelaxThreads, 0, e->s_comp>>>(a);
+    CK(cudaGetLastError());
+    e->stats.launches += 1;
+    e->stats.relax_launches += 1;
+    return SGW_OK;
+  }
   if (iter > 1) {
     k_pr_claim<<<grid_for(e, q.size, kRelaxThreads), kRelaxThreads, 0, e->s_comp>>>(a);
     CK(cudaGetLastError());

@@ -96,3 +96,26 @@ def test_sync_reads_every_transfer_form(gpu, orc, form, policy):
     b, _ = ref_eng.run("pr", "sync", pr_acc=0.001)
     # FP64 sums in another order, cast to FP32: one unit in the last place
     assert np.max(np.abs(a.astype(np.float64) - b) / b) < 1.2e-7 * 2
+
+
+@pytest.mark.parametrize("tile_degree_max", [8, 256])
+def test_pagerank_async_long_and_short_rows(gpu, orc, tile_degree_max):
+    """Later async passes as one launch (no row above the threshold) and as a
+    claim and a push cut by edges: within the residual bound of the exact
+    fixpoint, as the forms with one kernel per tile were."""
+    acc = 1e-6
+    g = gpu.Graph.er(3001, 24000, seed=3)
+    assert 8 < int(g.out_degree().max()) < 256
+    eng = gpu.Engine(g, tile_degree_max=tile_degree_max)
+    v, _ = eng.run("pr", "async", pr_acc=acc)
+    npt = g.node_pointer.astype(np.int64)
+    deg = np.diff(npt)
+    src = np.repeat(np.arange(g.n), deg)
+    rank = np.full(g.n, 0.15)
+    for _ in range(400):
+        nxt = np.full(g.n, 0.15)
+        np.add.at(nxt, g.ends, 0.85 * (rank / np.maximum(deg, 1))[src])
+        rank = nxt
+    # every vertex is left with a residual of at most acc, 1/0.15 of which can still arrive
+    bound = (acc / 0.15) * rank + 3e-7 * rank
+    assert np.all(np.abs(v - rank) <= bound)
