@@ -465,8 +465,9 @@ int sgw_range_trace_read(const sgw_engine *e, sgw_range_rec *out, uint64_t capac
  * frontier/relax iteration on the device until no lane improves.  Results
  * are bit-exact with single-source runs.
  * opts: budget_bytes (admission: SGW_EBUDGET if the graph, lanes x n
- * distances and the work lists do not fit), device, chunk_edges (edges per
- * work item, default 256), flags (SGW_OPT_NO_PACK). */
+ * distances and the work lists do not fit), device, chunk_edges (fewest edges
+ * that one warp's share of an iteration holds; 0: chosen by the algorithm),
+ * flags (SGW_OPT_NO_PACK). */
 typedef struct sgw_batch sgw_batch;
 typedef struct sgw_batch_stats {
   uint32_t iterations;      /* frontier iterations of the batch               */

@@ -64,7 +64,7 @@ def lib_sources():
 
 def lib_deps():
     return lib_sources() + [CSRC / "sgw_kernels.cuh", CSRC / "sgw_internal.h", CSRC / "sgw_mlp.cuh",
-                            INCLUDE / "subway_gb300.h", INCLUDE / "sgw_graphgen.h"]
+                            CSRC / "sgw_warp.cuh", INCLUDE / "subway_gb300.h", INCLUDE / "sgw_graphgen.h"]
 
 
 def build_lib(verbose=False, force=False) -> Path:

@@ -3,14 +3,14 @@
 // No counterpart in the reference, which answers one source per process.
 //
 // Device state: the CSR (packed 4-byte records when weights fit, as in the
-// engine), dist[v][lane] (vertex-major, so a warp touches one 128-byte line
-// per edge), and per-vertex 64-bit lane masks for the current and next
-// frontier.  One iteration:
-//   k_b_frontier  vertices with a next-mask move it to the current mask and
-//                 append (vertex, edge chunk) work items
-//   k_b_relax     one warp per work item: the 32 (or 2 x 32) lanes relax the
-//                 item's edges for their own query; improvements are
-//                 balloted into one atomicOr on the destination's next mask
+// engine), per-vertex 64-bit lane masks, and for SSSP dist[v][lane]
+// (vertex-major: an edge touches one 128-byte line per 32 queries), for BFS the
+// bits of the levels as planes in the same space.  One iteration:
+//   k_b_frontier  vertices with a next mask move it to the current mask and
+//                 become rows of a compacted frontier with a prefix of work units
+//   k_b_relax     the rows' edges, cut into equal shares for the warps: BFS one
+//                 edge per lane for all queries at once, SSSP one edge per eight
+//                 lanes and 32 queries
 //   k_b_cond      sets the conditional handle: loop while the frontier was
 //                 non-empty (bounded by an iteration limit)
 // The iteration is the body of a CUDA-graph conditional WHILE node, so a
@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "sgw_internal.h"
+#include "sgw_warp.cuh"
 
 #define CK(call)                                                                       \
   do {                                                                                 \
@@ -36,258 +37,410 @@
 
 namespace {
 
+using namespace sgw;
+
 constexpr uint32_t kBInf = 4294967294u;
 constexpr int kBThreads = 256;
-constexpr uint32_t kBUnroll = 4;
+constexpr int kBWarps = kBThreads / 32;
 
-struct BItem {
-  uint32_t u;    // source vertex
-  uint32_t e0;   // first edge: low 32 bits
-  uint32_t cnt;  // edges in this item
-  uint32_t e0hi; //   and high 32 bits
+// Per-vertex lane masks.  BFS keeps the queries that have reached a vertex
+// beside those that reach it next, so an edge tests both with one 16-byte
+// load; SSSP uses `next` alone.
+struct __align__(16) BMask {
+  unsigned long long seen, next;
 };
 
-// counters: [0] work items, [1] frontier vertices, [2] iterations run,
-// [3] error (1 = item list overflow, 2 = iteration limit)
-__global__ void k_b_fill(uint32_t *dist, size_t count, unsigned long long *next, unsigned long long *seen,
-                         uint32_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
-    dist[i] = kBInf;
-  for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
-    next[v] = 0ull;
-    seen[v] = 0ull;
+// Counter words (ctr).  Graph loop: [0..1] one 64-bit counter, the frontier's
+// rows (high word) and work units (low word), [2] iterations run, [3] error
+// (2 = iteration limit, 4 = a grid barrier gave up), [12] frontier vertices.
+// Persistent form: [4..5] / [6..7] and [12] / [13] the counters of even / odd
+// iterations, [8] barrier arrivals, [9] barrier generation.  [10] 16-bit
+// overflow.
+template <int L, bool SSSP>
+__global__ void k_b_fill(uint32_t *dist, BMask *mask, uint32_t n) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x, t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (SSSP) {  // BFS answers are built from level planes that need no fill
+    const uint4 inf = make_uint4(kBInf, kBInf, kBInf, kBInf);
+    for (size_t i = t; i < (size_t)n * (L / 4); i += stride) reinterpret_cast<uint4 *>(dist)[i] = inf;
   }
+  for (size_t v = t; v < n; v += stride) *reinterpret_cast<uint4 *>(&mask[v]) = make_uint4(0, 0, 0, 0);
 }
 
-template <int L>
-__global__ void k_b_seed(const uint32_t *src, uint32_t nsrc, uint32_t *dist, unsigned long long *next,
-                         unsigned long long *seen, uint32_t *ctr) {
+template <int L, bool SSSP>
+__global__ void k_b_seed(const uint32_t *src, uint32_t nsrc, uint32_t *dist, BMask *mask, uint32_t *ctr) {
   const uint32_t l = threadIdx.x;
   if (l < nsrc) {
     const uint32_t s = src[l];
-    dist[(size_t)s * L + l] = 0;
-    atomicOr(&next[s], 1ull << l);
-    atomicOr(&seen[s], 1ull << l);
+    if (SSSP) dist[(size_t)s * L + l] = 0;
+    atomicOr(&mask[s].next, 1ull << l);
   }
   if (l < 16) ctr[l] = 0;
 }
 
-__global__ void k_b_reset(uint32_t *ctr) {
-  ctr[0] = 0;
-  ctr[1] = 0;
-}
-
+// ---- frontier phase ----------------------------------------------------------------
+// Every vertex whose `next` mask holds a query that is new to it joins the
+// frontier: its mask moves to cur, and it gets a row in (rows, unit).  A row is
+// 1 + ceil(degree / kBUnit) work units; `unit` is its first one.  A CTA takes
+// kBVerts vertices at a time and reserves their rows and units with one
+// 64-bit add, so both counts are prefixes in the same order and the relax
+// phase can cut the units into equal shares.
+//
 // Loads that follow writes made earlier in the same launch (the persistent
 // form runs every phase in one kernel) go through L2 (__ldcg): L1 and the
 // read-only path are not kept coherent within a kernel.
-__device__ __forceinline__ BItem b_item(const BItem *items, uint32_t i) {
-  const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(items) + i);
-  BItem it;
-  it.u = v.x;
-  it.e0 = v.y;
-  it.cnt = v.z;
-  it.e0hi = v.w;
-  return it;
+constexpr uint32_t kBUnit = 8;    // edges
+constexpr int kBPer = 4;          // vertices per thread
+constexpr uint32_t kBVerts = kBThreads * kBPer;
+
+struct BState {
+  uint32_t n, pbits;
+  const uint32_t *off, *edges;
+  const unsigned long long *obase;
+  uint32_t *dist;                // SSSP distances / BFS level planes
+  unsigned long long *cur;
+  BMask *mask;
+  uint32_t *rows, *unit;         // frontier rows: vertex, first work unit
+  uint32_t min_units;            // fewest units in a warp's share
+};
+
+struct BFrontierSmem {
+  unsigned long long warp[kBWarps];
+  unsigned long long base;
+  uint32_t act;
+};
+
+// Level planes (BFS): bit l of plane k of vertex v is bit k of query l's
+// level.  Plane k is first written, for every vertex, at level 2^k, so planes
+// need no fill, a frontier vertex costs a few coalesced words per level instead
+// of a scattered store per query, and the planes that a traversal of D levels
+// writes take log2(D) words of the space that 32-bit levels would.
+template <int L> struct BPlane { using T = unsigned long long; };
+template <> struct BPlane<32> { using T = uint32_t; };
+
+template <int L>
+__device__ __forceinline__ void b_set_level(const BState &s, uint32_t v, unsigned long long fresh, uint32_t level) {
+  using T = typename BPlane<L>::T;
+  T *const plane = reinterpret_cast<T *>(s.dist);
+  if (level == 0) return;
+  if ((level & (level - 1)) == 0) {  // this level is the first with its highest bit
+    plane[(size_t)(31 - __clz((int)level)) * s.n + v] = (T)fresh;
+    return;
+  }
+  if (!fresh) return;
+  for (uint32_t m = level; m; m &= m - 1) {
+    T *const p = plane + (size_t)(__ffs((int)m) - 1) * s.n + v;
+    *p = __ldcg(p) | (T)fresh;
+  }
 }
 
-// Frontier phase.  ctr[0]: work items appended, ctr[1]: frontier vertices;
-// err: set to 1 when the item list overflows.
-__device__ __forceinline__ size_t b_first_edge(const BItem &it) { return ((size_t)it.e0hi << 32) | it.e0; }
-
-__device__ __forceinline__ void b_frontier(uint32_t n, const uint32_t *__restrict__ off,
-                                           const unsigned long long *__restrict__ obase, unsigned long long *cur,
-                                           unsigned long long *next, BItem *items, uint32_t cap, uint32_t *ctr,
-                                           uint32_t chunk, uint32_t *err) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  // loop bound rounded up to whole warps so every lane reaches the shuffles
-  const uint32_t limit = (n + 31) & ~31u;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < limit; v += stride) {
-    uint32_t nch = 0, deg = 0;
-    unsigned long long e0 = 0;
-    bool act = false;
-    if (v < n) {
-      const unsigned long long m = __ldcg(&next[v]);
-      if (m) {
-        act = true;
-        cur[v] = m;
-        next[v] = 0ull;
-        e0 = sgw::off_at(off, obase, v);
-        deg = off[v + 1] - off[v];
-        nch = (deg + chunk - 1) / chunk;
+template <bool SSSP, int L>
+__device__ __forceinline__ void b_frontier(const BState &s, BFrontierSmem &sm, unsigned long long *ctr,
+                                           uint32_t *active, uint32_t level) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (uint32_t base = blockIdx.x * kBVerts; base < s.n; base += gridDim.x * kBVerts) {
+    uint32_t units[kBPer], mine = 0, rows = 0, act = 0;
+#pragma unroll
+    for (int k = 0; k < kBPer; ++k) {
+      const uint32_t v = base + k * kBThreads + tid;
+      units[k] = 0;
+      if (v >= s.n) continue;
+      unsigned long long fresh;
+      if (SSSP) {
+        fresh = __ldcg(&s.mask[v].next);
+        if (fresh) s.mask[v].next = 0ull;
+      } else {
+        const ulonglong2 m = __ldcg(reinterpret_cast<const ulonglong2 *>(&s.mask[v]));
+        fresh = m.y & ~m.x;
+        if (m.y) *reinterpret_cast<ulonglong2 *>(&s.mask[v]) = make_ulonglong2(m.x | fresh, 0ull);
+        b_set_level<L>(s, v, fresh, level);
+      }
+      if (fresh) {
+        s.cur[v] = fresh;
+        ++act;
+        const uint32_t deg = s.off[v + 1] - s.off[v];
+        if (deg) {
+          units[k] = 1 + (deg + kBUnit - 1) / kBUnit;
+          mine += units[k];
+          ++rows;
+        }
       }
     }
-    const uint32_t nact = __popc(__ballot_sync(0xffffffffu, act));
-    if (lane == 0 && nact) atomicAdd(&ctr[1], nact);
-    // warp-aggregated reservation of item slots
-    uint32_t incl = nch;
+    // exclusive prefix of (rows, units) over the CTA's threads
+    unsigned long long incl = ((unsigned long long)rows << 32) | mine;
+    const unsigned long long own = incl;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += y;
     }
-    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t base = 0;
-    if (lane == 31 && tot) base = atomicAdd(&ctr[0], tot);
-    base = __shfl_sync(0xffffffffu, base, 31) + incl - nch;
-    for (uint32_t c = 0; c < nch; ++c) {
-      if (base + c < cap) {
-        BItem it;
-        it.u = v;
-        const unsigned long long f = e0 + (unsigned long long)c * chunk;
-        it.e0 = (uint32_t)f;
-        it.cnt = min(chunk, deg - c * chunk);
-        it.e0hi = (uint32_t)(f >> 32);
-        items[base + c] = it;
-      } else {
-        atomicExch(err, 1u);
+    const uint32_t wact = __reduce_add_sync(0xffffffffu, act);
+    if (tid == 0) sm.act = 0;
+    if (lane == 31) sm.warp[warp] = incl;
+    __syncthreads();
+    if (lane == 0 && wact) atomicAdd(&sm.act, wact);
+    if (tid == 0) {
+      unsigned long long acc = 0;
+#pragma unroll
+      for (int w = 0; w < kBWarps; ++w) {
+        const unsigned long long x = sm.warp[w];
+        sm.warp[w] = acc;
+        acc += x;
       }
+      sm.base = acc ? atomicAdd(ctr, acc) : 0ull;
+    }
+    __syncthreads();
+    if (tid == 0 && sm.act) atomicAdd(active, sm.act);
+    unsigned long long at = sm.base + sm.warp[warp] + incl - own;
+#pragma unroll
+    for (int k = 0; k < kBPer; ++k)
+      if (units[k]) {
+        s.rows[at >> 32] = base + k * kBThreads + tid;
+        s.unit[at >> 32] = (uint32_t)at;
+        at += (1ull << 32) | units[k];
+      }
+    __syncthreads();  // the tables are rewritten by the next tile
+  }
+}
+
+template <bool SSSP, int L>
+__global__ void __launch_bounds__(kBThreads) k_b_frontier(BState s, uint32_t *ctr) {
+  __shared__ BFrontierSmem sm;
+  b_frontier<SSSP, L>(s, sm, reinterpret_cast<unsigned long long *>(ctr), ctr + 12, ctr[2]);
+}
+
+// ---- relax phase -------------------------------------------------------------------
+// The frontier's work units are cut into equal shares of at most `share`; a warp
+// finds a share's first row with a 32-way search and goes through its rows 32
+// at a time, the first and the last clipped to the share.  (One warp per row or
+// per piece of 256 edges left most warps waiting at the end of an iteration for
+// the few that had drawn the long rows: 60% of the SSSP kernel's stalls.)
+// SSSP shares are short, since a warp takes several microseconds per edge group
+// and the rows, hubs first, should see each other's improvements (64 queries on
+// R-MAT 2^20: 5.4 ms with 16 units, 5.9 with 64, 6.6 with 4); BFS shares are long
+// enough to hide the search (0.50 ms with 256, 0.57 with 32, 0.73 with 16).
+// f(u, e0, d, mask) gets a lane's row part.
+constexpr uint32_t kBSsspShare = 16, kBBfsShare = 256;
+// CTAs per SM each form is compiled for: SSSP gains from more warps than its
+// registers would leave (1.39 ms unbounded, 1.01 at 5, 1.28 at 8 for 32 queries
+// on R-MAT 2^18), BFS loses (0.49 ms at 3, 0.52 at 4, 0.86 at 6).
+constexpr int kBSsspCtas = 5, kBBfsCtas = 3;
+template <class F>
+__device__ __forceinline__ void b_rows(const BState &s, unsigned long long total, uint32_t share, F f) {
+  const uint32_t count = (uint32_t)(total >> 32), units = (uint32_t)total;
+  const int lane = threadIdx.x & 31;
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t per = max(s.min_units, min(share, (units + nw - 1) / nw));
+  for (unsigned long long t0 = (unsigned long long)per * gw; t0 < units; t0 += (unsigned long long)per * nw) {
+    const unsigned long long t1 = min((unsigned long long)units, t0 + per);
+    uint32_t lo = 0, hi = count;  // last row whose first unit is <= t0
+    while (hi - lo > 32u) {
+      const uint32_t step = (hi - lo + 31u) / 32u, i = lo + (uint32_t)lane * step;
+      const uint32_t m = __ballot_sync(0xffffffffu, i < hi && __ldcg(&s.unit[i]) <= t0);
+      lo += (31u - (uint32_t)__clz((int)m)) * step;
+      hi = min(hi, lo + step);
+    }
+    {
+      const uint32_t i = lo + (uint32_t)lane;
+      const uint32_t m = __ballot_sync(0xffffffffu, i < hi && __ldcg(&s.unit[i]) <= t0);
+      lo += 31u - (uint32_t)__clz((int)m);
+    }
+    for (uint32_t i0 = lo; i0 < count; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      uint32_t u = 0, d = 0;
+      unsigned long long e0 = 0, mask = 0;
+      bool past = true;
+      if (i < count) {
+        const unsigned long long first = (unsigned long long)__ldcg(&s.unit[i]) + 1;  // the row's first edge unit
+        past = first > t1;
+        if (!past) {
+          u = __ldcg(&s.rows[i]);
+          const uint32_t deg = s.off[u + 1] - s.off[u];
+          const unsigned long long x = t0 > first ? (t0 - first) * kBUnit : 0, y = t1 > first ? (t1 - first) * kBUnit : 0;
+          const unsigned long long end = min(y, (unsigned long long)deg);
+          if (x < end) {
+            d = (uint32_t)(end - x);
+            e0 = off_at(s.off, s.obase, u) + x;
+            mask = __ldcg(&s.cur[u]);
+          }
+        }
+      }
+      f(u, e0, d, mask);
+      if (__any_sync(0xffffffffu, past)) break;
     }
   }
 }
 
-__global__ void __launch_bounds__(kBThreads) k_b_frontier(uint32_t n, const uint32_t *__restrict__ off,
-                                                          const unsigned long long *__restrict__ obase,
-                                                          unsigned long long *cur, unsigned long long *next,
-                                                          BItem *items, uint32_t cap, uint32_t *ctr,
-                                                          uint32_t chunk) {
-  b_frontier(n, off, obase, cur, next, items, cap, ctr, chunk, &ctr[3]);
+// What an edge needs of its row.
+struct BRow {
+  uint32_t lane;            // the row's lane
+  uint32_t lo32;            // low word of the row's first edge
+  unsigned long long e0;    // the row's first edge
+  unsigned long long mask;
+};
+__device__ __forceinline__ size_t b_edge(const BRow &r, uint32_t pos) { return (size_t)r.e0 + (uint32_t)(pos - r.lo32); }
+
+// BFS, bit-parallel over the lanes (multi-source BFS): lane i of a window takes
+// edge i and adds the row's queries that have not reached the destination to
+// its next mask.  The adds are non-returning, and only the frontier phase
+// writes `seen`, so an edge whose queries are all there already costs one
+// 16-byte load.
+template <int W>
+__device__ __forceinline__ void b_bfs_relax(const BState &s, WarpExpand<BRow> *exp, unsigned long long total) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t dmask = s.pbits ? ((1u << s.pbits) - 1u) : 0xffffffffu;
+  b_rows(s, total, kBBfsShare, [&](uint32_t, unsigned long long e0, uint32_t d, unsigned long long mask) {
+    BRow r;
+    r.lane = (uint32_t)lane;
+    r.lo32 = (uint32_t)e0;
+    r.e0 = e0;
+    r.mask = mask;
+    warp_expand(*exp, lane, d, (uint32_t)e0, r,
+                [&](const uint32_t (&pos)[kRelaxUnroll], const BRow (&row)[kRelaxUnroll],
+                    const bool (&ok)[kRelaxUnroll]) {
+                  uint32_t dst[kRelaxUnroll];
+                  ulonglong2 m[kRelaxUnroll];
+#pragma unroll
+                  for (int q = 0; q < kRelaxUnroll; ++q)
+                    if (ok[q]) {
+                      const size_t e = b_edge(row[q], pos[q]);
+                      dst[q] = W == 1 ? (s.edges[e] & dmask) : s.edges[2 * e];
+                    }
+#pragma unroll
+                  for (int q = 0; q < kRelaxUnroll; ++q)
+                    if (ok[q]) m[q] = __ldcg(reinterpret_cast<const ulonglong2 *>(&s.mask[dst[q]]));
+#pragma unroll
+                  for (int q = 0; q < kRelaxUnroll; ++q)
+                    if (ok[q]) {
+                      const unsigned long long add = row[q].mask & ~(m[q].x | m[q].y);
+                      if (add) atomicOr(&s.mask[dst[q]].next, add);
+                    }
+                });
+  });
 }
 
-// Distance-lane relaxation phase over the nitems work items.
-template <bool SSSP, int W, int L>
-__device__ __forceinline__ void b_relax(const BItem *items, uint32_t nitems,
-                                        const uint32_t *__restrict__ edges, uint32_t pbits, uint32_t *dist,
-                                        const unsigned long long *cur, unsigned long long *next) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t dmask = pbits ? ((1u << pbits) - 1u) : 0xffffffffu;
-  for (uint32_t i = gw; i < nitems; i += nw) {
-    const BItem it = b_item(items, i);
-    const unsigned long long mask = __ldcg(&cur[it.u]);
-#pragma unroll
+// SSSP: a lane relaxes one edge for four queries (16 bytes of distances), so
+// eight lanes cover the 32 queries of one half and a warp four edges at once;
+// kBGroup such groups of loads are in flight.  Lane i first loads edge i of a
+// window (destination, weight, its row's lane), then each eight lanes take
+// every fourth edge, reading the source's distances where the row changes and
+// the destination's.  What bounds a batch is issuing instructions, not the L2:
+// with one query per lane an edge cost a warp about 35 of them (32 queries on
+// R-MAT 2^18: 2.6 ms, now 1.0; 64 on 2^20: 10.9 and 5.3).  A candidate below the
+// value read improves the destination in this iteration (by this lane or by
+// whichever wins), so non-returning reductions suffice and the lane bits are
+// right.  In a small frontier, bound by latency, a query whose distance has
+// improved again since the frontier phase is left to the next iteration, which
+// it is in anyway, so the number of iterations does not hang on timing; in a
+// large one its fresh distance is used, which saves a fifth of the time.
+constexpr int kBGroup = 2;
+constexpr uint32_t kBLarge = 65536;  // work units
+
+template <int W, int L>
+__device__ __forceinline__ void b_sssp_relax(const BState &s, WarpExpand<BRow> *exp, unsigned long long total) {
+  const int lane = threadIdx.x & 31, g = lane >> 3, c = lane & 7;
+  const uint32_t dmask = s.pbits ? ((1u << s.pbits) - 1u) : 0xffffffffu;
+  const bool large = (uint32_t)total > kBLarge;
+  b_rows(s, total, kBSsspShare, [&](uint32_t u, unsigned long long e0, uint32_t d0, unsigned long long mask) {
+#pragma unroll 1
     for (int h = 0; h < L / 32; ++h) {
-      const uint32_t bits = (uint32_t)(mask >> (32 * h));
-      if (bits == 0) continue;
-      const bool active = (bits >> lane) & 1u;
-      const uint32_t du = active ? __ldcg(&dist[(size_t)it.u * L + 32 * h + lane]) : kBInf;
-      for (uint32_t c = 0; c < it.cnt; c += 32) {
-        // lane k loads edge c + k; the warp then walks them together
-        uint32_t rd = 0, rw = 0;
-        if (c + lane < it.cnt) {
-          const size_t e = b_first_edge(it) + c + lane;
-          if (W == 1) {
-            const uint32_t r = edges[e];
-            rd = r & dmask;
-            rw = pbits ? (r >> pbits) : 0u;
-          } else {
-            rd = edges[2 * e];
-            rw = edges[2 * e + 1];
-          }
-        }
-        const uint32_t cnt = min(32u, it.cnt - c);
-        // kBUnroll destination lines in flight per warp before the compares
-        for (uint32_t k0 = 0; k0 < cnt; k0 += kBUnroll) {
-          uint32_t dst[kBUnroll], w[kBUnroll], seen[kBUnroll];
-#pragma unroll
-          for (int q = 0; q < kBUnroll; ++q) {
-            dst[q] = __shfl_sync(0xffffffffu, rd, (k0 + q) & 31u);
-            w[q] = __shfl_sync(0xffffffffu, rw, (k0 + q) & 31u);
-          }
-#pragma unroll
-          for (int q = 0; q < kBUnroll; ++q)
-            seen[q] = (active && k0 + q < cnt) ? __ldcg(&dist[(size_t)dst[q] * L + 32 * h + lane]) : 0u;
-#pragma unroll
-          for (int q = 0; q < kBUnroll; ++q) {
-            if (k0 + q >= cnt) break;  // uniform across the warp
-            // a candidate below the value read improves the destination in
-            // this iteration (by this lane or by whichever wins), so the
-            // non-returning atomic suffices and the lane bit is right
-            bool improved = false;
-            if (active) {
-              const uint32_t cand = du + (SSSP ? w[q] : 1u);
-              if (cand < seen[q]) {
-                atomicMin(&dist[(size_t)dst[q] * L + 32 * h + lane], cand);
-                improved = true;
+      uint32_t *const dist = s.dist + 32 * h + 4 * c;
+      const uint32_t bits = d0 ? (uint32_t)(mask >> (32 * h)) : 0u;
+      BRow r;
+      r.lane = (uint32_t)lane;
+      r.lo32 = (uint32_t)e0;
+      r.e0 = e0;
+      r.mask = 0;
+      uint32_t held = 32;  // the row whose distances du holds
+      uint4 du = make_uint4(kBInf, kBInf, kBInf, kBInf);
+      warp_expand<1>(
+          *exp, lane, bits ? d0 : 0u, (uint32_t)e0, r,
+          [&](const uint32_t (&pos)[1], const BRow (&row)[1], const bool (&ok)[1]) {
+            uint32_t rd = 0, rw = 0;
+            if (ok[0]) {
+              const size_t e = b_edge(row[0], pos[0]);
+              if (W == 1) {
+                const uint32_t x = s.edges[e];
+                rd = x & dmask;
+                rw = s.pbits ? (x >> s.pbits) : 0u;
+              } else {
+                rd = s.edges[2 * e];
+                rw = s.edges[2 * e + 1];
               }
             }
-            const uint32_t imp = __ballot_sync(0xffffffffu, improved);
-            if (imp && lane == 0) atomicOr(&next[dst[q]], (unsigned long long)imp << (32 * h));
-          }
-        }
-      }
+            const uint32_t rl = row[0].lane;
+            const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, ok[0]));  // a prefix of lanes
+            for (uint32_t k0 = 0; k0 < cnt; k0 += 4 * kBGroup) {
+              uint32_t dst[kBGroup], w[kBGroup];
+              uint4 src[kBGroup], seen[kBGroup];
+#pragma unroll
+              for (int q = 0; q < kBGroup; ++q) {
+                const uint32_t k = k0 + 4 * q + g, kk = min(k, cnt - 1);
+                const uint32_t row_lane = __shfl_sync(0xffffffffu, rl, kk);
+                dst[q] = __shfl_sync(0xffffffffu, rd, kk);
+                w[q] = __shfl_sync(0xffffffffu, rw, kk);
+                const uint32_t ru = __shfl_sync(0xffffffffu, u, row_lane);
+                uint32_t on = __shfl_sync(0xffffffffu, bits, row_lane) >> (4 * c);
+                if (row_lane != held) {
+                  held = row_lane;
+                  du = make_uint4(kBInf, kBInf, kBInf, kBInf);
+                  if (on & 15u) {
+                    du = __ldcg(reinterpret_cast<const uint4 *>(dist + (size_t)ru * L));
+                    if (!large) on &= ~(__ldcg(reinterpret_cast<const uint32_t *>(&s.mask[ru].next) + h) >> (4 * c));
+                    if (!(on & 1u)) du.x = kBInf;
+                    if (!(on & 2u)) du.y = kBInf;
+                    if (!(on & 4u)) du.z = kBInf;
+                    if (!(on & 8u)) du.w = kBInf;
+                  }
+                }
+                src[q] = du;
+                seen[q] = make_uint4(0, 0, 0, 0);
+                if (k < cnt && (on & 15u)) seen[q] = __ldcg(reinterpret_cast<const uint4 *>(dist + (size_t)dst[q] * L));
+              }
+#pragma unroll
+              for (int q = 0; q < kBGroup; ++q) {
+                const uint32_t cand[4] = {src[q].x + w[q], src[q].y + w[q], src[q].z + w[q], src[q].w + w[q]};
+                uint32_t imp = 0;
+                if (src[q].x != kBInf && cand[0] < seen[q].x) imp |= 1u;
+                if (src[q].y != kBInf && cand[1] < seen[q].y) imp |= 2u;
+                if (src[q].z != kBInf && cand[2] < seen[q].z) imp |= 4u;
+                if (src[q].w != kBInf && cand[3] < seen[q].w) imp |= 8u;
+                if (!__any_sync(0xffffffffu, imp)) continue;
+                uint32_t m = imp << (4 * c);  // the edge's improved queries, from its eight lanes
+                m |= __shfl_xor_sync(0xffffffffu, m, 1);
+                m |= __shfl_xor_sync(0xffffffffu, m, 2);
+                m |= __shfl_xor_sync(0xffffffffu, m, 4);
+                if (c == 0 && m) atomicOr(&s.mask[dst[q]].next, (unsigned long long)m << (32 * h));
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if ((imp >> i) & 1u) atomicMin(dist + (size_t)dst[q] * L + i, cand[i]);
+              }
+            }
+          });
     }
-  }
+  });
 }
 
 template <bool SSSP, int W, int L>
-__global__ void __launch_bounds__(kBThreads) k_b_relax(const BItem *__restrict__ items, const uint32_t *ctr,
-                                                       uint32_t cap, const uint32_t *__restrict__ edges,
-                                                       uint32_t pbits, uint32_t *dist,
-                                                       const unsigned long long *__restrict__ cur,
-                                                       unsigned long long *next) {
-  b_relax<SSSP, W, L>(items, min(ctr[0], cap), edges, pbits, dist, cur, next);
-}
-
-// BFS, bit-parallel over the lanes (multi-source BFS): a vertex's 64-bit
-// `seen` mask holds the queries that have reached it.  Lane k of the warp
-// takes edge c + k of the item; one atomicOr claims, for every query whose
-// frontier holds the item's vertex, the destination's still-unseen lanes;
-// those get level = iteration + 1 and join the next frontier.  Each (vertex,
-// query) bit is claimed exactly once, so the levels are the BFS levels.
-template <int W, int L>
-__device__ __forceinline__ void b_bfs_relax(const BItem *items, uint32_t nitems, uint32_t level,
-                                            const uint32_t *__restrict__ edges, uint32_t pbits, uint32_t *dist,
-                                            const unsigned long long *cur, unsigned long long *next,
-                                            unsigned long long *seen) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t dmask = pbits ? ((1u << pbits) - 1u) : 0xffffffffu;
-  for (uint32_t i = gw; i < nitems; i += nw) {
-    const BItem it = b_item(items, i);
-    const unsigned long long f = __ldcg(&cur[it.u]);
-    if (f == 0ull) continue;
-    for (uint32_t c = lane; c < it.cnt; c += 32) {
-      const size_t e = b_first_edge(it) + c;
-      const uint32_t dst = W == 1 ? (edges[e] & dmask) : edges[2 * e];
-      if ((__ldcg(&seen[dst]) & f) == f) continue;  // every query here has been there (a stale read only costs the atomic)
-      const unsigned long long fresh = f & ~atomicOr(&seen[dst], f);
-      if (fresh == 0ull) continue;
-      atomicOr(&next[dst], fresh);
-      for (unsigned long long m = fresh; m; m &= m - 1) dist[(size_t)dst * L + (__ffsll((long long)m) - 1)] = level;
-    }
-  }
-}
-
-template <int W, int L>
-__global__ void __launch_bounds__(kBThreads) k_b_bfs_relax(const BItem *__restrict__ items, const uint32_t *ctr,
-                                                           uint32_t cap, const uint32_t *__restrict__ edges,
-                                                           uint32_t pbits, uint32_t *dist,
-                                                           const unsigned long long *__restrict__ cur,
-                                                           unsigned long long *next, unsigned long long *seen) {
-  b_bfs_relax<W, L>(items, min(ctr[0], cap), ctr[2] + 1, edges, pbits, dist, cur, next, seen);
+__global__ void __launch_bounds__(kBThreads, SSSP ? kBSsspCtas : kBBfsCtas) k_b_relax(BState s, const uint32_t *ctr) {
+  __shared__ WarpExpand<BRow> s_exp[kBWarps];
+  const unsigned long long total = *reinterpret_cast<const unsigned long long *>(ctr);
+  if (SSSP) b_sssp_relax<W, L>(s, &s_exp[threadIdx.x >> 5], total);
+  else b_bfs_relax<W>(s, &s_exp[threadIdx.x >> 5], total);
 }
 
 // ---- persistent form -----------------------------------------------------------
 // One cooperative launch runs every iteration of a batch: frontier phase,
 // grid barrier, relaxation phase, grid barrier, and the loop test, all on the
-// device.  Counter words (ctr): [0..3] as in the graph loop (items, frontier,
-// iterations, error), [4..7] the items / frontier counts of even and odd
-// iterations (the next iteration's pair is cleared during the relaxation
-// phase), [8] barrier arrivals, [9] barrier generation.  A barrier waits at
+// device.  The counters of even and odd iterations alternate (the next
+// iteration's are cleared during the relaxation phase).  A barrier waits at
 // most wait_ns (GPU global timer); a block that gives up records error 4 and
 // returns, and every other block then gives up at its next barrier, so a lost
 // block ends the kernel with an error instead of a hang.
 struct BPersist {
-  uint32_t n, cap, chunk, pbits, max_iters, expect_blocks;
+  BState s;
+  uint32_t max_iters, expect_blocks;
   unsigned long long wait_ns;
-  const uint32_t *off, *edges;
-  const unsigned long long *obase;
-  uint32_t *dist, *ctr;
-  unsigned long long *cur, *next, *seen;
-  BItem *items;
+  uint32_t *ctr;
 };
 
 __device__ __forceinline__ unsigned long long b_now() {
@@ -329,23 +482,25 @@ __device__ bool b_grid_sync(const BPersist &a) {
 }
 
 template <bool SSSP, int W, int L>
-__global__ void __launch_bounds__(kBThreads) k_b_persist(BPersist a) {
+__global__ void __launch_bounds__(kBThreads, SSSP ? kBSsspCtas : kBBfsCtas) k_b_persist(BPersist a) {
+  __shared__ union {
+    BFrontierSmem frontier;
+    WarpExpand<BRow> exp[kBWarps];
+  } sm;
   for (uint32_t it = 0;; ++it) {
-    uint32_t *c = a.ctr + 4 + 2 * (it & 1u);
-    b_frontier(a.n, a.off, a.obase, a.cur, a.next, a.items, a.cap, c, a.chunk, a.ctr + 3);
+    unsigned long long *c = reinterpret_cast<unsigned long long *>(a.ctr + 4 + 2 * (it & 1u));
+    uint32_t *const act = a.ctr + 12 + (it & 1u);
+    b_frontier<SSSP, L>(a.s, sm.frontier, c, act, it);
     if (!b_grid_sync(a)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-      uint32_t *cn = a.ctr + 4 + 2 * ((it + 1) & 1u);
-      cn[0] = 0;
-      cn[1] = 0;
+      *reinterpret_cast<unsigned long long *>(a.ctr + 4 + 2 * ((it + 1) & 1u)) = 0ull;
+      a.ctr[12 + ((it + 1) & 1u)] = 0;
     }
-    const uint32_t nitems = min(*(volatile uint32_t *)c, a.cap);
-    if (SSSP) b_relax<true, W, L>(a.items, nitems, a.edges, a.pbits, a.dist, a.cur, a.next);
-    else b_bfs_relax<W, L>(a.items, nitems, it + 1, a.edges, a.pbits, a.dist, a.cur, a.next, a.seen);
+    const unsigned long long total = *(volatile unsigned long long *)c;
+    if (SSSP) b_sssp_relax<W, L>(a.s, &sm.exp[threadIdx.x >> 5], total);
+    else b_bfs_relax<W>(a.s, &sm.exp[threadIdx.x >> 5], total);
     if (!b_grid_sync(a)) return;
-    const uint32_t frontier = *(volatile uint32_t *)(c + 1);
-    const uint32_t err = *(volatile uint32_t *)(a.ctr + 3);
-    const bool more = frontier > 0 && err == 0;
+    const bool more = *(volatile uint32_t *)act > 0;
     if (!more || it + 1 >= a.max_iters) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.ctr[2] = it + 1;
@@ -358,10 +513,48 @@ __global__ void __launch_bounds__(kBThreads) k_b_persist(BPersist a) {
 
 __global__ void k_b_cond(cudaGraphConditionalHandle handle, uint32_t *ctr, uint32_t max_iters) {
   const uint32_t it = ++ctr[2];
-  uint32_t go = ctr[1] > 0 ? 1u : 0u;
+  uint32_t go = ctr[12] > 0 ? 1u : 0u;
   if (ctr[3]) go = 0;
   if (go && it >= max_iters) { ctr[3] = 2; go = 0; }
+  ctr[0] = ctr[1] = 0;  // the next iteration's counters
+  ctr[12] = 0;
   cudaGraphSetConditional(handle, go);
+}
+
+// BFS answers of vertices [v0, v0 + len): out[l * len + v - v0] = query l's
+// level, put together from the level planes (lane i of a warp holds vertex i's
+// words, so planes are read and answers written coalesced).  The traversal's
+// last iteration found no fresh query: levels are below ctr[2].
+template <int L, class OUT>
+__global__ void k_b_levels(BState s, uint32_t v0, uint32_t len, uint32_t nsrc, OUT *out, uint32_t *ctr) {
+  using T = typename BPlane<L>::T;
+  const T *const plane = reinterpret_cast<const T *>(s.dist);
+  const uint32_t planes = 32u - (uint32_t)__clz((int)(ctr[2] > 0 ? ctr[2] - 1 : 0));
+  constexpr uint32_t kInf = sizeof(OUT) == 2 ? 0xffffu : kBInf;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= len) return;
+  const uint32_t v = v0 + i;
+  const T seen = (T)s.mask[v].seen;
+  bool over = false;
+  if (planes <= 4) {
+    T p[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) p[k] = k < planes ? plane[(size_t)k * s.n + v] : (T)0;
+    for (uint32_t l = 0; l < nsrc; ++l) {
+      const uint32_t x = (uint32_t)((p[0] >> l) & 1) | (uint32_t)((p[1] >> l) & 1) << 1 |
+                         (uint32_t)((p[2] >> l) & 1) << 2 | (uint32_t)((p[3] >> l) & 1) << 3;
+      out[(size_t)l * len + i] = (OUT)((seen >> l) & 1 ? x : kInf);
+    }
+    return;
+  }
+  for (uint32_t l = 0; l < nsrc; ++l) {
+    uint32_t x = 0;
+    for (uint32_t k = 0; k < planes; ++k) x |= (uint32_t)((plane[(size_t)k * s.n + v] >> l) & 1) << k;
+    if (!((seen >> l) & 1)) x = kInf;
+    else if (sizeof(OUT) == 2 && x >= 0xffffu) { over = true; x = 0xfffeu; }
+    out[(size_t)l * len + i] = (OUT)x;
+  }
+  if (over) atomicExch(&ctr[10], 1u);
 }
 
 // out[l * n + v - v0] = dist[v * L + l] for v in [v0, v0 + len), l < nsrc.
@@ -415,14 +608,14 @@ struct sgw_batch {
   uint32_t n = 0, W = 1, pbits = 0;
   uint64_t m = 0;
   uint32_t lanes = 64;            // 32 or 64 distance columns
-  uint32_t chunk = 256;           // edges per work item
-  uint32_t items_cap = 0;
+  uint32_t min_units = 0;         // option: fewest work units of a warp's share (0: by algorithm)
   char *d_arena = nullptr;
   size_t arena_bytes = 0;
   uint32_t *d_off = nullptr, *d_edges = nullptr, *d_dist = nullptr, *d_stage = nullptr;
   unsigned long long *d_obase = nullptr;  // u64 node pointers: full pointer of every 1024th vertex
-  unsigned long long *d_cur = nullptr, *d_next = nullptr, *d_seen = nullptr;
-  BItem *d_items = nullptr;
+  unsigned long long *d_cur = nullptr;
+  BMask *d_mask = nullptr;
+  uint32_t *d_rows = nullptr, *d_unit = nullptr;
   uint32_t *d_ctr = nullptr, *d_src = nullptr;
   uint32_t stage_vertices = 0;
   uint32_t *h_ctr = nullptr;      // pinned
@@ -439,19 +632,32 @@ namespace {
 
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
+BState state_of(const sgw_batch *b, bool sssp) {
+  BState s;
+  s.n = b->n;
+  s.pbits = b->pbits;
+  s.off = b->d_off;
+  s.edges = b->d_edges;
+  s.obase = b->d_obase;
+  s.dist = b->d_dist;
+  s.cur = b->d_cur;
+  s.mask = b->d_mask;
+  s.rows = b->d_rows;
+  s.unit = b->d_unit;
+  // a warp's share is at least 128 edges of BFS (one round of its loads) and 16 of
+  // SSSP (two of its groups): a small frontier is spread over as many warps
+  s.min_units = b->min_units ? b->min_units : sssp ? 2u : 16u;
+  return s;
+}
+
 template <bool SSSP, int W, int L>
 int capture_body(sgw_batch *b, cudaGraph_t body, cudaGraphConditionalHandle h) {
   CK(cudaStreamBeginCaptureToGraph(b->s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  k_b_reset<<<1, 1, 0, b->s>>>(b->d_ctr);
+  const BState s = state_of(b, SSSP);
+  const uint32_t tiles = (b->n + kBVerts - 1) / kBVerts;
   const uint32_t grid = (uint32_t)b->num_sms * 8;
-  k_b_frontier<<<grid, kBThreads, 0, b->s>>>(b->n, b->d_off, b->d_obase, b->d_cur, b->d_next, b->d_items, b->items_cap,
-                                             b->d_ctr, b->chunk);
-  if (SSSP)
-    k_b_relax<SSSP, W, L><<<grid, kBThreads, 0, b->s>>>(b->d_items, b->d_ctr, b->items_cap, b->d_edges, b->pbits,
-                                                        b->d_dist, b->d_cur, b->d_next);
-  else
-    k_b_bfs_relax<W, L><<<grid, kBThreads, 0, b->s>>>(b->d_items, b->d_ctr, b->items_cap, b->d_edges, b->pbits,
-                                                      b->d_dist, b->d_cur, b->d_next, b->d_seen);
+  k_b_frontier<SSSP, L><<<std::min(tiles, grid), kBThreads, 0, b->s>>>(s, b->d_ctr);
+  k_b_relax<SSSP, W, L><<<grid, kBThreads, 0, b->s>>>(s, b->d_ctr);
   k_b_cond<<<1, 1, 0, b->s>>>(h, b->d_ctr, b->max_iters);
   cudaGraph_t out = nullptr;
   CK(cudaStreamEndCapture(b->s, &out));
@@ -496,22 +702,11 @@ int launch_persist_t(sgw_batch *b, uint32_t extra_blocks, unsigned long long wai
   if (per_sm < 1) return sgw::fail(SGW_ECUDA, "persistent batch kernel does not fit on an SM");
   const uint32_t grid = (uint32_t)b->num_sms * (uint32_t)std::min(per_sm, 8);
   BPersist a;
-  a.n = b->n;
-  a.cap = b->items_cap;
-  a.chunk = b->chunk;
-  a.pbits = b->pbits;
+  a.s = state_of(b, SSSP);
   a.max_iters = b->max_iters;
   a.expect_blocks = grid + extra_blocks;
   a.wait_ns = wait_ns;
-  a.off = b->d_off;
-  a.obase = b->d_obase;
-  a.edges = b->d_edges;
-  a.dist = b->d_dist;
   a.ctr = b->d_ctr;
-  a.cur = b->d_cur;
-  a.next = b->d_next;
-  a.seen = b->d_seen;
-  a.items = b->d_items;
   void *args[] = {&a};
   CK(cudaLaunchCooperativeKernel((const void *)k_b_persist<SSSP, W, L>, dim3(grid), dim3(kBThreads), args, 0,
                                  b->s));
@@ -571,7 +766,7 @@ int sgw_batch_create(const sgw_graph *g, const sgw_engine_opts *opts, uint32_t l
   b->n = g->n;
   b->m = g->m;
   b->lanes = lanes;
-  b->chunk = o.chunk_edges ? o.chunk_edges : 256;
+  b->min_units = o.chunk_edges ? std::max<uint32_t>(1, o.chunk_edges / kBUnit) : 0;
   if ((o.flags & SGW_OPT_BATCH_PERSISTENT) && (o.flags & SGW_OPT_BATCH_GRAPH)) {
     delete b;
     return sgw::fail(SGW_EINVAL, "SGW_OPT_BATCH_PERSISTENT and SGW_OPT_BATCH_GRAPH exclude each other");
@@ -600,12 +795,11 @@ int sgw_batch_create(const sgw_graph *g, const sgw_engine_opts *opts, uint32_t l
     b->W = 1;
     src_edges = packed;
   }
-  b->items_cap = (uint32_t)std::min<uint64_t>((uint64_t)g->m / b->chunk + g->n + 64, 0xffffffffull);
   b->stage_vertices = std::min<uint32_t>(g->n, 1u << 22);
   const bool wide = g->node_pointer64 != nullptr;
   const size_t nbase = (g->n >> sgw::kOffGroupLog2) + 2;
   const size_t need = al(4ull * (g->n + 1)) + (wide ? al(8 * nbase) : 0) + al((size_t)g->m * 4 * b->W) + al((size_t)g->n * lanes * 4) +
-                      3 * al(8ull * g->n) + al(sizeof(BItem) * (size_t)b->items_cap) + al(64) + al(256) +
+                      al(8ull * g->n) + al(sizeof(BMask) * (size_t)g->n) + 2 * al(4ull * g->n) + al(64) + al(256) +
                       al((size_t)b->stage_vertices * lanes * 4);
   if (o.budget_bytes && need > o.budget_bytes) {
     sgw::host_free(packed);
@@ -623,9 +817,9 @@ int sgw_batch_create(const sgw_graph *g, const sgw_engine_opts *opts, uint32_t l
   b->d_edges = (uint32_t *)take((size_t)g->m * 4 * b->W);
   b->d_dist = (uint32_t *)take((size_t)g->n * lanes * 4);
   b->d_cur = (unsigned long long *)take(8ull * g->n);
-  b->d_next = (unsigned long long *)take(8ull * g->n);
-  b->d_seen = (unsigned long long *)take(8ull * g->n);
-  b->d_items = (BItem *)take(sizeof(BItem) * (size_t)b->items_cap);
+  b->d_mask = (BMask *)take(sizeof(BMask) * (size_t)g->n);
+  b->d_rows = (uint32_t *)take(4ull * g->n);
+  b->d_unit = (uint32_t *)take(4ull * g->n);
   b->d_ctr = (uint32_t *)take(64);
   b->d_src = (uint32_t *)take(256);
   b->d_stage = (uint32_t *)take((size_t)b->stage_vertices * lanes * 4);
@@ -729,16 +923,25 @@ int batch_run(sgw_batch *b, int algo, const uint32_t *sources, uint32_t nsrc, vo
   const auto w0 = std::chrono::steady_clock::now();
   CK(cudaMemcpyAsync(b->d_src, sources, 4ull * nsrc, cudaMemcpyHostToDevice, b->s));
   CK(cudaEventRecord(b->t0, b->s));
-  const size_t cells = (size_t)b->n * b->lanes;
-  k_b_fill<<<b->num_sms * 8, 256, 0, b->s>>>(b->d_dist, cells, b->d_next, b->d_seen, b->n);
-  if (b->lanes == 64) k_b_seed<64><<<1, 64, 0, b->s>>>(b->d_src, nsrc, b->d_dist, b->d_next, b->d_seen, b->d_ctr);
-  else k_b_seed<32><<<1, 64, 0, b->s>>>(b->d_src, nsrc, b->d_dist, b->d_next, b->d_seen, b->d_ctr);
+  const bool sssp = algo == SGW_SSSP;
+  const uint32_t fill = (uint32_t)b->num_sms * 8;
+  if (b->lanes == 64) {
+    if (sssp) k_b_fill<64, true><<<fill, 256, 0, b->s>>>(b->d_dist, b->d_mask, b->n);
+    else k_b_fill<64, false><<<fill, 256, 0, b->s>>>(b->d_dist, b->d_mask, b->n);
+    if (sssp) k_b_seed<64, true><<<1, 64, 0, b->s>>>(b->d_src, nsrc, b->d_dist, b->d_mask, b->d_ctr);
+    else k_b_seed<64, false><<<1, 64, 0, b->s>>>(b->d_src, nsrc, b->d_dist, b->d_mask, b->d_ctr);
+  } else {
+    if (sssp) k_b_fill<32, true><<<fill, 256, 0, b->s>>>(b->d_dist, b->d_mask, b->n);
+    else k_b_fill<32, false><<<fill, 256, 0, b->s>>>(b->d_dist, b->d_mask, b->n);
+    if (sssp) k_b_seed<32, true><<<1, 64, 0, b->s>>>(b->d_src, nsrc, b->d_dist, b->d_mask, b->d_ctr);
+    else k_b_seed<32, false><<<1, 64, 0, b->s>>>(b->d_src, nsrc, b->d_dist, b->d_mask, b->d_ctr);
+  }
   CK(cudaGetLastError());
   if (persistent) {
-    const int st = launch_persist(b, algo == SGW_SSSP, extra_blocks, wait_ns);
+    const int st = launch_persist(b, sssp, extra_blocks, wait_ns);
     if (st != SGW_OK) return st;
   } else {
-    CK(cudaGraphLaunch(b->exec[algo == SGW_SSSP ? 1 : 0], b->s));
+    CK(cudaGraphLaunch(b->exec[sssp ? 1 : 0], b->s));
   }
   CK(cudaEventRecord(b->t1, b->s));
   // lane-major results, staged through a transposed device tile
@@ -748,7 +951,17 @@ int batch_run(sgw_batch *b, int algo, const uint32_t *sources, uint32_t nsrc, vo
     const uint32_t len = std::min(b->stage_vertices, b->n - v0);
     const uint32_t blocks = (len + 31) / 32;
     uint16_t *st16 = reinterpret_cast<uint16_t *>(b->d_stage);
-    if (ab == 2) {
+    if (!sssp) {
+      const BState s = state_of(b, false);
+      const uint32_t lb = (len + 255) / 256;
+      if (ab == 2) {
+        if (b->lanes == 64) k_b_levels<64, uint16_t><<<lb, 256, 0, b->s>>>(s, v0, len, nsrc, st16, b->d_ctr);
+        else k_b_levels<32, uint16_t><<<lb, 256, 0, b->s>>>(s, v0, len, nsrc, st16, b->d_ctr);
+      } else {
+        if (b->lanes == 64) k_b_levels<64, uint32_t><<<lb, 256, 0, b->s>>>(s, v0, len, nsrc, b->d_stage, b->d_ctr);
+        else k_b_levels<32, uint32_t><<<lb, 256, 0, b->s>>>(s, v0, len, nsrc, b->d_stage, b->d_ctr);
+      }
+    } else if (ab == 2) {
       if (b->lanes == 64) k_b_transpose16<64><<<blocks, 256, 0, b->s>>>(b->d_dist, v0, len, nsrc, st16, b->d_ctr + 10);
       else k_b_transpose16<32><<<blocks, 256, 0, b->s>>>(b->d_dist, v0, len, nsrc, st16, b->d_ctr + 10);
     } else {
@@ -761,7 +974,6 @@ int batch_run(sgw_batch *b, int algo, const uint32_t *sources, uint32_t nsrc, vo
   }
   CK(cudaMemcpyAsync(b->h_ctr, b->d_ctr, 64, cudaMemcpyDeviceToHost, b->s));
   CK(cudaStreamSynchronize(b->s));
-  if (b->h_ctr[3] == 1) return sgw::fail(SGW_ERANGE, "work item list overflow");
   if (b->h_ctr[3] == 2) return sgw::fail(SGW_ETIMEOUT, "iteration limit reached");
   if (b->h_ctr[3] == 4) return sgw::fail(SGW_ETIMEOUT, "grid barrier wait timed out");
   if (b->h_ctr[10]) return sgw::fail(SGW_ERANGE, "a distance does not fit 16 bits: use sgw_batch_run");
