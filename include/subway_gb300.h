@@ -514,9 +514,10 @@ int sgw_batch_results(const sgw_batch *b, const uint32_t **results);
  * every byte of device memory through its own pool.  It runs the engine's activeness -> scan -> compaction kernel on
  * device arrays the caller provides (label1, label2 bytes of n vertices;
  * node_pointer of n+1 entries; queue of n and ptr of n+1 entries), with the
- * scan's tile state in a static device array inside this library
- * (about 321 KB, held by every GPU that loads the library until exit).  It
- * calls no allocating routine.
+ * running totals in a static device array inside this library
+ * (about 33 KB, held by every GPU that loads the library until exit).  It
+ * calls no allocating routine.  Arrays that start on 16-byte boundaries are
+ * read as 16-byte words.
  *  - n must be at most SGW_NOALLOC_MAX_VERTICES; larger n returns SGW_ERANGE.
  *  - consume != 0 clears the labels of queued vertices (the sync form);
  *    labels of active vertices with no out-edges are always cleared.

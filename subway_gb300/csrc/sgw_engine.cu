@@ -86,9 +86,9 @@ struct sgw_engine {
   uint32_t range_inner_cap = 0;  // learned policy: inner-iteration cap of the running range
   uint64_t hub_iters = 0;        // single-vertex partitions relaxed (counted on the host)
   uint32_t *d_queue = nullptr, *d_ptr = nullptr;
-  uint32_t *d_tflag = nullptr;
   uint32_t *d_gmask = nullptr;             // generate: keep | clear bits per 16-vertex group
-  unsigned long long *d_tagg = nullptr, *d_tincl = nullptr;
+  unsigned long long *d_tagg = nullptr;    // generate: per-tile totals
+  GenTotals *d_runs = nullptr;             // and those of each CTA's run of tiles
   Ctl *d_ctl = nullptr;
   Part *d_parts = nullptr;
   WorkItem *d_wl = nullptr;
@@ -131,7 +131,6 @@ struct sgw_engine {
   cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
   std::vector<ProfEvent> prof;
   size_t prof_used = 0;
-  uint32_t epoch = 0;
 
   // run state
   sgw_run_params params{};
@@ -214,10 +213,8 @@ int prof_collect(sgw_engine *e) {
 int check_ctl_error(sgw_engine *e) {
   uint32_t err = e->h_ctl->error;
   if (err == 0) return SGW_OK;
-  if (err == 1) return fail(SGW_ETIMEOUT, "scan look-back wait timed out");
   if (err == 2) return fail(SGW_ERANGE, "partition table overflow");
   if (err == 3) return fail(SGW_ERANGE, "chunk list overflow");
-  if (err == 4) return fail(SGW_ESTATE, "scan ticket counter out of step");
   return fail(SGW_ECUDA, "device error code %u", err);
 }
 
@@ -400,8 +397,10 @@ int read_ctl(sgw_engine *e) {
 // followed by the partition table, the chunk list and the edge buffers.
 enum Family { FAM_INT = 0, FAM_PR = 1 };
 
+constexpr uint32_t kGenMaxRuns = 2048;  // CTAs of a generate
+
 struct Layout {
-  size_t off, obase, tflag, tagg, tincl, ctl, mlp, sel, gmask, hct;  // common
+  size_t off, obase, tagg, runs, ctl, mlp, sel, gmask, hct;  // common
   size_t value, l1, l2, queue, ptr, delta, qpush;     // family
   size_t parts, ranges, rstat, wl, buf[kMaxBuf], total;
   uint64_t cap;
@@ -415,9 +414,8 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
   auto take = [&](size_t bytes) { size_t at = p; p += align_up(bytes, 256); return at; };
   L.off = take(4ull * (n + 1));
   L.obase = take(wide ? 8ull * ((n >> kOffGroupLog2) + 2) : 0);
-  L.tflag = take(4ull * num_tiles);
   L.tagg = take(8ull * num_tiles);
-  L.tincl = take(8ull * num_tiles);
+  L.runs = take(sizeof(GenTotals) * std::min(num_tiles, kGenMaxRuns));
   L.ctl = take(sizeof(Ctl));
   L.mlp = take(sizeof(__nv_bfloat16) * kMlpParams);
   L.sel = take(sizeof(unsigned long long) * kSelBins);
@@ -479,9 +477,8 @@ int carve(sgw_engine *e, int fam, uint64_t cap) {
   char *b = e->d_arena;
   e->d_off = (uint32_t *)(b + L.off);
   e->d_obase = (unsigned long long *)(b + L.obase);
-  e->d_tflag = (uint32_t *)(b + L.tflag);
   e->d_tagg = (unsigned long long *)(b + L.tagg);
-  e->d_tincl = (unsigned long long *)(b + L.tincl);
+  e->d_runs = (GenTotals *)(b + L.runs);
   e->d_ctl = (Ctl *)(b + L.ctl);
   e->d_gmask = (uint32_t *)(b + L.gmask);
   e->d_hct = (unsigned long long *)(b + L.hct);
@@ -579,7 +576,15 @@ int launch_select(sgw_engine *e) {
   return SGW_OK;
 }
 
-int launch_generate(sgw_engine *e, int consume) {
+// Cuts a generate's tiles into one run per CTA; returns the grid.
+uint32_t cut_tiles(GenArgs &a, int num_sms, int ctas_per_sm) {
+  const uint32_t max_runs = std::min<uint32_t>((uint32_t)num_sms * ctas_per_sm, kGenMaxRuns);
+  a.run_tiles = (a.num_tiles + max_runs - 1) / max_runs;
+  return (a.num_tiles + a.run_tiles - 1) / a.run_tiles;
+}
+
+// plan: the partition plan is made by the same launches.
+int launch_generate(sgw_engine *e, int consume, bool plan) {
   GenArgs a;
   a.n = e->n;
   a.l1 = e->d_l1;
@@ -587,14 +592,16 @@ int launch_generate(sgw_engine *e, int consume) {
   a.off = e->d_off;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
-  a.tflag = e->d_tflag;
   a.tagg = e->d_tagg;
-  a.tincl = e->d_tincl;
+  a.runs = e->d_runs;
   a.ctl = e->d_ctl;
   a.gmask = e->d_gmask;
-  e->epoch = (e->epoch + 1) & 0x3fffffffu;
-  if (e->epoch == 0) e->epoch = 1;
-  a.epoch = e->epoch;
+  a.aligned = 1;
+  if (plan) {
+    a.parts = e->d_parts;
+    a.max_parts = e->max_parts;
+    a.cap = (unsigned long long)e->cap;
+  }
   a.num_tiles = e->num_tiles;
   a.consume = consume;
   a.edge_limit = e->edge_limit;
@@ -616,17 +623,16 @@ int launch_generate(sgw_engine *e, int consume) {
       TRY(launch_select(e));
     }
   }
-  CK(cudaMemsetAsync(&e->d_ctl->max_degree, 0, sizeof(uint32_t), e->s_comp));
   size_t slot = 0;
   TRY(prof_begin(e, K_GENERATE, e->s_comp, &slot));
-  if (e->fam == FAM_PR) k_generate_count<true><<<e->num_tiles, kGenThreads, 0, e->s_comp>>>(a);
-  else k_generate_count<false><<<e->num_tiles, kGenThreads, 0, e->s_comp>>>(a);
+  const uint32_t grid = cut_tiles(a, e->num_sms, e->fam == FAM_PR ? 2 : kGenCtas);
+  if (e->fam == FAM_PR) k_generate_count_pr<<<grid, kGenPrThreads, 0, e->s_comp>>>(a);
+  else if (a.sel_mode) k_generate_count<true><<<grid, kGenThreads, 0, e->s_comp>>>(a);
+  else k_generate_count<false><<<grid, kGenThreads, 0, e->s_comp>>>(a);
   CK(cudaGetLastError());
-  k_generate_scan<<<1, kGenScanThreads, 0, e->s_comp>>>(a);
-  CK(cudaGetLastError());
-  if (e->fam == FAM_PR) k_generate_write<true><<<e->num_tiles, kGenThreads, 0, e->s_comp>>>(a);
-  else k_generate_write<false><<<e->num_tiles, kGenThreads, 0, e->s_comp>>>(a);
-  e->stats.launches += 3;
+  if (e->fam == FAM_PR) k_generate_write_pr<<<grid, kGenPrThreads, 0, e->s_comp>>>(a);
+  else k_generate_write<true><<<grid, kGenThreads, 0, e->s_comp>>>(a);
+  e->stats.launches += 2;
   CK(cudaGetLastError());
   TRY(prof_end(e, e->s_comp, slot));
   e->stats.generate_launches += 1;
@@ -639,7 +645,7 @@ int launch_generate(sgw_engine *e, int consume) {
 int launch_plan(sgw_engine *e) {
   size_t slot = 0;
   TRY(prof_begin(e, K_PLAN, e->s_comp, &slot));
-  k_plan<<<1, 32, 0, e->s_comp>>>(e->d_ptr, e->d_queue, e->d_ctl, e->d_parts, e->max_parts,
+  k_plan<<<1, kGenThreads, 0, e->s_comp>>>(e->d_ptr, e->d_queue, e->d_ctl, e->d_parts, e->max_parts,
                                    (unsigned long long)e->cap);
   CK(cudaGetLastError());
   TRY(prof_end(e, e->s_comp, slot));
@@ -647,24 +653,29 @@ int launch_plan(sgw_engine *e) {
   return SGW_OK;
 }
 
+// The control block and the partition table behind the queued launches: one
+// read-back, a second only for a table longer than the block carries.
+int read_plan(sgw_engine *e) {
+  TRY(read_ctl(e));
+  e->num_parts = e->h_ctl->num_parts;
+  if (e->num_parts > kCtlParts) {
+    CK(cudaMemcpyAsync(e->h_parts, e->d_parts, sizeof(Part) * e->num_parts, cudaMemcpyDeviceToHost, e->s_comp));
+    CK(cudaStreamSynchronize(e->s_comp));
+    e->stats.d2h_bytes += sizeof(Part) * e->num_parts;
+  } else {
+    memcpy(e->h_parts, e->h_ctl->first, sizeof(Part) * e->num_parts);
+  }
+  e->parts_valid = true;
+  return SGW_OK;
+}
+
 // generate + plan + one read-back: the per-global-iteration host sync.
 int generate_and_plan(sgw_engine *e, int consume) {
-  TRY(launch_generate(e, consume));
-  TRY(launch_plan(e));
-  CK(cudaMemcpyAsync(e->h_ctl, e->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, e->s_comp));
-  CK(cudaStreamSynchronize(e->s_comp));
-  TRY(check_ctl_error(e));
+  TRY(launch_generate(e, consume, true));
+  TRY(read_plan(e));
   e->num_active = e->h_ctl->num_active;
   e->num_active_edges = e->h_ctl->num_active_edges;
   e->max_degree = e->h_ctl->max_degree;
-  e->num_parts = e->h_ctl->num_parts;
-  if (e->num_parts > 0) {
-    CK(cudaMemcpyAsync(e->h_parts, e->d_parts, sizeof(Part) * e->num_parts,
-                       cudaMemcpyDeviceToHost, e->s_comp));
-    CK(cudaStreamSynchronize(e->s_comp));
-  }
-  e->stats.d2h_bytes += sizeof(Ctl) + sizeof(Part) * e->num_parts;
-  e->parts_valid = true;
   return SGW_OK;
 }
 
@@ -1152,7 +1163,7 @@ int process_iteration(sgw_engine *e) {
 // ---- learned policy ------------------------------------------------------------
 // generate + per-range statistics and predictions + one read-back.
 int generate_and_stats(sgw_engine *e, int consume) {
-  TRY(launch_generate(e, consume));
+  TRY(launch_generate(e, consume, false));
   const uint32_t S = (uint32_t)e->ranges.size();
   const __nv_bfloat16 *w = e->have_model ? e->d_mlp : nullptr;
   size_t slot = 0;
@@ -1615,7 +1626,7 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   }
   e->arena_bytes = arena;
   carve(e, FAM_INT, e->cap_fam[FAM_INT]);
-  uint32_t parts_host = 0;
+  uint32_t parts_host = kCtlParts;
   for (int fam = 0; fam < 2; ++fam)
     if (e->cap_fam[fam])
       parts_host = std::max(parts_host, make_layout(fam, e->n, e->m, esz, e->nbuf, e->num_tiles,
@@ -1724,7 +1735,6 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
     if (ce == cudaSuccess) ce = cudaMemcpy(e->d_obase, base.data(), 8 * base.size(), cudaMemcpyHostToDevice);
   }
   if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_ctl, 0, sizeof(Ctl), e->s_comp);
-  if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_tflag, 0, 4ull * e->num_tiles, e->s_comp);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->s_comp);
   if (ce != cudaSuccess) return cleanup(fail(SGW_ECUDA, "engine setup copies: %s", cudaGetErrorString(ce)));
   st = probe_stream_dma(e);
@@ -1785,7 +1795,7 @@ int sgw_generate(sgw_engine *e, uint32_t *num_active_nodes, uint64_t *num_active
   clear_error();
   if (!e || !e->initialized) return fail(SGW_ESTATE, "engine not initialised");
   CK(cudaSetDevice(e->device));
-  TRY(launch_generate(e, e->params.mode == SGW_SYNC ? 1 : 0));
+  TRY(launch_generate(e, e->params.mode == SGW_SYNC ? 1 : 0, false));
   TRY(read_ctl(e));
   e->num_active = e->h_ctl->num_active;
   e->num_active_edges = e->h_ctl->num_active_edges;
@@ -1800,13 +1810,7 @@ int sgw_partition(sgw_engine *e, uint32_t *num_partitions) {
   if (!e || !e->initialized) return fail(SGW_ESTATE, "engine not initialised");
   CK(cudaSetDevice(e->device));
   TRY(launch_plan(e));
-  TRY(read_ctl(e));
-  e->num_parts = e->h_ctl->num_parts;
-  if (e->num_parts) {
-    CK(cudaMemcpyAsync(e->h_parts, e->d_parts, sizeof(Part) * e->num_parts, cudaMemcpyDeviceToHost, e->s_comp));
-    CK(cudaStreamSynchronize(e->s_comp));
-  }
-  e->parts_valid = true;
+  TRY(read_plan(e));
   if (num_partitions) *num_partitions = e->num_parts;
   return SGW_OK;
 }
@@ -2028,31 +2032,27 @@ int sgw_run(sgw_engine *e, const sgw_run_params *p, void *out_values, sgw_run_st
 }  // extern "C"
 
 // ---- allocation-free compaction ---------------------------------------------
-// sgw_generate_noalloc runs the single-pass generate kernel (k_generate, one
-// launch, decoupled look-back) on caller-owned device arrays, with the scan's tile state and counters in the
-// file-scope array below instead of an engine arena.  Nothing here allocates.
+// sgw_generate_noalloc runs the generate kernels on caller-owned device arrays,
+// with the tile totals and counters in the file-scope array below instead of
+// an engine arena.  Nothing here allocates.
 //
-// Limit: SGW_NOALLOC_MAX_VERTICES vertices = 16384 scan tiles of 4096.
-// Size: 16384 x (4 B flag + 8 B aggregate + 8 B inclusive prefix) plus the
-// control block, about 321 KB, held by every GPU that loads the library.
+// Limit: SGW_NOALLOC_MAX_VERTICES vertices (documented; earlier forms kept per-
+// tile state).  Size: the runs' totals and the control block, about 33 KB,
+// held by every GPU that loads the library.
 
 #include <mutex>
 
 namespace {
 
-constexpr uint32_t kNoAllocTiles = SGW_NOALLOC_MAX_VERTICES / kGenTile;
-constexpr size_t kNaFlagOff = 0;
-constexpr size_t kNaAggOff = kNaFlagOff + 4ull * kNoAllocTiles;
-constexpr size_t kNaInclOff = kNaAggOff + 8ull * kNoAllocTiles;
-constexpr size_t kNaCtlOff = kNaInclOff + 8ull * kNoAllocTiles;
-constexpr size_t kNoAllocBytes = kNaCtlOff + ((sizeof(Ctl) + 255) / 256) * 256;
+constexpr size_t kNaRunsOff = 0;
+constexpr size_t kNaCtlOff = kNaRunsOff + sizeof(GenTotals) * kGenMaxRuns;
+constexpr size_t kNoAllocBytes = kNaCtlOff + sizeof(Ctl);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
 unsigned char *g_noalloc_ptr[kNoAllocMaxDevices] = {};  // device address per device
-uint32_t g_noalloc_epoch[kNoAllocMaxDevices] = {};
 
 }  // namespace
 
@@ -2070,7 +2070,8 @@ extern "C" int sgw_generate_noalloc(uint8_t *d_label1, uint8_t *d_label2,
   CK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kNoAllocMaxDevices) return fail(SGW_ERANGE, "device %d", dev);
   unsigned char *scratch = nullptr;
-  uint32_t epoch = 0;
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   {
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     if (!g_noalloc_ptr[dev]) {  // once per device, with that device current
@@ -2083,8 +2084,6 @@ extern "C" int sgw_generate_noalloc(uint8_t *d_label1, uint8_t *d_label2,
       g_noalloc_ptr[dev] = static_cast<unsigned char *>(p);
     }
     scratch = g_noalloc_ptr[dev];
-    epoch = g_noalloc_epoch[dev] = (g_noalloc_epoch[dev] + 1) & 0x3fffffffu;
-    if (epoch == 0) epoch = g_noalloc_epoch[dev] = 1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Ctl *ctl = reinterpret_cast<Ctl *>(scratch + kNaCtlOff);
@@ -2097,23 +2096,25 @@ extern "C" int sgw_generate_noalloc(uint8_t *d_label1, uint8_t *d_label2,
   a.off = d_node_pointer;
   a.queue = d_queue;
   a.ptr = d_ptr;
-  a.tflag = reinterpret_cast<uint32_t *>(scratch + kNaFlagOff);
-  a.tagg = reinterpret_cast<unsigned long long *>(scratch + kNaAggOff);
-  a.tincl = reinterpret_cast<unsigned long long *>(scratch + kNaInclOff);
+  a.tagg = nullptr;  // no edge limit
+  a.runs = reinterpret_cast<GenTotals *>(scratch + kNaRunsOff);
   a.ctl = ctl;
   a.gmask = nullptr;
-  a.epoch = epoch;
+  // a caller's arrays may start anywhere: 16-byte words only where all three allow them
+  a.aligned = ((reinterpret_cast<uintptr_t>(d_label1) | reinterpret_cast<uintptr_t>(d_label2) |
+                reinterpret_cast<uintptr_t>(d_node_pointer)) & 15u) == 0;
   a.num_tiles = (n + kGenTile - 1) / kGenTile;
   a.consume = consume ? 1 : 0;
   a.delta = a.pval = a.qpush = nullptr;
   a.acc = a.damping = 0.0;
-  k_generate<<<a.num_tiles, kGenThreads, 0, s>>>(a);
+  const uint32_t grid = cut_tiles(a, sms, kGenCtas);
+  k_generate_count<false><<<grid, kGenThreads, 0, s>>>(a);
+  CK(cudaGetLastError());
+  k_generate_write<false><<<grid, kGenThreads, 0, s>>>(a);
   CK(cudaGetLastError());
   Ctl h;
-  CK(cudaMemcpyAsync(&h, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&h, ctl, offsetof(Ctl, num_parts), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  if (h.error == 1) return fail(SGW_ETIMEOUT, "scan look-back wait timed out");
-  if (h.error) return fail(SGW_ESTATE, "scan error %u", h.error);
   if (num_active) *num_active = h.num_active;
   if (num_active_edges) *num_active_edges = h.num_active_edges;
   return SGW_OK;

@@ -2,20 +2,23 @@
 //
 // Hot path per global iteration (reference: shared/subgraph_generator.cu:
 // 128-204 and subway/*-{sync,async}.cu):
-//   k_generate_count / _scan / _write (BFS, SSSP, SSWP, CC) and k_generate
-//                (PageRank; single-pass decoupled-lookback scan): activeness,
+//   k_generate_count / k_generate_write (_pr: PageRank) activeness,
 //                scan and compaction into the active queue (replaces
 //                prePrefix, thrust::reduce, two thrust::exclusive_scan,
-//                makeQueue, makeActiveNodesPointer)
-//   k_plan       greedy partition boundaries on the device (Partitioner)
+//                makeQueue, makeActiveNodesPointer), and the greedy partition
+//                boundaries (Partitioner); k_plan: the boundaries on their own
 //   k_gather_v   active-edge gather from the engine's mapped pinned transfer
 //                copy of the edges into an HBM edge buffer, 16-byte reads
 //                (replaces the host std::thread copy dynamic<E>); k_gather
 //                is the one-record-per-thread form
-//   k_relax_warp warp-cooperative expansion of 32 frontier sources at a time
-//                (bfs/sssp/sswp/cc kernels, sync and async forms); k_relax_tile
+//   k_relax_all  a first pass over a queue whose every source is active, cut by
+//                edges; sync passes read the host copy themselves
+//                (bfs/sssp/sswp/cc kernels, sync and async forms)
+//   k_relax_warp label-driven expansion of 32 sources at a time by a warp
+//                (later async inner iterations); k_relax_tile
 //                the CTA-tile form staged in shared memory
 //   k_relax_chunks warp-per-chunk expansion of high-degree sources
+//   k_pr_all, k_pr_claim, k_pr_warp the same for PageRank
 // Learned policy only (no reference counterpart):
 //   k_select_*   value range, degree histogram and cut of the frontier when
 //                far vertices are deferred
@@ -36,14 +39,23 @@ namespace sgw {
 constexpr uint32_t kInf = 4294967294u;  // DIST_INFINITY (shared/globals.hpp:27)
 
 // ---- device control block -------------------------------------------------
+struct Part {                // one partition of the active queue
+  uint32_t from;             // first queue index
+  uint32_t size;             // queue entries
+  uint32_t edge_from;        // ptr[from]
+  uint32_t first_vertex;     // queue[from]
+  unsigned long long edge_count;
+};
+constexpr uint32_t kCtlParts = 16;  // partitions reported with the control block
+
 struct Ctl {
-  uint32_t tile_ticket;      // dynamic tile index of the running scan
-  uint32_t tile_done;        // finished tiles of the running scan
-  uint32_t error;            // nonzero: a bounded wait gave up
+  uint32_t tile_done;        // finished tiles of the running generate
+  uint32_t degree_max;       // largest degree queued so far by the running generate
+  uint32_t error;            // nonzero: a device-side check failed
   uint32_t num_active;       // queued vertices (degree > 0) of the last generate
   unsigned long long num_active_edges;
   uint32_t num_parts;        // partitions of the last plan
-  uint32_t max_degree;       // largest degree queued by the last generate (engine form)
+  uint32_t max_degree;       // largest degree queued by the last generate
   uint32_t upd[4];           // async inner iteration k: relaxations that improved
   uint32_t wl_count[4];      // chunk-list items of inner iteration k
   uint32_t iters_run;        // inner iterations that did work
@@ -55,14 +67,7 @@ struct Ctl {
   unsigned long long relaxed_edges;
   unsigned long long relaxed_sources;
   double hub_push;           // single-vertex PR partition: its push value
-};
-
-struct Part {                // one partition of the active queue
-  uint32_t from;             // first queue index
-  uint32_t size;             // queue entries
-  uint32_t edge_from;        // ptr[from]
-  uint32_t first_vertex;     // queue[from]
-  unsigned long long edge_count;
+  Part first[kCtlParts];     // the partition table's first entries
 };
 
 struct WorkItem {            // a chunk of one high-degree source's edges
@@ -78,17 +83,6 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_u32(uint32_t *p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 // First index in a[0, n) whose value is >= x (a sorted ascending).
 __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t n, uint32_t x) {
   uint32_t lo = 0, hi = n;
@@ -99,98 +93,14 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t 
   return lo;
 }
 
-// Bounded wait on a scan tile flag; returns the flag, or 0 after the limit
-// (and records the error).  Flags are (epoch << 2) | status, status 1 =
-// aggregate available, 2 = inclusive prefix available.
-constexpr uint32_t kSpinLimit = 1u << 22;
-__device__ __forceinline__ uint32_t wait_tile_flag(const uint32_t *flag, uint32_t epoch, Ctl *ctl) {
-  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-    uint32_t f = ld_acquire_u32(flag);
-    if ((f >> 2) == epoch && (f & 3u) != 0) return f;
-    __nanosleep(spin < 64 ? 32 : 256);
-  }
-  atomicExch(&ctl->error, 1u);
-  return 0;
-}
-
-// Decoupled look-back for tile `tile` with aggregate `agg`, run by a whole
-// warp.  Values are packed (count << 32) | edges; both sums stay below 2^32
-// so the packed add never carries.  Lane k examines predecessors
-// tile - 1 - (kLookPer k + q) - 32 kLookPer r, q < kLookPer, so one round
-// covers 32 kLookPer predecessors; the sum stops at the nearest predecessor
-// whose inclusive prefix is published.  One per lane measured best: with 4
-// per lane (128 per round) a tile waits on more unpublished neighbours and
-// the scan ran 30-40% longer.  Called by all lanes of one warp; returns the
-// exclusive prefix on every lane.
-constexpr int kLookPer = 1;
-__device__ __forceinline__ unsigned long long lookback_warp(
-    uint32_t tile, unsigned long long agg, uint32_t *tflag, unsigned long long *tagg,
-    unsigned long long *tincl, uint32_t epoch, Ctl *ctl, int lane) {
-  if (tile == 0) {
-    if (lane == 0) {
-      st_relaxed_u64(&tincl[0], agg);
-      st_release_u32(&tflag[0], (epoch << 2) | 2u);
-    }
-    return 0ull;
-  }
-  if (lane == 0) {
-    st_relaxed_u64(&tagg[tile], agg);
-    st_release_u32(&tflag[tile], (epoch << 2) | 1u);
-  }
-  unsigned long long excl = 0;
-  for (int32_t base = (int32_t)tile - 1;; base -= 32 * kLookPer) {
-    unsigned long long v[kLookPer];
-    uint32_t f[kLookPer];
-    int stop_q = kLookPer;  // nearest of this lane's predecessors that ends the walk
-    // the lane's 4 flags are read together; only a flag not yet published
-    // for this epoch is waited on (bounded)
-#pragma unroll
-    for (int q = 0; q < kLookPer; ++q) {
-      const int32_t j = base - (lane * kLookPer + q);
-      f[q] = j >= 0 ? ld_acquire_u32(&tflag[j]) : 0u;
-    }
-#pragma unroll
-    for (int q = 0; q < kLookPer; ++q) {
-      const int32_t j = base - (lane * kLookPer + q);
-      if (j >= 0 && !((f[q] >> 2) == epoch && (f[q] & 3u) != 0)) f[q] = wait_tile_flag(&tflag[j], epoch, ctl);
-    }
-#pragma unroll
-    for (int q = 0; q < kLookPer; ++q) {
-      const int32_t j = base - (lane * kLookPer + q);
-      v[q] = 0;
-      if (j < 0 || f[q] == 0) {  // before tile 0 (an inclusive 0), or timed out (error recorded)
-        if (stop_q == kLookPer) stop_q = q;
-      } else if ((f[q] & 3u) == 2u) {
-        v[q] = ld_relaxed_u64(&tincl[j]);
-        if (stop_q == kLookPer) stop_q = q;
-      } else {
-        v[q] = ld_relaxed_u64(&tagg[j]);
-      }
-    }
-    // the walk ends at the nearest (lowest lane, then lowest q) stopping predecessor
-    const uint32_t stop = __ballot_sync(0xffffffffu, stop_q < kLookPer);
-    const int first = stop ? __ffs(stop) - 1 : 32;
-    const int first_q = __shfl_sync(0xffffffffu, stop_q, first < 32 ? first : 0);
-    unsigned long long s = 0;
-#pragma unroll
-    for (int q = 0; q < kLookPer; ++q)
-      if (lane < first || (lane == first && q <= first_q)) s += v[q];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    excl += s;
-    if (stop) break;
-  }
-  if (lane == 0) {
-    st_relaxed_u64(&tincl[tile], excl + agg);
-    st_release_u32(&tflag[tile], (epoch << 2) | 2u);
-  }
-  return excl;
-}
-
 // ---- generate: activeness -> scan -> compaction --------------------------
 constexpr int kGenThreads = 256;
 constexpr int kGenRounds = 16;
 constexpr uint32_t kGenTile = kGenThreads * kGenRounds;  // 4096 vertices
+
+struct GenTotals {
+  unsigned long long cnt, edges;
+};
 
 struct GenArgs {
   uint32_t n;
@@ -199,15 +109,15 @@ struct GenArgs {
   const uint32_t *off;       // n + 1 node pointers (device copy)
   uint32_t *queue;           // activeNodes
   uint32_t *ptr;             // activeNodesPointer (count + 1)
-  uint32_t *tflag;
-  unsigned long long *tagg;
-  unsigned long long *tincl;
+  unsigned long long *tagg;  // per tile: queued vertices << 32 | edges (under an edge limit)
+  GenTotals *runs;           // per CTA: the totals of its run of tiles
+  uint32_t run_tiles;        // tiles per CTA
   Ctl *ctl;
-  uint32_t *gmask;           // count/write form: per 16-vertex group, keep bits | clear bits << 16
-  uint32_t epoch;
+  uint32_t *gmask;           // per 16-vertex group, keep bits | clear bits << 16 (null: recomputed)
   uint32_t num_tiles;
+  int aligned;               // the label, pointer and value arrays start on 16-byte boundaries
   int consume;               // sync: labels of queued vertices are cleared
-  // Count/write form: most edges one generate queues (0: no limit).  Only
+  // Most edges one generate queues (0: no limit).  Only
   // whole tiles are queued, in order, up to the limit (the first tile with
   // edges always); the later tiles keep their labels, and the count pass
   // leaves label clearing to the write pass of the tiles that are queued.
@@ -226,6 +136,10 @@ struct GenArgs {
   int sel_mode = 0;
   int algo = 0;
   const uint32_t *value = nullptr;
+  // Partition plan, made by the last tile to finish (null: none)
+  Part *parts = nullptr;
+  uint32_t max_parts = 0;
+  unsigned long long cap = 0;
 };
 
 // Whether a vertex with this value produces candidates when relaxed.
@@ -250,138 +164,45 @@ __device__ __forceinline__ bool selected(int algo, uint32_t v, uint32_t bin) {
   return algo == SGW_SSWP ? b >= bin : b <= bin;
 }
 
-// One CTA per 4096-vertex tile.  Each warp owns 512 consecutive vertices,
-// 32 per round: a lane reads label1|label2 of its vertex, the warp ballots the
-// activeness, and only active lanes read their node pointers to get degrees.
-// Active vertices of degree 0 have nothing to relax: their labels are
-// cleared here and they are not queued.  Integer algorithms; the engine uses
-// the count / scan / write form, this single-pass form serves the
-// allocation-free entry point.
-__global__ void __launch_bounds__(kGenThreads) k_generate(GenArgs a) {
-  __shared__ uint32_t s_tile;
-  __shared__ unsigned long long s_warp[kGenThreads / 32];
-  __shared__ unsigned long long s_prefix;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(&a.ctl->tile_ticket, 1u);
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  if (tile >= a.num_tiles) {  // stale ticket counter: refuse to index past the tiles
-    if (tid == 0) atomicExch(&a.ctl->error, 4u);
-    return;
-  }
-  const uint32_t wbase = tile * kGenTile + warp * (32 * kGenRounds);
-
-  uint32_t deg[kGenRounds];
-  uint32_t keepmask[kGenRounds];
-  uint32_t wcount = 0, wedges = 0;
-  uint32_t sel_bin = 0;
-  if (a.sel_mode & 2) sel_bin = a.ctl->sel_bin;
-#pragma unroll
-  for (int r = 0; r < kGenRounds; ++r) {
-    const uint32_t v = wbase + r * 32 + lane;
-    bool act = false, defer = false;
-    uint32_t d = 0;
-    if (v < a.n) {
-      act = (a.l1[v] | a.l2[v]) != 0;
-      if (act) {
-        d = __ldg(&a.off[v + 1]) - __ldg(&a.off[v]);
-        bool drop = d == 0;
-        if (a.sel_mode && !drop) {
-          const uint32_t val = a.value[v];
-          if (!pushable(a.algo, val)) drop = (a.sel_mode & 1) != 0;
-          else if ((a.sel_mode & 2) && !selected(a.algo, val, sel_bin)) defer = true;
-        }
-        if (!defer && (a.consume || drop)) { a.l1[v] = 0; a.l2[v] = 0; }
-        if (drop) d = 0;
-      }
-    }
-    const bool keep = act && d > 0 && !defer;
-    keepmask[r] = __ballot_sync(0xffffffffu, keep);
-    deg[r] = keep ? d : 0;
-    wcount += __popc(keepmask[r]);
-    wedges += __reduce_add_sync(0xffffffffu, deg[r]);
-  }
-  if (lane == 0) {
-    s_warp[warp] = ((unsigned long long)wcount << 32) | wedges;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    unsigned long long acc = 0;
-    if (lane == 0) {
-#pragma unroll
-      for (int w = 0; w < kGenThreads / 32; ++w) {
-        unsigned long long x = s_warp[w];
-        s_warp[w] = acc;
-        acc += x;
-      }
-    }
-    acc = __shfl_sync(0xffffffffu, acc, 0);
-    const unsigned long long excl = lookback_warp(tile, acc, a.tflag, a.tagg, a.tincl, a.epoch, a.ctl, lane);
-    if (lane == 0) {
-      s_prefix = excl;
-      if (tile == a.num_tiles - 1) {
-        const unsigned long long tot = excl + acc;
-        const uint32_t cnt = (uint32_t)(tot >> 32);
-        a.ctl->num_active = cnt;
-        a.ctl->num_active_edges = tot & 0xffffffffull;
-        a.ptr[cnt] = (uint32_t)(tot & 0xffffffffull);  // sentinel (subgraph_generator.cu:160)
-      }
-    }
-  }
-  __syncthreads();
-  unsigned long long run = s_prefix + s_warp[warp];
-  const uint32_t lt = lanemask_lt();
-#pragma unroll
-  for (int r = 0; r < kGenRounds; ++r) {
-    const uint32_t incl = warp_incl_scan(deg[r], lane);
-    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
-    if (keepmask[r] & (1u << lane)) {
-      const uint32_t pos = (uint32_t)(run >> 32) + __popc(keepmask[r] & lt);
-      a.queue[pos] = wbase + r * 32 + lane;
-      a.ptr[pos] = (uint32_t)(run & 0xffffffffull) + (incl - deg[r]);
-    }
-    run += ((unsigned long long)__popc(keepmask[r]) << 32) | tot;
-  }
-  if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(&a.ctl->tile_done, 1u) == a.num_tiles - 1) {
-      a.ctl->tile_ticket = 0;
-      a.ctl->tile_done = 0;
-    }
-  }
-}
-
-// Integer-family generate with 16 consecutive vertices per lane, in three
-// launches with no chain between CTAs: k_generate_count, k_generate_scan,
-// k_generate_write.  A lane reads its vertices' labels as two 16-byte words
+// Generate in two launches, with no chain between CTAs: k_generate_count and
+// k_generate_write, each CTA a run of neighbouring 4096-vertex tiles (as many
+// CTAs as fit on the GPU at once), 16 consecutive vertices per lane.  A lane
+// reads its vertices' labels as two 16-byte words, the next tile's while it
+// works on this one's,
 // and, only if one of them is active, their 17 node pointers (and values, for
 // the learned policy's selection) as 16-byte words.  The count pass stores
-// each 4096-vertex tile's (queued vertices, edges) total; one CTA turns the
-// totals into exclusive tile prefixes; the write pass recomputes the same
-// selection from the same labels and values, scans within the tile, writes
+// each run's (queued vertices, edges) total; a CTA of the write pass sums the
+// totals before its own, scans within its tiles, writes
 // the queue and pointers in order and clears the consumed labels.  Labels
 // and values do not change between the passes (nothing else runs on the
-// stream in between), so both passes select the same vertices.  Same results
-// as k_generate<false>; the label, pointer and value arrays must be 16-byte
-// aligned (the engine's arena is).
+// stream in between), so both passes select the same vertices.
+// Active vertices of degree 0 have nothing to relax: their labels are
+// cleared here and they are not queued.
 //
-// The single-pass form with a decoupled look-back (k_generate, kept for
-// PageRank and the allocation-free entry point) took 1.7-2x as long on
-// RMAT-24: with hundreds of tiles in flight the prefixes travel 32 tiles per
-// look-back step and every CTA of a wave waits for them, while the second
-// pass's labels and pointers come mostly from L2.
+// Where the caller gives no room for the keep bits (the allocation-free entry
+// point) the write pass selects again, from labels and pointers that are
+// mostly still in L2.
+//
+// Bound by memory traffic on large graphs and by the launches on small ones.
+// A single pass with a decoupled look-back was slower: with hundreds of tiles
+// in flight the prefixes travel 32 tiles per round trip to L2 (a whole call of
+// the allocation-free entry point on 16.8 M vertices, a quarter active: 181 us,
+// two passes 78-87); so was a scan kernel of one CTA
+// between the two (3.5 us per generate, 11 at 2^25 vertices), and giving each
+// tile a CTA of its own, which sums the prefix once per tile (94 us).
 constexpr uint32_t kGenVPerLane = 16;
+constexpr int kGenCtas = 4;  // per SM; the grid is one wave of them (3: 87 us for the call above, 5: 87)
 
-struct GenLane {
-  uint32_t keepmask = 0, clearmask = 0, cnt = 0, edges = 0, maxd = 0;
+struct GenLabels {
   uint32_t l1w[4] = {0, 0, 0, 0}, l2w[4] = {0, 0, 0, 0};
+};
+struct GenLane : GenLabels {
+  uint32_t keepmask = 0, clearmask = 0, cnt = 0, edges = 0, maxd = 0;
   uint32_t o[kGenVPerLane + 1];  // node pointers; a queued vertex's degree is o[k + 1] - o[k]
 };
 
-// Selection for the lane's 16 vertices starting at v0.
-__device__ __forceinline__ void gen_lane(const GenArgs &a, uint32_t v0, bool full, GenLane &L) {
-  uint32_t sel_bin = 0;
-  if (a.sel_mode & 2) sel_bin = a.ctl->sel_bin;
+// The labels of the lane's 16 vertices starting at v0.
+__device__ __forceinline__ void gen_labels(const GenArgs &a, uint32_t v0, bool full, GenLabels &L) {
   if (full) {
     const uint4 x = *reinterpret_cast<const uint4 *>(a.l1 + v0);
     const uint4 y = *reinterpret_cast<const uint4 *>(a.l2 + v0);
@@ -389,11 +210,19 @@ __device__ __forceinline__ void gen_lane(const GenArgs &a, uint32_t v0, bool ful
     L.l2w[0] = y.x; L.l2w[1] = y.y; L.l2w[2] = y.z; L.l2w[3] = y.w;
   } else {
     for (uint32_t k = 0; k < kGenVPerLane; ++k)
-      if (v0 + k < a.n) {
+      if (v0 < a.n && v0 + k < a.n) {
         L.l1w[k / 4] |= (uint32_t)a.l1[v0 + k] << (8 * (k % 4));
         L.l2w[k / 4] |= (uint32_t)a.l2[v0 + k] << (8 * (k % 4));
       }
   }
+}
+
+// Selection for the lane's 16 vertices, whose labels L holds.  SEL: by value
+// too (a.sel_mode).
+template <bool SEL>
+__device__ __forceinline__ void gen_select(const GenArgs &a, uint32_t v0, bool full, GenLane &L) {
+  uint32_t sel_bin = 0;
+  if (SEL && (a.sel_mode & 2)) sel_bin = a.ctl->sel_bin;
   uint32_t actmask = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -411,7 +240,7 @@ __device__ __forceinline__ void gen_lane(const GenArgs &a, uint32_t v0, bool ful
       L.o[4 * q] = p.x; L.o[4 * q + 1] = p.y; L.o[4 * q + 2] = p.z; L.o[4 * q + 3] = p.w;
     }
     L.o[kGenVPerLane] = __ldg(&a.off[v0 + kGenVPerLane]);
-    if (a.sel_mode) {
+    if (SEL) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const uint4 p = reinterpret_cast<const uint4 *>(a.value + v0)[q];
@@ -422,65 +251,19 @@ __device__ __forceinline__ void gen_lane(const GenArgs &a, uint32_t v0, bool ful
 #pragma unroll
     for (uint32_t k = 0; k <= kGenVPerLane; ++k) L.o[k] = (v0 + k <= a.n) ? __ldg(&a.off[v0 + k]) : 0u;
 #pragma unroll
-    for (uint32_t k = 0; k < kGenVPerLane; ++k) val[k] = (a.sel_mode && v0 + k < a.n) ? a.value[v0 + k] : 0u;
+    for (uint32_t k = 0; k < kGenVPerLane; ++k) val[k] = (SEL && v0 + k < a.n) ? a.value[v0 + k] : 0u;
   }
 #pragma unroll
   for (uint32_t k = 0; k < kGenVPerLane; ++k) {
     if (!((actmask >> k) & 1u)) continue;
     uint32_t d = L.o[k + 1] - L.o[k];
     bool drop = d == 0, defer = false;
-    if (a.sel_mode && !drop) {
+    if (SEL && !drop) {
       if (!pushable(a.algo, val[k])) drop = (a.sel_mode & 1) != 0;
       else if ((a.sel_mode & 2) && !selected(a.algo, val[k], sel_bin)) defer = true;
     }
     if (!defer && (a.consume || drop)) L.clearmask |= 1u << k;
     if (!drop && !defer) {
-      L.keepmask |= 1u << k;
-      ++L.cnt;
-      L.edges += d;
-      L.maxd = max(L.maxd, d);
-    }
-  }
-}
-
-// PageRank selection for the lane's 16 vertices (prePrefix PR overload,
-// shared/subgraph_generator.cu:24-41): active = delta > acc.  keepmask: the
-// active vertices with out-edges (queued); clearmask: every active vertex,
-// whose residual the write pass moves into its rank.  Reads only.
-__device__ __forceinline__ void gen_lane_pr(const GenArgs &a, uint32_t v0, bool full, GenLane &L) {
-  double dl[kGenVPerLane];
-  if (full) {
-#pragma unroll
-    for (int q = 0; q < kGenVPerLane / 2; ++q) {
-      const double2 p = reinterpret_cast<const double2 *>(a.delta + v0)[q];
-      dl[2 * q] = p.x;
-      dl[2 * q + 1] = p.y;
-    }
-  } else {
-#pragma unroll
-    for (uint32_t k = 0; k < kGenVPerLane; ++k) dl[k] = v0 + k < a.n ? a.delta[v0 + k] : 0.0;
-  }
-  uint32_t actmask = 0;
-#pragma unroll
-  for (uint32_t k = 0; k < kGenVPerLane; ++k)
-    if (dl[k] > a.acc) actmask |= 1u << k;
-  L.clearmask = actmask;
-  if (!actmask) return;
-  if (full) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint4 p = __ldg(reinterpret_cast<const uint4 *>(a.off + v0) + q);
-      L.o[4 * q] = p.x; L.o[4 * q + 1] = p.y; L.o[4 * q + 2] = p.z; L.o[4 * q + 3] = p.w;
-    }
-    L.o[kGenVPerLane] = __ldg(&a.off[v0 + kGenVPerLane]);
-  } else {
-#pragma unroll
-    for (uint32_t k = 0; k <= kGenVPerLane; ++k) L.o[k] = (v0 + k <= a.n) ? __ldg(&a.off[v0 + k]) : 0u;
-  }
-#pragma unroll
-  for (uint32_t k = 0; k < kGenVPerLane; ++k) {
-    const uint32_t d = L.o[k + 1] - L.o[k];
-    if (((actmask >> k) & 1u) && d) {
       L.keepmask |= 1u << k;
       ++L.cnt;
       L.edges += d;
@@ -512,241 +295,380 @@ __device__ __forceinline__ void gen_clear(const GenArgs &a, uint32_t v0, bool fu
   }
 }
 
+// Sums of two words over the CTA, on every thread.
+template <int THREADS>
+__device__ __forceinline__ GenTotals gen_block_sum(GenTotals x, GenTotals *s_warp) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    x.cnt += __shfl_xor_sync(0xffffffffu, x.cnt, d);
+    x.edges += __shfl_xor_sync(0xffffffffu, x.edges, d);
+  }
+  if (lane == 0) s_warp[warp] = x;
+  __syncthreads();
+  GenTotals y{0, 0};
+  if (lane < THREADS / 32) y = s_warp[lane];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    y.cnt += __shfl_xor_sync(0xffffffffu, y.cnt, d);
+    y.edges += __shfl_xor_sync(0xffffffffu, y.edges, d);
+  }
+  return y;
+}
+
+// What the runs before this CTA's queue.
+template <int THREADS>
+__device__ __forceinline__ GenTotals gen_prefix(const GenArgs &a, GenTotals *s_warp) {
+  GenTotals x{0, 0};
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += THREADS) {
+    const GenTotals y = a.runs[i];
+    x.cnt += y.cnt;
+    x.edges += y.edges;
+  }
+  return gen_block_sum<THREADS>(x, s_warp);
+}
+
+// Whether a tile whose predecessors queue `before` is queued.  Under an edge
+// limit the queued tiles are a prefix: those whose edges end within the limit,
+// and the first with edges in any case.
+__device__ __forceinline__ bool gen_queued(const GenArgs &a, unsigned long long before, unsigned long long own) {
+  return !a.edge_limit || before + own <= a.edge_limit || before == 0;
+}
+
+// The totals and the pointer sentinel (subgraph_generator.cu:160), by one
+// thread of the write pass: what the tiles before `tile` queue, called for the
+// first tile that is not queued or past the last one.
+__device__ __forceinline__ void gen_report(const GenArgs &a, const GenTotals &total) {
+  a.ctl->num_active = (uint32_t)total.cnt;
+  a.ctl->num_active_edges = total.edges;
+  a.ptr[total.cnt] = (uint32_t)total.edges;
+}
+
+// One tile's turn in a write pass under an edge limit, on every thread: whether
+// it is queued; the first that is not reports the totals.
+__device__ __forceinline__ bool gen_limit(const GenArgs &a, uint32_t tile, const GenTotals &before) {
+  if (gen_queued(a, before.edges, a.tagg[tile] & 0xffffffffull)) return true;
+  // tile 0 is always queued, so there is a predecessor
+  const unsigned long long prev = a.tagg[tile - 1] & 0xffffffffull;
+  if (threadIdx.x == 0 && gen_queued(a, before.edges - prev, prev)) gen_report(a, before);
+  return false;
+}
+
+__device__ void plan_cta(const uint32_t *ptr, const uint32_t *queue, Ctl *ctl, Part *parts, uint32_t max_parts,
+                          unsigned long long cap);
+
+// End of a CTA's write pass: the last one to finish makes the partition plan
+// and readies the counters for the next generate.
+__device__ __forceinline__ void gen_finish(const GenArgs &a, uint32_t *s_last) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *s_last = atomicAdd(&a.ctl->tile_done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!*s_last) return;
+  __threadfence();
+  if (threadIdx.x == 0) {
+    a.ctl->tile_done = 0;
+    a.ctl->max_degree = __ldcg(&a.ctl->degree_max);
+    a.ctl->degree_max = 0;
+  }
+  if (a.parts) plan_cta(a.ptr, a.queue, a.ctl, a.parts, a.max_parts, a.cap);
+}
+
+__device__ __forceinline__ uint32_t gen_v0(uint32_t tile) {
+  return tile * kGenTile + (threadIdx.x >> 5) * (32 * kGenRounds) + (threadIdx.x & 31) * kGenVPerLane;
+}
+__device__ __forceinline__ bool gen_full(const GenArgs &a, uint32_t v0) {
+  return a.aligned && v0 + kGenVPerLane <= a.n;
+}
+
 // Count pass: the selection of every lane's 16 vertices, whose keep and
 // clear bits it records per group (so the write pass reads 4 bytes per 16
 // vertices instead of the labels and values again), the label clearing, and
-// the tile's (count, edges) total.
-template <bool PR>
-__global__ void __launch_bounds__(kGenThreads) k_generate_count(GenArgs a) {
-  __shared__ unsigned long long s_warp[kGenThreads / 32];
+// the run's (count, edges) total.
+template <bool SEL>
+__global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_count(GenArgs a) {
+  __shared__ GenTotals s_sum[kGenThreads / 32];
+  const int lane = threadIdx.x & 31;
+  const uint32_t t0 = blockIdx.x * a.run_tiles, t1 = min(a.num_tiles, t0 + a.run_tiles);
+  GenTotals sum{0, 0};
+  uint32_t maxd = 0;
+  GenLabels next;
+  gen_labels(a, gen_v0(t0), gen_full(a, gen_v0(t0)), next);
+  for (uint32_t tile = t0; tile < t1; ++tile) {
+    const uint32_t v0 = gen_v0(tile);
+    const bool full = gen_full(a, v0);
+    GenLane L;
+    static_cast<GenLabels &>(L) = next;
+    next = GenLabels();
+    if (tile + 1 < t1) gen_labels(a, gen_v0(tile + 1), gen_full(a, gen_v0(tile + 1)), next);
+    if (v0 < a.n) {
+      gen_select<SEL>(a, v0, full, L);
+      if (a.gmask) {
+        if (!a.edge_limit) gen_clear(a, v0, full, L);
+        a.gmask[v0 / kGenVPerLane] = L.keepmask | (L.clearmask << 16);
+      }
+    }
+    sum.cnt += L.cnt;
+    sum.edges += L.edges;
+    maxd = max(maxd, L.maxd);
+    if (a.edge_limit) {
+      const GenTotals t = gen_block_sum<kGenThreads>(GenTotals{L.cnt, L.edges}, s_sum);
+      if (threadIdx.x == 0) a.tagg[tile] = t.cnt << 32 | t.edges;
+      __syncthreads();
+    }
+  }
+  maxd = __reduce_max_sync(0xffffffffu, maxd);
+  if (lane == 0 && maxd) atomicMax(&a.ctl->degree_max, maxd);
+  sum = gen_block_sum<kGenThreads>(sum, s_sum);
+  if (threadIdx.x == 0) a.runs[blockIdx.x] = sum;
+}
+
+// Write pass: the group's keep bits from the count pass (MASKS) or selected
+// again, the node pointers of groups that queue a vertex, and the queue /
+// pointer entries.
+template <bool MASKS>
+__global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_write(GenArgs a) {
+  __shared__ GenTotals s_sum[kGenThreads / 32];
+  __shared__ unsigned long long s_warp[2][kGenThreads / 32];
+  __shared__ uint32_t s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t tile = blockIdx.x;
-  const uint32_t v0 = tile * kGenTile + warp * (32 * kGenRounds) + lane * kGenVPerLane;
-  const bool full = v0 + kGenVPerLane <= a.n;
-  GenLane L;
-  if (v0 < a.n) {
-    if (PR) {
-      gen_lane_pr(a, v0, full, L);  // residuals move in the write pass
+  const uint32_t t0 = blockIdx.x * a.run_tiles, t1 = min(a.num_tiles, t0 + a.run_tiles);
+  GenLabels next;
+  uint32_t next_gm = 0;
+  auto fetch = [&](uint32_t tile) {
+    const uint32_t v0 = gen_v0(tile);
+    next = GenLabels();
+    next_gm = 0;
+    if (MASKS) {
+      if (v0 < a.n) next_gm = a.gmask[v0 / kGenVPerLane];
     } else {
-      gen_lane(a, v0, full, L);
-      if (!a.edge_limit) gen_clear(a, v0, full, L);
+      gen_labels(a, v0, gen_full(a, v0), next);
     }
-    a.gmask[v0 / kGenVPerLane] = L.keepmask | (L.clearmask << 16);
-  }
-  const uint32_t maxd = __reduce_max_sync(0xffffffffu, L.maxd);
-  const uint32_t c = __reduce_add_sync(0xffffffffu, L.cnt);
-  const uint32_t e = __reduce_add_sync(0xffffffffu, L.edges);
-  if (lane == 0) {
-    s_warp[warp] = ((unsigned long long)c << 32) | e;
-    if (maxd) atomicMax(&a.ctl->max_degree, maxd);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    unsigned long long acc = 0;
-#pragma unroll
-    for (int w = 0; w < kGenThreads / 32; ++w) acc += s_warp[w];
-    a.tagg[tile] = acc;
-  }
-}
-
-// One CTA: exclusive prefixes of the tile totals (count << 32 | edges) into
-// tincl, the totals into the control block and the pointer sentinel
-// (subgraph_generator.cu:160).
-constexpr int kGenScanThreads = 1024;
-
-// Exclusive prefix of x over the CTA's threads (kGenScanThreads), in thread order.
-__device__ __forceinline__ unsigned long long gen_block_excl(unsigned long long x, unsigned long long *s_warp) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned long long incl = x;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += y;
-  }
-  __syncthreads();  // s_warp may still be read by a previous call
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    const unsigned long long w = s_warp[lane];
-    unsigned long long wi = w;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xffffffffu, wi, d);
-      if (lane >= d) wi += y;
+  };
+  fetch(t0);  // goes out before the prefix's loads
+  GenTotals before = gen_prefix<kGenThreads>(a, s_sum);
+  bool cut = false;
+  for (uint32_t tile = t0; tile < t1; ++tile) {
+    const uint32_t v0 = gen_v0(tile);
+    const bool full = gen_full(a, v0);
+    GenLane L;
+    static_cast<GenLabels &>(L) = next;
+    const uint32_t gm = next_gm;
+    if (tile + 1 < t1) fetch(tile + 1);
+    if (a.edge_limit && !gen_limit(a, tile, before)) {  // beyond the limit, as all later tiles: labels kept
+      cut = true;
+      break;
     }
-    s_warp[lane] = wi - w;
-  }
-  __syncthreads();
-  return s_warp[warp] + incl - x;
-}
-
-// The scan under an edge limit: tile t is queued when the edges of the tiles
-// before it plus its own stay within the limit, or when no tile before it has
-// edges.  The queued tiles are a prefix (the edge prefix only grows); each
-// gets its (count, edges) prefix in tincl, the others ~0, and the last
-// queued tile writes the totals and the sentinel.
-__device__ __forceinline__ void gen_scan_limited(const GenArgs &a, uint32_t lo, uint32_t hi,
-                                                 unsigned long long *s_warp) {
-  unsigned long long sc = 0, se = 0;
-  for (uint32_t t = lo; t < hi; ++t) {
-    const unsigned long long x = a.tagg[t];
-    sc += x >> 32;
-    se += x & 0xffffffffull;
-  }
-  unsigned long long rc = gen_block_excl(sc, s_warp);
-  unsigned long long re = gen_block_excl(se, s_warp);
-  const unsigned long long lim = a.edge_limit;
-  for (uint32_t t = lo; t < hi; ++t) {
-    const unsigned long long x = a.tagg[t];
-    const unsigned long long ct = x >> 32, et = x & 0xffffffffull;
-    const bool in = re + et <= lim || re == 0;
-    a.tincl[t] = in ? ((rc << 32) | re) : ~0ull;
-    if (in) {
-      bool next_in = false;
-      if (t + 1 < a.num_tiles) {
-        const unsigned long long ne = re + et, en = a.tagg[t + 1] & 0xffffffffull;
-        next_in = ne + en <= lim || ne == 0;
+    if (!MASKS) {
+      if (v0 < a.n) {
+        gen_select<false>(a, v0, full, L);
+        gen_clear(a, v0, full, L);
       }
-      if (!next_in) {
-        const uint32_t c = (uint32_t)(rc + ct);
-        a.ctl->num_active = c;
-        a.ctl->num_active_edges = re + et;
-        a.ptr[c] = (uint32_t)(re + et);
+    } else {
+      L.keepmask = gm & 0xffffu;
+      if (a.edge_limit && (gm >> 16)) {  // the clearing the count pass left to this tile
+        gen_labels(a, v0, full, L);
+        L.clearmask = gm >> 16;
+        gen_clear(a, v0, full, L);
       }
-    }
-    rc += ct;
-    re += et;
-  }
-}
-
-__global__ void __launch_bounds__(kGenScanThreads) k_generate_scan(GenArgs a) {
-  __shared__ unsigned long long s_warp[kGenScanThreads / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t per = (a.num_tiles + kGenScanThreads - 1) / kGenScanThreads;
-  const uint32_t lo = min(a.num_tiles, tid * per), hi = min(a.num_tiles, lo + per);
-  if (a.edge_limit) {
-    gen_scan_limited(a, lo, hi, s_warp);
-    return;
-  }
-  unsigned long long sum = 0;
-  for (uint32_t t = lo; t < hi; ++t) sum += a.tagg[t];
-  unsigned long long incl = sum;
+      if (L.keepmask) {
+        if (full) {
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += y;
-  }
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    unsigned long long w = s_warp[lane];
-    unsigned long long wi = w;
+          for (int q = 0; q < 4; ++q) {
+            const uint4 p = __ldg(reinterpret_cast<const uint4 *>(a.off + v0) + q);
+            L.o[4 * q] = p.x; L.o[4 * q + 1] = p.y; L.o[4 * q + 2] = p.z; L.o[4 * q + 3] = p.w;
+          }
+          L.o[kGenVPerLane] = __ldg(&a.off[v0 + kGenVPerLane]);
+        } else {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xffffffffu, wi, d);
-      if (lane >= d) wi += y;
-    }
-    s_warp[lane] = wi - w;
-    if (lane == 31) {
-      const uint32_t c = (uint32_t)(wi >> 32);
-      a.ctl->num_active = c;
-      a.ctl->num_active_edges = wi & 0xffffffffull;
-      a.ptr[c] = (uint32_t)(wi & 0xffffffffull);
-    }
-  }
-  __syncthreads();
-  unsigned long long run = s_warp[warp] + incl - sum;
-  for (uint32_t t = lo; t < hi; ++t) {
-    const unsigned long long x = a.tagg[t];
-    a.tincl[t] = run;
-    run += x;
-  }
-}
-
-// Write pass: the group's keep bits from the count pass, the node pointers
-// of groups that queue a vertex, and the queue / pointer entries.  PR: every
-// active vertex's residual moves into its rank (value += delta, delta = 0,
-// the first half of pr_kernel, shared/gpu_kernels.cu:234-250) and its queue
-// entry carries the push damping * delta / outdeg, so each round is a
-// bulk-synchronous snapshot.
-template <bool PR>
-__global__ void __launch_bounds__(kGenThreads) k_generate_write(GenArgs a) {
-  __shared__ unsigned long long s_warp[kGenThreads / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t tile = blockIdx.x;
-  const uint32_t v0 = tile * kGenTile + warp * (32 * kGenRounds) + lane * kGenVPerLane;
-  const bool full = v0 + kGenVPerLane <= a.n;
-  if (a.edge_limit && a.tincl[tile] == ~0ull) return;  // beyond the limit: labels kept for later
-  GenLane L;
-  if (v0 < a.n) {
-    const uint32_t gm = a.gmask[v0 / kGenVPerLane];
-    L.keepmask = gm & 0xffffu;
-    if (!PR && a.edge_limit && (gm >> 16)) {  // the clearing the count pass left to this tile
-      L.clearmask = gm >> 16;
-      if (full) {
-        const uint4 x = *reinterpret_cast<const uint4 *>(a.l1 + v0);
-        const uint4 y = *reinterpret_cast<const uint4 *>(a.l2 + v0);
-        L.l1w[0] = x.x; L.l1w[1] = x.y; L.l1w[2] = x.z; L.l1w[3] = x.w;
-        L.l2w[0] = y.x; L.l2w[1] = y.y; L.l2w[2] = y.z; L.l2w[3] = y.w;
-      }
-      gen_clear(a, v0, full, L);
-    }
-    if (L.keepmask) {
-      if (full) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint4 p = __ldg(reinterpret_cast<const uint4 *>(a.off + v0) + q);
-          L.o[4 * q] = p.x; L.o[4 * q + 1] = p.y; L.o[4 * q + 2] = p.z; L.o[4 * q + 3] = p.w;
+          for (uint32_t k = 0; k <= kGenVPerLane; ++k) L.o[k] = (v0 + k <= a.n) ? __ldg(&a.off[v0 + k]) : 0u;
         }
-        L.o[kGenVPerLane] = __ldg(&a.off[v0 + kGenVPerLane]);
-      } else {
+        L.cnt = (uint32_t)__popc(L.keepmask);
 #pragma unroll
-        for (uint32_t k = 0; k <= kGenVPerLane; ++k) L.o[k] = (v0 + k <= a.n) ? __ldg(&a.off[v0 + k]) : 0u;
+        for (uint32_t k = 0; k < kGenVPerLane; ++k)
+          if ((L.keepmask >> k) & 1u) L.edges += L.o[k + 1] - L.o[k];
       }
-      L.cnt = (uint32_t)__popc(L.keepmask);
-#pragma unroll
-      for (uint32_t k = 0; k < kGenVPerLane; ++k)
-        if ((L.keepmask >> k) & 1u) L.edges += L.o[k + 1] - L.o[k];
     }
-  }
-  const uint32_t incl_c = warp_incl_scan(L.cnt, lane);
-  const uint32_t incl_e = warp_incl_scan(L.edges, lane);
-  if (lane == 31) s_warp[warp] = ((unsigned long long)incl_c << 32) | incl_e;
-  __syncthreads();
-  if (tid == 0) {
-    unsigned long long acc = a.tincl[tile];
+    if (!__syncthreads_or(L.keepmask != 0)) continue;  // a tile that queues nothing
+    const uint32_t incl_c = warp_incl_scan(L.cnt, lane);
+    const uint32_t incl_e = warp_incl_scan(L.edges, lane);
+    unsigned long long *const sums = s_warp[tile & 1u];  // the other half may still be read
+    if (lane == 31) sums[warp] = ((unsigned long long)incl_c << 32) | incl_e;
+    __syncthreads();
+    // positions stay below 2^32: so do the edges of a queue
+    uint32_t pos = (uint32_t)before.cnt + incl_c - L.cnt, ep = (uint32_t)before.edges + incl_e - L.edges;
 #pragma unroll
     for (int w = 0; w < kGenThreads / 32; ++w) {
-      const unsigned long long x = s_warp[w];
-      s_warp[w] = acc;
-      acc += x;
+      const unsigned long long x = sums[w];
+      before.cnt += x >> 32;
+      before.edges += x & 0xffffffffull;
+      if (w < warp) {
+        pos += (uint32_t)(x >> 32);
+        ep += (uint32_t)x;
+      }
     }
-  }
-  __syncthreads();
-  if (L.keepmask) {
-    const unsigned long long run = s_warp[warp] + (((unsigned long long)(incl_c - L.cnt) << 32) | (incl_e - L.edges));
-    uint32_t pos = (uint32_t)(run >> 32), ep = (uint32_t)(run & 0xffffffffull);
+    if (L.keepmask) {
 #pragma unroll
-    for (uint32_t k = 0; k < kGenVPerLane; ++k) {
-      if ((L.keepmask >> k) & 1u) {
-        const uint32_t d = L.o[k + 1] - L.o[k];
-        a.queue[pos] = v0 + k;
-        a.ptr[pos] = ep;
-        if (PR) a.qpush[pos] = a.damping * a.delta[v0 + k] / (double)d;
-        ++pos;
-        ep += d;
+      for (uint32_t k = 0; k < kGenVPerLane; ++k) {
+        if ((L.keepmask >> k) & 1u) {
+          const uint32_t d = L.o[k + 1] - L.o[k];
+          a.queue[pos] = v0 + k;
+          a.ptr[pos] = ep;
+          ++pos;
+          ep += d;
+        }
       }
     }
   }
-  if (PR && v0 < a.n) {  // residuals of every active vertex (queued or of degree 0) into the ranks
-    const uint32_t cm = a.gmask[v0 / kGenVPerLane] >> 16;
+  // past the last tile: the totals, unless a tile was beyond the limit
+  if (t1 == a.num_tiles && !cut && tid == 0) gen_report(a, before);
+  gen_finish(a, &s_last);
+}
+
+// PageRank's two passes (prePrefix PR overload, shared/subgraph_generator.cu:
+// 24-41): active = delta > acc; the queue takes the active vertices with
+// out-edges.  A tile of 4096 vertices by 1024 threads, four neighbouring-lane
+// rounds each, so the 8-byte residuals and ranks are read and written
+// coalesced, two CTAs per SM.  PageRank's generate at 2^20 vertices, plan included:
+// 34 us and four launches before, 28 us and two now.  The write pass moves every active vertex's residual into
+// its rank (value += delta, delta = 0, the first half of pr_kernel,
+// shared/gpu_kernels.cu:234-250); its queue entry carries the push
+// damping * delta / outdeg, so each round is a bulk-synchronous snapshot.
+constexpr int kGenPrThreads = 1024;
+constexpr int kGenPrRounds = kGenTile / kGenPrThreads;
+
+// x > acc for acc > 0, as integers (a 64-bit floating-point compare holds a warp
+// for about 15 cycles): non-negative doubles order as their bits, negative
+// ones have the sign bit, and NaN is not above anything.
+__device__ __forceinline__ bool pr_above(double x, double acc) {
+  const long long b = __double_as_longlong(x);
+  return b > __double_as_longlong(acc) && b <= 0x7ff0000000000000ll;
+}
+
+__device__ __forceinline__ void gen_pr_select(const GenArgs &a, uint32_t tile, double (&dl)[kGenPrRounds],
+                                              uint32_t (&deg)[kGenPrRounds]) {
 #pragma unroll
-    for (uint32_t k = 0; k < kGenVPerLane; ++k)
-      if ((cm >> k) & 1u) {
-        a.pval[v0 + k] += a.delta[v0 + k];
-        a.delta[v0 + k] = 0.0;
-      }
+  for (int r = 0; r < kGenPrRounds; ++r) {
+    const uint32_t v = tile * kGenTile + r * kGenPrThreads + threadIdx.x;
+    dl[r] = v < a.n ? a.delta[v] : 0.0;
   }
+#pragma unroll
+  for (int r = 0; r < kGenPrRounds; ++r) {
+    const uint32_t v = tile * kGenTile + r * kGenPrThreads + threadIdx.x;
+    deg[r] = v < a.n && pr_above(dl[r], a.acc) ? __ldg(&a.off[v + 1]) - __ldg(&a.off[v]) : 0u;
+  }
+}
+
+__global__ void __launch_bounds__(kGenPrThreads, 2) k_generate_count_pr(GenArgs a) {
+  __shared__ GenTotals s_sum[kGenPrThreads / 32];
+  const uint32_t t0 = blockIdx.x * a.run_tiles, t1 = min(a.num_tiles, t0 + a.run_tiles);
+  GenTotals sum{0, 0};
+  uint32_t maxd = 0;
+  for (uint32_t tile = t0; tile < t1; ++tile) {
+    double dl[kGenPrRounds];
+    uint32_t deg[kGenPrRounds];
+    gen_pr_select(a, tile, dl, deg);
+    GenTotals x{0, 0};
+#pragma unroll
+    for (int r = 0; r < kGenPrRounds; ++r) {
+      x.cnt += deg[r] > 0;
+      x.edges += deg[r];
+      maxd = max(maxd, deg[r]);
+    }
+    sum.cnt += x.cnt;
+    sum.edges += x.edges;
+    if (a.edge_limit) {
+      x = gen_block_sum<kGenPrThreads>(x, s_sum);
+      if (threadIdx.x == 0) a.tagg[tile] = x.cnt << 32 | x.edges;
+      __syncthreads();
+    }
+  }
+  maxd = __reduce_max_sync(0xffffffffu, maxd);
+  if ((threadIdx.x & 31) == 0 && maxd) atomicMax(&a.ctl->degree_max, maxd);
+  sum = gen_block_sum<kGenPrThreads>(sum, s_sum);
+  if (threadIdx.x == 0) a.runs[blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(kGenPrThreads, 2) k_generate_write_pr(GenArgs a) {
+  constexpr int kWarps = kGenPrThreads / 32, kParts = kGenPrRounds * kWarps;
+  __shared__ GenTotals s_sum[kWarps];
+  __shared__ unsigned long long s_part[kParts + 1];  // (round, warp): count << 32 | edges, then the tile's total
+  __shared__ uint32_t s_last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t t0 = blockIdx.x * a.run_tiles, t1 = min(a.num_tiles, t0 + a.run_tiles);
+  GenTotals before = gen_prefix<kGenPrThreads>(a, s_sum);
+  bool cut = false;
+  for (uint32_t tile = t0; tile < t1; ++tile) {
+    if (a.edge_limit && !gen_limit(a, tile, before)) {  // beyond the limit: residuals kept
+      cut = true;
+      break;
+    }
+    double dl[kGenPrRounds];
+    uint32_t deg[kGenPrRounds], incl[kGenPrRounds];
+    gen_pr_select(a, tile, dl, deg);
+#pragma unroll
+    for (int r = 0; r < kGenPrRounds; ++r) {
+      incl[r] = warp_incl_scan(deg[r], lane);
+      const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, deg[r] > 0));
+      if (lane == 31) s_part[r * kWarps + warp] = ((unsigned long long)c << 32) | incl[r];
+    }
+    __syncthreads();
+    if (warp == 0) {  // exclusive prefixes in (round, warp) order, kGenPrRounds entries per lane
+      unsigned long long x[kGenPrRounds], sum = 0;
+#pragma unroll
+      for (int k = 0; k < kGenPrRounds; ++k) {
+        x[k] = s_part[lane * kGenPrRounds + k];
+        sum += x[k];
+      }
+      unsigned long long run = sum;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, run, d);
+        if (lane >= d) run += y;
+      }
+      if (lane == 31) s_part[kParts] = run;
+      run -= sum;
+#pragma unroll
+      for (int k = 0; k < kGenPrRounds; ++k) {
+        s_part[lane * kGenPrRounds + k] = run;
+        run += x[k];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kGenPrRounds; ++r) {
+      const uint32_t v = tile * kGenTile + r * kGenPrThreads + tid;
+      const uint32_t keep = __ballot_sync(0xffffffffu, deg[r] > 0);
+      if (v < a.n && pr_above(dl[r], a.acc)) {  // every active vertex, queued or of degree 0
+        a.pval[v] += dl[r];
+        a.delta[v] = 0.0;
+      }
+      if (deg[r]) {
+        const unsigned long long p = s_part[r * kWarps + warp];
+        const uint32_t pos = (uint32_t)before.cnt + (uint32_t)(p >> 32) + __popc(keep & lanemask_lt());
+        a.queue[pos] = v;
+        a.ptr[pos] = (uint32_t)before.edges + (uint32_t)p + incl[r] - deg[r];
+        a.qpush[pos] = a.damping * dl[r];
+      }
+    }
+    // the divisions, over the tile's queue entries instead of its vertices: a
+    // 64-bit division holds a warp for a few hundred cycles whether one of its
+    // lanes needs it or all
+    const unsigned long long total = s_part[kParts];
+    const uint32_t cnt = (uint32_t)(total >> 32), end = (uint32_t)before.edges + (uint32_t)total;
+    __syncthreads();
+    for (uint32_t i = tid; i < cnt; i += kGenPrThreads) {
+      const uint32_t pos = (uint32_t)before.cnt + i;
+      const uint32_t d = (i + 1 < cnt ? a.ptr[pos + 1] : end) - a.ptr[pos];
+      a.qpush[pos] = a.qpush[pos] / (double)d;
+    }
+    before.cnt += cnt;
+    before.edges += total & 0xffffffffull;
+  }
+  if (t1 == a.num_tiles && !cut && tid == 0) gen_report(a, before);
+  gen_finish(a, &s_last);
 }
 
 // ---- frontier deferral (learned policy) --------------------------------------
@@ -851,51 +773,71 @@ __global__ void __launch_bounds__(kSelBins / 4) k_select_pick(int algo, const un
 }
 
 // ---- partition planner ------------------------------------------------------
-// One warp.  For each partition: the largest run of queue entries starting at
-// `from` whose edges fit `cap`, found by a 32-way search (each step probes 32
-// evenly spaced entries and keeps the bracket of the last one that fits).
-__global__ void k_plan(const uint32_t *ptr, const uint32_t *queue, Ctl *ctl,
-                       Part *parts, uint32_t max_parts, unsigned long long cap) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t count = ctl->num_active;
+// One CTA.  For each partition: the largest run of queue entries starting at
+// `from` whose edges fit `cap`, found by a search as many ways as the CTA has
+// threads (each step probes evenly spaced entries and keeps the bracket of the
+// last one that fits: two round trips to L2 for 64 K entries and 256 threads,
+// where one warp takes four).
+// Loads go through L2: the CTAs of the generate that runs it wrote the queue.
+__device__ void plan_cta(const uint32_t *ptr, const uint32_t *queue, Ctl *ctl, Part *parts, uint32_t max_parts,
+                         unsigned long long cap) {
+  const uint32_t tid = threadIdx.x, nth = blockDim.x;
+  const uint32_t count = __ldcg(&ctl->num_active);
+  const unsigned long long edges = __ldcg(&ctl->num_active_edges);
   uint32_t from = 0, p = 0;
+  if (count && edges <= cap) {  // everything in one partition: nothing to search
+    if (tid == 0) {
+      const Part q{0, count, 0, __ldcg(&queue[0]), edges};
+      if (max_parts) parts[0] = q;
+      ctl->first[0] = q;
+    }
+    from = count;
+    p = 1;
+  }
   while (from < count) {
-    const unsigned long long limit = (unsigned long long)ptr[from] + cap;
+    const uint32_t start = __ldcg(&ptr[from]);
+    const unsigned long long limit = (unsigned long long)start + cap;
     // answer t in [from, count]: largest index with ptr[t] <= limit
     uint32_t lo = from + 1, hi = count;  // candidates above `from`
     uint32_t best = from;
     while (lo <= hi) {
       const uint32_t span = hi - lo + 1;
-      const uint32_t step = (span + 31) / 32;
-      const uint32_t idx = lo + (uint32_t)lane * step;
-      const bool ok = idx <= hi && (unsigned long long)ptr[idx] <= limit;
-      const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-      const int k = __popc(bal);  // ok is a prefix of the lanes
+      const uint32_t step = (span + nth - 1) / nth;
+      const unsigned long long idx = lo + (unsigned long long)tid * step;
+      const bool ok = idx <= hi && (unsigned long long)__ldcg(&ptr[idx]) <= limit;
+      const uint32_t k = (uint32_t)__syncthreads_count(ok);  // ok is a prefix of the threads
       if (k == 0) break;
-      const uint32_t last_ok = lo + (uint32_t)(k - 1) * step;
+      const uint32_t last_ok = lo + (k - 1) * step;
       best = last_ok;
       if (step == 1) break;
       lo = last_ok + 1;
-      const uint32_t next_bad = lo - 1 + step;  // first probe that failed
-      if (k < 32 && next_bad - 1 < hi) hi = next_bad - 1;
+      const unsigned long long next_bad = (unsigned long long)last_ok + step;  // first probe that failed
+      if (k < nth && next_bad - 1 < hi) hi = (uint32_t)next_bad - 1;
     }
-    uint32_t to = best > from ? best : from + 1;  // a vertex beyond cap runs alone
-    if (lane == 0 && p < max_parts) {
+    const uint32_t to = best > from ? best : from + 1;  // a vertex beyond cap runs alone
+    if (tid == 0 && p < max_parts) {
       Part q;
       q.from = from;
       q.size = to - from;
-      q.edge_from = ptr[from];
-      q.first_vertex = queue[from];
-      q.edge_count = (unsigned long long)ptr[to] - ptr[from];
+      q.edge_from = start;
+      q.first_vertex = __ldcg(&queue[from]);
+      q.edge_count = (unsigned long long)__ldcg(&ptr[to]) - start;
       parts[p] = q;
+      if (p < kCtlParts) ctl->first[p] = q;
     }
     ++p;
     from = to;
   }
-  if (lane == 0) {
+  if (tid == 0) {
     ctl->num_parts = p;
     if (p > max_parts) atomicExch(&ctl->error, 2u);
   }
+}
+
+// The plan on its own (the step API's sgw_partition).
+__global__ void k_plan(const uint32_t *ptr, const uint32_t *queue, Ctl *ctl, Part *parts, uint32_t max_parts,
+                       unsigned long long cap) {
+  plan_cta(ptr, queue, ctl, parts, max_parts, cap);
 }
 
 // ---- gather: host CSR -> device edge buffer -------------------------------
