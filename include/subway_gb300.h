@@ -183,7 +183,7 @@ typedef struct sgw_engine_opts {
   uint64_t budget_bytes;
   int32_t device;          /* CUDA device ordinal (--device)                  */
   uint32_t flags;          /* SGW_OPT_*                                       */
-  uint32_t inner_batch;    /* async inner iterations launched per host check  */
+  uint32_t inner_batch;    /* async inner iterations launched ahead, at most 3 */
   uint32_t tile_degree_max;/* sources above this degree go to the chunk list  */
   uint32_t chunk_edges;    /* edges per chunk-list item (multiple of 32)      */
   uint32_t gather_ctas;    /* CTAs of the gather kernel, 0 = 2 per SM (3 per SM

@@ -105,6 +105,11 @@ struct sgw_engine {
   uint32_t max_parts = 0, wl_cap = 0, num_tiles = 0;
 
   // host side
+  volatile unsigned long long *h_poll = nullptr;  // mapped: progress of the running partition
+  unsigned long long *d_poll = nullptr;
+  uint32_t poll_tag = 0;
+  uint32_t iter_base = 0;                  // inner iterations launched so far in the run
+  uint64_t iters_known = 0;                // inner iterations that did work, at the last read-back
   Ctl *h_ctl = nullptr;
   Part *h_parts = nullptr;
   HostStream hs_ends;                      // transfer records (destination words)
@@ -384,6 +389,7 @@ int read_ctl(sgw_engine *e) {
   CK(cudaMemcpyAsync(e->h_ctl, e->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, e->s_comp));
   e->stats.d2h_bytes += sizeof(Ctl);
   CK(cudaStreamSynchronize(e->s_comp));
+  e->iters_known = e->h_ctl->iters_total;
   e->stats.inner_iterations = (uint64_t)e->h_ctl->iters_total + e->hub_iters;
   return check_ctl_error(e);
 }
@@ -818,6 +824,9 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   a.size = q.size;
   a.edge_from = q.edge_from;
   a.iter = iter;
+  a.base = e->iter_base;
+  a.poll = ASYNC ? e->d_poll : nullptr;
+  a.poll_tag = e->poll_tag;
   a.tile_degree_max = e->opts.tile_degree_max;
   a.chunk_edges = e->opts.chunk_edges;
   a.pbits = e->pbits;
@@ -880,6 +889,9 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   a.size = q.size;
   a.edge_from = q.edge_from;
   a.iter = iter;
+  a.base = e->iter_base;
+  a.poll = e->d_poll;
+  a.poll_tag = e->poll_tag;
   a.pbits = e->pbits;
   a.streamed = e->cur_streamed;
   a.stream_base = (uint32_t)e->cur_stream_base;  // with the low words of off: offsets mod 2^32
@@ -986,28 +998,49 @@ int process_hub(sgw_engine *e, const Part &q, uint32_t b) {
   return SGW_OK;
 }
 
-// Relaxation of one resident partition: sync = one pass; async = mixLabels
-// then inner iterations until no relaxation improves (or max_inner).
-// Inner iterations are counted on the device (Ctl::iters_total, refreshed
-// into the statistics by every control-block read).  With sync_always false
-// a partition whose inner cap is reached returns without waiting for it
-// (*iters_out is then 0: unknown until the next read).  The learned policy
-// keeps the wait: letting the host run ahead put more gathers beside each
+// Waits until the running partition reports an iteration later than `begun` (or
+// that it has converged) and returns the report.  The host polls mapped memory:
+// waiting for a copy of the control block instead left the GPU idle for about
+// 12 us per partition.
+int poll_wait(sgw_engine *e, uint64_t begun, uint64_t *iter, bool *done) {
+  for (uint64_t spin = 1;; ++spin) {
+    const unsigned long long x = *e->h_poll;
+    if ((uint32_t)(x >> 48) == e->poll_tag) {
+      *iter = (x & 0xffffffffffffull) >> 1;
+      *done = x & 1u;
+      if (*iter > begun || *done) return SGW_OK;
+    }
+    if (spin % 65536 == 0) {  // nothing for a while: a failed launch reports here
+      const cudaError_t q = cudaStreamQuery(e->s_comp);
+      if (q == cudaSuccess && *e->h_poll == x)
+        return fail(SGW_ECUDA, "a partition's inner iterations ended without a report");
+      if (q != cudaSuccess && q != cudaErrorNotReady)
+        return fail(SGW_ECUDA, "inner iterations failed: %s", cudaGetErrorString(q));
+    }
+  }
+}
+
+// Relaxation of one resident partition: sync = one pass; async = inner
+// iterations until no relaxation improves (or max_inner), at most kPollAhead
+// of them launched beyond the last that is known to have begun, so that a
+// partition costs at most that many idle launches (batches of eight wasted a
+// third of them).  Returns when the partition is done.  The learned policy
+// needs that wait: letting the host run ahead put more gathers beside each
 // relaxation and made both slower (RMAT-24 SSSP-async: 12.2 against 17.0
-// GTEPS).
+// GTEPS).  iters_out: iterations that did work, counted on the device.
 // first: no partition of this global iteration has been relaxed before.
-int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool first,
-                     bool sync_always = true) {
+constexpr uint32_t kPollAhead = 3;
+
+int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool first) {
   const bool async = e->params.mode == SGW_ASYNC;
   const bool tiles = (e->opts.flags & SGW_OPT_CTA_TILES) != 0;
   const bool all = !tiles && !(async && e->labels_partial);  // the first pass relaxes every queued source
-  // upd, wl_count, iters_run
-  CK(cudaMemsetAsync(&e->d_ctl->upd[0], 0, sizeof(uint32_t) * 9, e->s_comp));
+  size_t slot = 0;
   if (!async) {
-    size_t slot = 0;
     TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
     TRY(launch_relax(e, q, b, 1, false, all));
     TRY(prof_end(e, e->s_comp, slot));
+    e->iter_base += 1;
     if (iters_out) *iters_out = 1;
     return SGW_OK;
   }
@@ -1024,24 +1057,33 @@ int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_o
   }
   uint32_t max_inner = e->params.max_inner ? e->params.max_inner : 0xffffffffu;
   if (e->range_inner_cap) max_inner = std::min(max_inner, e->range_inner_cap);
-  uint32_t iter = 1;
-  const uint32_t batch = std::max<uint32_t>(1, e->opts.inner_batch);
-  while (true) {
-    const uint32_t nb = std::min<uint32_t>(batch, max_inner - (iter - 1));
-    size_t slot = 0;
-    TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
-    for (uint32_t k = 0; k < nb; ++k, ++iter) TRY(launch_relax(e, q, b, iter, true, all && iter == 1));
-    TRY(prof_end(e, e->s_comp, slot));
-    const uint32_t last = iter - 1;
-    if (!sync_always && last >= max_inner) {  // capped: nothing to decide on the host
-      if (iters_out) *iters_out = 0;
-      return SGW_OK;
+  const uint64_t ahead = std::min<uint64_t>(std::max<uint32_t>(1, e->opts.inner_batch), kPollAhead);
+  e->poll_tag = (e->poll_tag + 1) & 0xffffu;
+  const uint64_t total0 = e->iters_known;
+  uint64_t launched = 0, begun = 1;
+  bool done = false;
+  TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
+  while (!done) {
+    while (launched < max_inner && launched < begun + ahead) {
+      ++launched;
+      TRY(launch_relax(e, q, b, (uint32_t)launched, true, all && launched == 1));
     }
-    TRY(read_ctl(e));
-    if (e->h_ctl->upd[last & 3u] == 0) break;  // converged
-    if (last >= max_inner) break;             // leftover labels go to the next generate
+    if (launched >= max_inner) {  // capped: leftover labels go to the next generate
+      k_poll_end<<<1, 1, 0, e->s_comp>>>(e->d_poll, e->poll_tag, (uint32_t)std::min<uint64_t>(launched + 1, 0xffffffffu));
+      CK(cudaGetLastError());
+      e->stats.launches += 1;
+      do TRY(poll_wait(e, launched, &begun, &done));
+      while (!done);
+      break;
+    }
+    TRY(poll_wait(e, begun, &begun, &done));
   }
-  if (iters_out) *iters_out = e->h_ctl->iters_run;
+  TRY(prof_end(e, e->s_comp, slot));
+  e->iter_base += (uint32_t)launched;
+  if (iters_out) {
+    TRY(read_ctl(e));
+    *iters_out = (uint32_t)(e->iters_known - total0);
+  }
   return SGW_OK;
 }
 
@@ -1060,6 +1102,7 @@ int process_from_host(sgw_engine *e, const Part &q) {
   size_t slot = 0;
   TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
   TRY(launch_relax(e, q, kFromHost, 1, false, true));
+  e->iter_base += 1;
   TRY(prof_end(e, e->s_comp, slot));
   e->stats.h2d_bytes += q.edge_count * (4ull * e->W + (e->use_w ? 1 : 0));
   return SGW_OK;
@@ -1089,6 +1132,8 @@ int state_init(sgw_engine *e, const sgw_run_params *p, bool take_labels) {
   e->use_w = e->split && (p->algo == SGW_SSSP || p->algo == SGW_SSWP);
   e->stats = sgw_run_stats{};
   e->hub_iters = 0;
+  e->iter_base = 0;
+  e->iters_known = 0;
   e->prof_used = 0;
   e->initialized = false;
   e->gitr = 0;
@@ -1150,7 +1195,7 @@ int process_iteration(sgw_engine *e) {
       TRY(process_hub(e, q, b));
     } else {
       CK(cudaStreamWaitEvent(e->s_comp, e->ev_ready[b], 0));
-      TRY(process_resident(e, q, b, &inner, p == 0));
+      TRY(process_resident(e, q, b, e->trace_on ? &inner : nullptr, p == 0));
     }
     CK(cudaEventRecord(e->ev_free[b], e->s_comp));
     trace_partition(e, p, inner);
@@ -1177,6 +1222,7 @@ int generate_and_stats(sgw_engine *e, int consume) {
   CK(cudaMemcpyAsync(e->h_ctl, e->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, e->s_comp));
   CK(cudaMemcpyAsync(e->h_rstat, e->d_rstat, sizeof(RangeStat) * S, cudaMemcpyDeviceToHost, e->s_comp));
   CK(cudaStreamSynchronize(e->s_comp));
+  e->iters_known = e->h_ctl->iters_total;
   TRY(check_ctl_error(e));
   e->num_active = e->h_ctl->num_active;
   e->num_active_edges = e->h_ctl->num_active_edges;
@@ -1373,7 +1419,7 @@ int process_iteration_ranges(sgw_engine *e) {
       for (uint32_t s = j.s; s < j.s_end; ++s) pred = std::max(pred, e->h_rstat[s].pred);
       const bool cappable = kept || (e->opts.sched_flags & SGW_SCHED_CAP_COMPACT);
       e->range_inner_cap = cappable && (double)pred >= thr ? (e->opts.sched_inner ? e->opts.sched_inner : 3u) : 0u;
-      const int st = process_resident(e, q, (uint32_t)j.buf, &inner, k == 0);
+      const int st = process_resident(e, q, (uint32_t)j.buf, e->trace_on ? &inner : nullptr, k == 0);
       e->cur_streamed = 0;
       e->range_inner_cap = 0;
       TRY(st);
@@ -1719,11 +1765,20 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   }
   if (cudaEventCreate(&e->ev_t0) != cudaSuccess || cudaEventCreate(&e->ev_t1) != cudaSuccess)
     return cleanup(fail(SGW_ECUDA, "event creation"));
-  if (cudaMallocHost(&e->h_ctl, sizeof(Ctl)) != cudaSuccess ||
+  if (cudaHostAlloc(&e->h_ctl, align_up(sizeof(Ctl), 64) + 64, cudaHostAllocMapped) != cudaSuccess ||
       cudaMallocHost(&e->h_parts, sizeof(Part) * (size_t)parts_host) != cudaSuccess ||
       cudaMallocHost(&e->h_rstat, sizeof(RangeStat) * (size_t)parts_host) != cudaSuccess)
     return cleanup(fail(SGW_ECUDA, "pinned control block"));
   memset(e->h_ctl, 0, sizeof(Ctl));
+  {  // the progress word lies behind the control block
+    char *word = reinterpret_cast<char *>(e->h_ctl) + align_up(sizeof(Ctl), 64);
+    void *dp = nullptr;
+    if (cudaHostGetDevicePointer(&dp, word, 0) != cudaSuccess)
+      return cleanup(fail(SGW_ECUDA, "mapped progress word"));
+    e->h_poll = reinterpret_cast<volatile unsigned long long *>(word);
+    *e->h_poll = 0;
+    e->d_poll = static_cast<unsigned long long *>(dp);
+  }
   if (!e->wide) {
     ce = cudaMemcpyAsync(e->d_off, g->node_pointer, 4ull * (e->n + 1), cudaMemcpyHostToDevice, e->s_comp);
   } else {  // low words of every node pointer, full pointers of every group start

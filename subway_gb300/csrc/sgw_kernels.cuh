@@ -58,7 +58,6 @@ struct Ctl {
   uint32_t max_degree;       // largest degree queued by the last generate
   uint32_t upd[4];           // async inner iteration k: relaxations that improved
   uint32_t wl_count[4];      // chunk-list items of inner iteration k
-  uint32_t iters_run;        // inner iterations that did work
   uint32_t hub_active;       // single-vertex partition: the source was dirty
   uint32_t hub_value;        // single-vertex partition: its value
   uint32_t sel_bin;          // deferral: the last value bin selected this iteration
@@ -1275,7 +1274,10 @@ struct RelaxArgs {
   WorkItem *wl;
   uint32_t wl_cap;
   uint32_t from, size, edge_from;
-  uint32_t iter;             // inner iteration number (1-based)
+  uint32_t iter;             // inner iteration of the partition (1-based)
+  uint32_t base;             // inner iterations launched before this partition's
+  unsigned long long *poll;  // host word that async iterations > 1 report to (null: none)
+  uint32_t poll_tag;
   uint32_t tile_degree_max;  // sources above this go to the chunk list
   uint32_t chunk_edges;
   uint32_t pbits;            // packed records: bits of the destination
@@ -1289,6 +1291,18 @@ struct RelaxArgs {
 };
 
 constexpr int kRelaxThreads = 256;
+
+// Tells the host that inner iteration `iter` has begun (the one before it is
+// complete) and whether it has nothing to do: one 64-bit word of mapped host
+// memory that the host polls instead of waiting for a copy of the control block.
+__device__ __forceinline__ void poll_report(unsigned long long *poll, uint32_t tag, uint32_t iter, int skip) {
+  if (poll && iter > 1) {
+    const unsigned long long x = (unsigned long long)tag << 48 | (unsigned long long)iter << 1 | (unsigned)skip;
+    asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(poll), "l"(x) : "memory");
+  }
+}
+// The same for the iteration after a capped partition's last.
+__global__ void k_poll_end(unsigned long long *poll, uint32_t tag, uint32_t iter) { poll_report(poll, tag, iter, 1); }
 
 // Tile of kRelaxThreads partition sources per CTA (grid-stride).  Each thread
 // claims one source (async: only if its label is set, clearing it), the CTA
@@ -1316,18 +1330,16 @@ __device__ __forceinline__ void relax_tile_phase(const RelaxArgs &a, TileSmem &s
   uint32_t &s_wbase = sm.wbase;
   int &s_skip = sm.skip;
   const int tid = threadIdx.x;
-  const uint32_t slot = a.iter & 3u;
+  const uint32_t slot = (a.base + a.iter) & 3u;
   if (tid == 0) {
     int skip = 0;
-    if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.iter - 1) & 3u]) == 0) skip = 1;
+    if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.base + a.iter - 1) & 3u]) == 0) skip = 1;
     s_skip = skip;
     if (blockIdx.x == 0) {
-      a.ctl->upd[(a.iter + 1) & 3u] = 0;
-      a.ctl->wl_count[(a.iter + 1) & 3u] = 0;
-      if (!skip) {
-        atomicAdd(&a.ctl->iters_run, 1u);
-        atomicAdd(&a.ctl->iters_total, 1u);
-      }
+      a.ctl->upd[(a.base + a.iter + 1) & 3u] = 0;
+      a.ctl->wl_count[(a.base + a.iter + 1) & 3u] = 0;
+      if (!skip) atomicAdd(&a.ctl->iters_total, 1u);
+      if (ASYNC) poll_report(a.poll, a.poll_tag, a.iter, skip);
     }
   }
   __syncthreads();
@@ -1498,19 +1510,17 @@ template <bool ASYNC, class Args>
 __device__ __forceinline__ bool iter_begin(const Args &a, CtaTally &t) {
   if (threadIdx.x == 0) {
     int skip = 0;
-    if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.iter - 1) & 3u]) == 0) skip = 1;
+    if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.base + a.iter - 1) & 3u]) == 0) skip = 1;
     t.skip = skip;
     t.edges = 0;
     t.srcs = 0;
     t.any = 0;
     t.done = 0;
     if (blockIdx.x == 0) {
-      a.ctl->upd[(a.iter + 1) & 3u] = 0;
-      a.ctl->wl_count[(a.iter + 1) & 3u] = 0;
-      if (!skip) {
-        atomicAdd(&a.ctl->iters_run, 1u);
-        atomicAdd(&a.ctl->iters_total, 1u);
-      }
+      a.ctl->upd[(a.base + a.iter + 1) & 3u] = 0;
+      a.ctl->wl_count[(a.base + a.iter + 1) & 3u] = 0;
+      if (!skip) atomicAdd(&a.ctl->iters_total, 1u);
+      if (ASYNC) poll_report(a.poll, a.poll_tag, a.iter, skip);
     }
   }
   __syncthreads();
@@ -1540,7 +1550,7 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_w
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<uint32_t> s_exp[kWarpsPerCta];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const uint32_t slot = a.iter & 3u;
+  const uint32_t slot = (a.base + a.iter) & 3u;
   if (!iter_begin<ASYNC>(a, s_tally)) return;
   bool any_update = false;
   unsigned long long my_edges = 0, my_srcs = 0;
@@ -1696,14 +1706,14 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_a
       if (__any_sync(0xffffffffu, past)) break;
     }
   }
-  warp_publish(s_tally, a.ctl, a.iter & 3u, lane, any_update, my_edges, my_srcs);
+  warp_publish(s_tally, a.ctl, (a.base + a.iter) & 3u, lane, any_update, my_edges, my_srcs);
 }
 
 // Chunk list of inner iteration `iter`: one warp per item.
 template <int ALGO, bool ASYNC, int W>
 __device__ __forceinline__ void relax_chunks_phase(const RelaxArgs &a) {
-  const uint32_t slot = a.iter & 3u;
-  if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.iter - 1) & 3u]) == 0) return;
+  const uint32_t slot = (a.base + a.iter) & 3u;
+  if (ASYNC && a.iter > 1 && ld_acquire_u32(&a.ctl->upd[(a.base + a.iter - 1) & 3u]) == 0) return;
   const uint32_t items = min(ld_acquire_u32(&a.ctl->wl_count[slot]), a.wl_cap);
   const int lane = threadIdx.x & 31;
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1746,7 +1756,6 @@ __global__ void k_hub_claim(uint32_t u, const uint32_t *value, uint8_t *l1, uint
   }
   ctl->hub_active = act;
   ctl->hub_value = value[u];
-  ctl->upd[1] = 0;
 }
 
 template <int ALGO, int W>
@@ -1755,13 +1764,11 @@ __global__ void k_relax_flat(const uint32_t *buf, const uint8_t *wbuf, uint32_t 
   if (!ctl->hub_active) return;
   const uint32_t sval = ctl->hub_value;
   if (!can_push<ALGO>(sval)) return;
-  bool any = false;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
     uint32_t dst, w;
     load_edge<W>(buf, j, pbits, dst, w, wbuf);
-    any |= relax_edge<ALGO>(sval, dst, w, value, nxt);
+    relax_edge<ALGO>(sval, dst, w, value, nxt);
   }
-  if (__syncthreads_or(any) && threadIdx.x == 0) atomicAdd(&ctl->upd[1], 1u);
 }
 
 // ---- label hand-off (shared/gpu_kernels.cu:515-534) ------------------------
@@ -1843,7 +1850,9 @@ struct PrArgs {
   double *qpush;             // push of each queued source (0: none this iteration)
   Ctl *ctl;
   uint32_t from, size, edge_from;
-  uint32_t iter;
+  uint32_t iter, base;
+  unsigned long long *poll;
+  uint32_t poll_tag;
   uint32_t pbits;
   uint32_t streamed;
   uint32_t stream_base;
@@ -1888,7 +1897,7 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<double> s_exp[kWarpsPerCta];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t slot = a.iter & 3u;
+  const uint32_t slot = (a.base + a.iter) & 3u;
   if (a.iter > 1) {  // k_pr_claim began the iteration and counted its sources
     if (ld_acquire_u32(&a.ctl->upd[slot]) == 0) return;
     if (threadIdx.x == 0) s_tally = CtaTally{};
@@ -1961,7 +1970,7 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_warp
                             [&](const uint32_t (&pos)[kRelaxUnroll], const double (&pv)[kRelaxUnroll],
                                 const bool (&ok)[kRelaxUnroll]) { pr_lane<W, false>(a, pos, pv, ok); });
   }
-  warp_publish(s_tally, a.ctl, a.iter & 3u, lane, my_srcs != 0, my_edges, my_srcs);
+  warp_publish(s_tally, a.ctl, (a.base + a.iter) & 3u, lane, my_srcs != 0, my_edges, my_srcs);
 }
 
 // Async inner iterations > 1 where some row is long: the partition's sources
@@ -1990,7 +1999,7 @@ __global__ void __launch_bounds__(kRelaxThreads) k_pr_claim(PrArgs a) {
     }
     srcs += __popc(__ballot_sync(0xffffffffu, act));
   }
-  warp_publish(s_tally, a.ctl, a.iter & 3u, lane, srcs != 0, 0, srcs);
+  warp_publish(s_tally, a.ctl, (a.base + a.iter) & 3u, lane, srcs != 0, 0, srcs);
 }
 
 // Single-vertex PR partition: the generate snapshot of its push.

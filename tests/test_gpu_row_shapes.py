@@ -119,3 +119,31 @@ def test_pagerank_async_long_and_short_rows(gpu, orc, tile_degree_max):
     # every vertex is left with a residual of at most acc, 1/0.15 of which can still arrive
     bound = (acc / 0.15) * rank + 3e-7 * rank
     assert np.all(np.abs(v - rank) <= bound)
+
+
+@pytest.mark.parametrize("inner_batch", [1, 2, 8])
+@pytest.mark.parametrize("max_inner", [0, 1, 2, 4, 5])
+def test_async_iterations_polled(gpu, orc, inner_batch, max_inner):
+    """The host follows the inner iterations through a word of mapped memory:
+    caps below, at and above the launches it keeps ahead, with and without the
+    trace (whose per-partition counts come from the device and add up)."""
+    import ctypes as C
+    g = gpu.Graph.rmat(12, 12, seed=5, weighted=True)
+    eng = gpu.Engine(g, budget_bytes=18 * g.n + 96 * 1024 + 9000 * 8, inner_batch=inner_batch)
+    src = int(g.pick_sources(1, seed=6)[0])
+    for algo in ("sssp", "cc"):
+        e = g.edges if algo == "sssp" else np.ascontiguousarray(g.ends)
+        ref = orc.run(algo, g.node_pointer, e, src)
+        eng.trace_enable(False)
+        vals, st = eng.run(algo, "async", src, max_inner=max_inner)
+        assert np.array_equal(vals, ref)
+        eng.trace_enable(True)
+        vals, st = eng.run(algo, "async", src, max_inner=max_inner)
+        assert np.array_equal(vals, ref)
+        cnt = C.c_uint64()
+        gpu.check(gpu.lib().sgw_trace_count(eng.h, C.byref(cnt)), "trace")
+        rec = np.zeros(cnt.value, gpu.TRACE_REC)
+        gpu.check(gpu.lib().sgw_trace_read(eng.h, rec.ctypes.data, cnt.value, C.byref(cnt)), "trace")
+        assert len(rec) == st["partitions"] and int(rec["inner_iterations"].sum()) == st["inner_iterations"]
+        if max_inner:
+            assert int(rec["inner_iterations"].max()) <= max_inner
