@@ -394,6 +394,8 @@ __device__ __forceinline__ bool gen_full(const GenArgs &a, uint32_t v0) {
 // the run's (count, edges) total.
 template <bool SEL>
 __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_count(GenArgs a) {
+  chain_wait();
+  chain_open();
   __shared__ GenTotals s_sum[kGenThreads / 32];
   const int lane = threadIdx.x & 31;
   const uint32_t t0 = blockIdx.x * a.run_tiles, t1 = min(a.num_tiles, t0 + a.run_tiles);
@@ -435,6 +437,8 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_count(GenArg
 // pointer entries.
 template <bool MASKS>
 __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_write(GenArgs a) {
+  chain_wait();
+  chain_open();
   __shared__ GenTotals s_sum[kGenThreads / 32];
   __shared__ unsigned long long s_warp[2][kGenThreads / 32];
   __shared__ uint32_t s_last;
@@ -567,6 +571,8 @@ __device__ __forceinline__ void gen_pr_select(const GenArgs &a, uint32_t tile, d
 }
 
 __global__ void __launch_bounds__(kGenPrThreads, 2) k_generate_count_pr(GenArgs a) {
+  chain_wait();
+  chain_open();
   __shared__ GenTotals s_sum[kGenPrThreads / 32];
   const uint32_t t0 = blockIdx.x * a.run_tiles, t1 = min(a.num_tiles, t0 + a.run_tiles);
   GenTotals sum{0, 0};
@@ -597,6 +603,8 @@ __global__ void __launch_bounds__(kGenPrThreads, 2) k_generate_count_pr(GenArgs 
 }
 
 __global__ void __launch_bounds__(kGenPrThreads, 2) k_generate_write_pr(GenArgs a) {
+  chain_wait();
+  chain_open();
   constexpr int kWarps = kGenPrThreads / 32, kParts = kGenPrRounds * kWarps;
   __shared__ GenTotals s_sum[kWarps];
   __shared__ unsigned long long s_part[kParts + 1];  // (round, warp): count << 32 | edges, then the tile's total
@@ -735,6 +743,8 @@ __global__ void __launch_bounds__(256) k_select_hist(uint32_t n, int algo, const
 // selection order; sel_bin = first bin at which it reaches `target`.
 __global__ void __launch_bounds__(kSelBins / 4) k_select_pick(int algo, const unsigned long long *hist,
                                                               unsigned long long target, Ctl *ctl) {
+  chain_wait();
+  chain_open();
   __shared__ unsigned long long s_part[kSelBins / 4 / 32];
   __shared__ uint32_t s_k;  // first position (selection order) reaching the target
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1302,7 +1312,11 @@ __device__ __forceinline__ void poll_report(unsigned long long *poll, uint32_t t
   }
 }
 // The same for the iteration after a capped partition's last.
-__global__ void k_poll_end(unsigned long long *poll, uint32_t tag, uint32_t iter) { poll_report(poll, tag, iter, 1); }
+__global__ void k_poll_end(unsigned long long *poll, uint32_t tag, uint32_t iter) {
+  chain_wait();
+  chain_open();
+  poll_report(poll, tag, iter, 1);
+}
 
 // Tile of kRelaxThreads partition sources per CTA (grid-stride).  Each thread
 // claims one source (async: only if its label is set, clearing it), the CTA
@@ -1547,6 +1561,7 @@ __device__ __forceinline__ void warp_publish(CtaTally &t, Ctl *ctl, uint32_t slo
 
 template <int ALGO, bool ASYNC, int W>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_warp(RelaxArgs a) {
+  chain_wait();
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<uint32_t> s_exp[kWarpsPerCta];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1672,6 +1687,7 @@ template <int ALGO, int W, bool HOST>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_all(RelaxArgs a,
                                                                                   unsigned long long units,
                                                                                   unsigned long long per_warp) {
+  chain_wait();
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<uint32_t> s_exp[kWarpsPerCta];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1740,6 +1756,7 @@ __device__ __forceinline__ void relax_chunks_phase(const RelaxArgs &a) {
 
 template <int ALGO, bool ASYNC, int W>
 __global__ void __launch_bounds__(kRelaxThreads) k_relax_chunks(RelaxArgs a) {
+  chain_wait();
   relax_chunks_phase<ALGO, ASYNC, W>(a);
 }
 
@@ -1783,6 +1800,8 @@ __global__ void k_mix(const uint32_t *queue, uint32_t from, uint32_t size, uint8
 // Every source of the partition is relaxed by its first pass: its labels are
 // taken now, so that what is set from here on marks improvements.
 __global__ void k_claim(const uint32_t *queue, uint32_t from, uint32_t size, uint8_t *l1, uint8_t *l2) {
+  chain_wait();
+  chain_open();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < size; i += gridDim.x * blockDim.x) {
     const uint32_t u = queue[from + i];
     l1[u] = 0;
@@ -1894,6 +1913,7 @@ __device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[k
 template <int W, bool HOST>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(PrArgs a, unsigned long long units,
                                                                                unsigned long long per_warp) {
+  chain_wait();
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<double> s_exp[kWarpsPerCta];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1944,6 +1964,8 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(
 // with the claim and the cut, which pays where rows are long.
 template <int W>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_warp(PrArgs a) {
+  chain_wait();
+  chain_open();
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<double> s_exp[kWarpsPerCta];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1977,6 +1999,8 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_warp
 // whose residual grew above acc are active again (value += delta; delta -= delta, atomically
 // against pushes still to come); their pushes go to qpush.
 __global__ void __launch_bounds__(kRelaxThreads) k_pr_claim(PrArgs a) {
+  chain_wait();
+  chain_open();
   __shared__ CtaTally s_tally;
   const int lane = threadIdx.x & 31;
   if (!iter_begin<true>(a, s_tally)) return;
@@ -2050,6 +2074,8 @@ __global__ void k_range_stats(const RangeInfo *__restrict__ ranges, uint32_t num
                               const uint32_t *__restrict__ queue, const uint32_t *__restrict__ ptr,
                               const Ctl *__restrict__ ctl, RangeStat *st,
                               const __nv_bfloat16 *__restrict__ w, uint32_t iter, uint32_t cap) {
+  chain_wait();
+  chain_open();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= num_ranges) return;

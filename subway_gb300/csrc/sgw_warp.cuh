@@ -12,6 +12,15 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   return m;
 }
 
+// First thing in a kernel that may be launched while its predecessor in the
+// stream still runs (programmatic dependent launch): waits for the predecessor
+// and its writes.  chain_open() then lets the successor's blocks be placed at
+// once, where they wait in turn; only the short kernels do that, since blocks
+// waiting beside a wide relaxation keep the registers that the next gather's
+// blocks need (PageRank-async 3.0 against 2.8 ms).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Warp-inclusive scan of a u32.
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
 #pragma unroll
