@@ -375,7 +375,8 @@ int sgw_device_info(int device, uint32_t *sm_count, uint64_t *total_bytes);
  * No counterpart in the reference, whose only schedule is: compact every
  * active vertex's edges, cut the queue greedily into budget-sized partitions,
  * process them in vertex order, iterate each async partition to convergence
- * (SGW_POLICY_PLAIN, the default, which this engine reproduces).
+ * (SGW_POLICY_PLAIN, the default, which this engine reproduces; in sync runs
+ * the rows that fit the edge buffers cross the host link once per run).
  *
  * SGW_POLICY_LEARNED cuts the vertex ids into static ranges that each fit one
  * edge buffer.  After every generate step a kernel counts each range's active

@@ -87,6 +87,8 @@ struct sgw_engine {
   uint64_t hub_iters = 0;        // single-vertex partitions relaxed (counted on the host)
   uint32_t *d_queue = nullptr, *d_ptr = nullptr;
   uint32_t *d_gmask = nullptr;             // generate: keep | clear bits per 16-vertex group
+  uint32_t *d_have = nullptr;              // edge cache: rows held, per 16-vertex group
+  EdgeCache cache{};                       // of the current run (have null: none)
   unsigned long long *d_tagg = nullptr;    // generate: per-tile totals
   GenTotals *d_runs = nullptr;             // and those of each CTA's run of tiles
   Ctl *d_ctl = nullptr;
@@ -425,7 +427,7 @@ enum Family { FAM_INT = 0, FAM_PR = 1 };
 constexpr uint32_t kGenMaxRuns = 2048;  // CTAs of a generate
 
 struct Layout {
-  size_t off, obase, tagg, runs, ctl, mlp, sel, gmask, hct;  // common
+  size_t off, obase, tagg, runs, ctl, mlp, sel, gmask, have, hct;  // common
   size_t value, l1, l2, queue, ptr, delta, qpush;     // family
   size_t parts, ranges, rstat, wl, buf[kMaxBuf], total;
   uint64_t cap;
@@ -465,6 +467,9 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
   L.ranges = take(sizeof(RangeInfo) * (size_t)L.max_parts);
   L.rstat = take(sizeof(RangeStat) * (size_t)L.max_parts);
   L.wl = take(sizeof(WorkItem) * (size_t)L.wl_cap);
+  // behind the vertex state, whose addresses matter: shifting the residuals by
+  // 32 KB moved their hottest sectors to other L2 slices and PageRank-async on 2^17 by 12%
+  L.have = take(4ull * ((n + kGenVPerLane - 1) / kGenVPerLane));
   for (uint32_t b = 0; b < kMaxBuf; ++b) L.buf[b] = b < nbuf ? take(cap * esz) : L.buf[0];
   L.total = p;
   return L;
@@ -506,6 +511,7 @@ int carve(sgw_engine *e, int fam, uint64_t cap) {
   e->d_runs = (GenTotals *)(b + L.runs);
   e->d_ctl = (Ctl *)(b + L.ctl);
   e->d_gmask = (uint32_t *)(b + L.gmask);
+  e->d_have = (uint32_t *)(b + L.have);
   e->d_hct = (unsigned long long *)(b + L.hct);
   e->d_value = (uint32_t *)(b + L.value);
   e->d_l1 = fam == FAM_INT ? (uint8_t *)(b + L.l1) : nullptr;
@@ -621,6 +627,7 @@ int launch_generate(sgw_engine *e, int consume, bool plan) {
   a.runs = e->d_runs;
   a.ctl = e->d_ctl;
   a.gmask = e->d_gmask;
+  a.have = e->cache.have;
   a.aligned = 1;
   if (plan) {
     a.parts = e->d_parts;
@@ -706,7 +713,7 @@ int generate_and_plan(sgw_engine *e, int consume) {
 
 bool is_hub(const sgw_engine *e, const Part &p) { return p.edge_count > e->cap; }
 
-void trace_partition(sgw_engine *e, uint32_t p, uint32_t inner) {
+void trace_partition(sgw_engine *e, uint32_t p, uint32_t inner, uint64_t bytes) {
   if (!e->trace_on) return;
   const Part &q = e->h_parts[p];
   sgw_trace_rec r;
@@ -720,7 +727,7 @@ void trace_partition(sgw_engine *e, uint32_t p, uint32_t inner) {
   r.active_edges = q.edge_count;
   r.iteration_active_nodes = e->num_active;
   r.iteration_active_edges = e->num_active_edges;
-  r.bytes_h2d = q.edge_count * (4ull * e->W + (e->use_w ? 1 : 0));
+  r.bytes_h2d = bytes;
   r.transfer = is_hub(e, q) ? 2 : 0;
   e->trace.push_back(r);
 }
@@ -800,9 +807,6 @@ int gather_into(sgw_engine *e, const Part &q, uint32_t b, cudaStream_t s) {
   return SGW_OK;
 }
 
-// In place of an edge buffer: the pass reads the host copy itself.
-constexpr uint32_t kFromHost = 0xffffffffu;
-
 HostEdges host_edges(const sgw_engine *e) {
   return HostEdges{HostChunks{e->d_hct, e->hs_ends.shift}, HostChunks{e->d_hct + kMaxHostChunks, e->hs_w.shift},
                    e->use_w ? 1u : 0u};
@@ -828,11 +832,11 @@ WarpCut cut_warps(const sgw_engine *e, const Part &q) {
 // the queue holds a source above tile_degree_max, its chunk list.
 template <int ALGO, bool ASYNC, int W>
 int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, uint8_t *cur,
-                      uint8_t *nxt, bool all) {
+                      uint8_t *nxt, bool all, int src) {
   RelaxArgs a;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
-  a.buf = b == kFromHost ? nullptr : e->d_buf[b];
+  a.buf = e->d_buf[b];
   a.value = e->d_value;
   a.cur = cur;
   a.nxt = nxt;
@@ -852,13 +856,14 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   a.streamed = e->cur_streamed;
   a.stream_base = (uint32_t)e->cur_stream_base;  // with the low words of off: offsets mod 2^32
   a.off = e->d_off;
-  a.wbuf = e->use_w && b != kFromHost ? e->d_wbuf[b] : nullptr;
+  a.wbuf = e->use_w ? e->d_wbuf[b] : nullptr;
   a.host = host_edges(e);
+  a.cache = e->cache;
   if (all) {
     const WarpCut c = cut_warps(e, q);
-    if (b == kFromHost) CK(chain(k_relax_all<ALGO, W, true>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
-    else CK(chain(k_relax_all<ALGO, W, false>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
-    CK(cudaGetLastError());
+    if (src == kSrcCache) CK(chain(k_relax_all<ALGO, W, kSrcCache>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
+    else if (src == kSrcHost) CK(chain(k_relax_all<ALGO, W, kSrcHost>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
+    else CK(chain(k_relax_all<ALGO, W, kSrcBuffer>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
     e->stats.launches += 1;
     e->stats.relax_launches += 1;
     return SGW_OK;
@@ -880,26 +885,26 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
 
 template <int ALGO, int W>
 int relax_dispatch_w(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async,
-                     uint8_t *cur, uint8_t *nxt, bool all) {
-  if (async) return launch_relax_pass<ALGO, true, W>(e, q, b, iter, cur, nxt, all);
-  return launch_relax_pass<ALGO, false, W>(e, q, b, iter, cur, nxt, all);
+                     uint8_t *cur, uint8_t *nxt, bool all, int src) {
+  if (async) return launch_relax_pass<ALGO, true, W>(e, q, b, iter, cur, nxt, all, src);
+  return launch_relax_pass<ALGO, false, W>(e, q, b, iter, cur, nxt, all, src);
 }
 
 template <int ALGO>
 int relax_dispatch(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async,
-                   uint8_t *cur, uint8_t *nxt, bool all) {
-  if (e->W == 1) return relax_dispatch_w<ALGO, 1>(e, q, b, iter, async, cur, nxt, all);
-  return relax_dispatch_w<ALGO, 2>(e, q, b, iter, async, cur, nxt, all);
+                   uint8_t *cur, uint8_t *nxt, bool all, int src) {
+  if (e->W == 1) return relax_dispatch_w<ALGO, 1>(e, q, b, iter, async, cur, nxt, all, src);
+  return relax_dispatch_w<ALGO, 2>(e, q, b, iter, async, cur, nxt, all, src);
 }
 
 // One PageRank inner iteration: the first pushes the generate step's snapshot
 // (every queued source), later async ones what has grown above acc again.
 template <int W>
-int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
+int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, int src) {
   PrArgs a;
   a.queue = e->d_queue;
   a.ptr = e->d_ptr;
-  a.buf = b == kFromHost ? nullptr : e->d_buf[b];
+  a.buf = e->d_buf[b];
   a.pval = e->d_pval;
   a.delta = e->d_delta;
   a.qpush = e->d_qpush;
@@ -918,6 +923,7 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
   a.acc = (double)e->params.pr_acc;
   a.damping = (double)e->params.pr_damping;
   a.host = host_edges(e);
+  a.cache = e->cache;
   // without a row above tile_degree_max a warp's 32 rows are short enough to
   // need no cut by edges, and the claim and the pushes fit one launch
   if (iter > 1 && e->max_degree <= e->opts.tile_degree_max) {
@@ -934,25 +940,26 @@ int launch_pr_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter) {
     e->stats.relax_launches += 1;
   }
   const WarpCut c = cut_warps(e, q);
-  if (b == kFromHost) CK(chain(k_pr_all<W, true>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
-  else CK(chain(k_pr_all<W, false>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
-  CK(cudaGetLastError());
+  if (src == kSrcCache) CK(chain(k_pr_all<W, kSrcCache>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
+  else if (src == kSrcHost) CK(chain(k_pr_all<W, kSrcHost>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
+  else CK(chain(k_pr_all<W, kSrcBuffer>, c.grid, kRelaxThreads, e->s_comp, a, c.units, c.per_warp));
   e->stats.launches += 1;
   e->stats.relax_launches += 1;
   return SGW_OK;
 }
 
-int launch_relax(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async, bool all) {
+int launch_relax(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, bool async, bool all,
+                 int src = kSrcBuffer) {
   if (e->params.algo == SGW_PR) {
-    return e->W == 1 ? launch_pr_pass<1>(e, q, b, iter) : launch_pr_pass<2>(e, q, b, iter);
+    return e->W == 1 ? launch_pr_pass<1>(e, q, b, iter, src) : launch_pr_pass<2>(e, q, b, iter, src);
   }
   uint8_t *cur = e->d_l1, *nxt = e->d_l2;
   if (async && (iter % 2 == 0)) std::swap(cur, nxt);  // ping-pong (sssp-async.cu:108-109)
   switch (e->params.algo) {
-    case SGW_BFS: return relax_dispatch<SGW_BFS>(e, q, b, iter, async, cur, nxt, all);
-    case SGW_SSSP: return relax_dispatch<SGW_SSSP>(e, q, b, iter, async, cur, nxt, all);
-    case SGW_SSWP: return relax_dispatch<SGW_SSWP>(e, q, b, iter, async, cur, nxt, all);
-    case SGW_CC: return relax_dispatch<SGW_CC>(e, q, b, iter, async, cur, nxt, all);
+    case SGW_BFS: return relax_dispatch<SGW_BFS>(e, q, b, iter, async, cur, nxt, all, src);
+    case SGW_SSSP: return relax_dispatch<SGW_SSSP>(e, q, b, iter, async, cur, nxt, all, src);
+    case SGW_SSWP: return relax_dispatch<SGW_SSWP>(e, q, b, iter, async, cur, nxt, all, src);
+    case SGW_CC: return relax_dispatch<SGW_CC>(e, q, b, iter, async, cur, nxt, all, src);
     default: return fail(SGW_EINVAL, "algorithm %d not supported", e->params.algo);
   }
 }
@@ -1106,6 +1113,9 @@ int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_o
   return SGW_OK;
 }
 
+// Bytes per edge that this run moves.
+uint64_t run_rec(const sgw_engine *e) { return 4ull * e->W + (e->use_w ? 1 : 0); }
+
 // Whether a sync pass reads the host copy itself instead of a gathered
 // buffer.  Each partition of a sync iteration is relaxed once, so gathering
 // it first only adds a trip through HBM and, for the first partition, the wait
@@ -1116,14 +1126,32 @@ bool sync_from_host(const sgw_engine *e) {
          !(e->opts.flags & (SGW_OPT_SCALAR_GATHER | SGW_OPT_CTA_TILES | SGW_OPT_NO_OVERLAP));
 }
 
+// The edge cache of a plain sync run that may queue a vertex more than once
+// (BFS levels do not): the edge buffers hold the graph's first records, as many
+// as fit, instead of partitions.  A vertex beyond a buffer is streamed through
+// one, so graphs with such vertices go without.
+void cache_setup(sgw_engine *e, bool run_loop) {
+  e->cache = EdgeCache{};
+  if (!run_loop || !sync_from_host(e) || e->policy != SGW_POLICY_PLAIN || e->params.algo == SGW_BFS) return;
+  for (const RangeInfo &r : e->ranges)
+    if (r.e1 - r.e0 > e->cap) return;
+  const uint64_t space = (uint64_t)(e->d_arena + e->arena_bytes - (char *)e->d_buf[0]);
+  const uint64_t edges = std::min<uint64_t>(e->m, (space - std::min<uint64_t>(space, 256)) / run_rec(e));
+  if (edges == 0) return;
+  e->cache.buf = e->d_buf[0];
+  e->cache.wbuf = e->use_w ? (uint8_t *)e->d_buf[0] + 4ull * edges : nullptr;
+  e->cache.have = e->d_have;
+  e->cache.edges = (uint32_t)edges;
+}
+
 // One sync pass over partition q, its records read over the host link.
 int process_from_host(sgw_engine *e, const Part &q) {
   size_t slot = 0;
   TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
-  TRY(launch_relax(e, q, kFromHost, 1, false, true));
+  TRY(launch_relax(e, q, 0, 1, false, true, e->cache.have ? kSrcCache : kSrcHost));
   e->iter_base += 1;
   TRY(prof_end(e, e->s_comp, slot));
-  e->stats.h2d_bytes += q.edge_count * (4ull * e->W + (e->use_w ? 1 : 0));
+  if (!e->cache.have) e->stats.h2d_bytes += q.edge_count * run_rec(e);  // else counted on the device
   return SGW_OK;
 }
 
@@ -1171,6 +1199,8 @@ int state_init(sgw_engine *e, const sgw_run_params *p, bool take_labels) {
                                                           e->d_l1, e->d_l2);
   CK(cudaGetLastError());
   CK(cudaMemsetAsync(e->d_ctl, 0, sizeof(Ctl), e->s_comp));
+  cache_setup(e, take_labels);
+  if (e->cache.have) CK(cudaMemsetAsync(e->d_have, 0, 4ull * ((e->n + kGenVPerLane - 1) / kGenVPerLane), e->s_comp));
   e->stats.launches += 1;
   const bool async = p->mode == SGW_ASYNC;
   const int consume = !async || take_labels ? 1 : 0;
@@ -1199,7 +1229,13 @@ int process_iteration(sgw_engine *e) {
       const Part &q = e->h_parts[p];
       if (is_hub(e, q)) TRY(process_hub(e, q, 0));
       else TRY(process_from_host(e, q));
-      trace_partition(e, p, 1);
+      uint64_t bytes = q.edge_count * run_rec(e);
+      if (e->cache.have && e->trace_on && !is_hub(e, q)) {
+        const uint64_t before = e->h_ctl->host_edges;
+        TRY(read_ctl(e));
+        bytes = (e->h_ctl->host_edges - before) * run_rec(e);
+      }
+      trace_partition(e, p, 1, bytes);
       e->stats.partitions += 1;
     }
     return SGW_OK;
@@ -1217,7 +1253,7 @@ int process_iteration(sgw_engine *e) {
       TRY(process_resident(e, q, b, e->trace_on ? &inner : nullptr, p == 0));
     }
     CK(cudaEventRecord(e->ev_free[b], e->s_comp));
-    trace_partition(e, p, inner);
+    trace_partition(e, p, inner, q.edge_count * run_rec(e));
     if (e->nbuf == 1 && p + 1 < P) TRY(enqueue_gather(e, p + 1, e->s_copy));
     e->stats.partitions += 1;
   }
@@ -1923,7 +1959,7 @@ int sgw_process_partition(sgw_engine *e, uint32_t i, uint32_t *inner_iterations)
   TRY(read_ctl(e));
   e->stats.partitions += 1;
   if (i == 0) e->gitr += 1;
-  trace_partition(e, i, iters);
+  trace_partition(e, i, iters, q.edge_count * run_rec(e));
   if (inner_iterations) *inner_iterations = iters;
   return SGW_OK;
 }
@@ -2099,6 +2135,7 @@ int sgw_run(sgw_engine *e, const sgw_run_params *p, void *out_values, sgw_run_st
   e->stats.reached_edges = pr ? e->m : e->h_ctl->reached_edges;
   e->stats.relaxed_edges = e->h_ctl->relaxed_edges;
   e->stats.relaxed_sources = e->h_ctl->relaxed_sources;
+  e->stats.h2d_bytes += e->h_ctl->host_edges * run_rec(e);
   e->stats.inner_iterations = (uint64_t)e->h_ctl->iters_total + e->hub_iters;
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, e->ev_t0, e->ev_t1));
@@ -2179,6 +2216,7 @@ extern "C" int sgw_generate_noalloc(uint8_t *d_label1, uint8_t *d_label2,
   a.runs = reinterpret_cast<GenTotals *>(scratch + kNaRunsOff);
   a.ctl = ctl;
   a.gmask = nullptr;
+  a.have = nullptr;
   // a caller's arrays may start anywhere: 16-byte words only where all three allow them
   a.aligned = ((reinterpret_cast<uintptr_t>(d_label1) | reinterpret_cast<uintptr_t>(d_label2) |
                 reinterpret_cast<uintptr_t>(d_node_pointer)) & 15u) == 0;

@@ -65,6 +65,7 @@ struct Ctl {
   unsigned long long reached_edges;
   unsigned long long relaxed_edges;
   unsigned long long relaxed_sources;
+  unsigned long long host_edges;  // records that caching passes read from the host copy
   double hub_push;           // single-vertex PR partition: its push value
   Part first[kCtlParts];     // the partition table's first entries
 };
@@ -119,6 +120,7 @@ struct GenArgs {
   uint32_t run_tiles;        // tiles per CTA
   Ctl *ctl;
   uint32_t *gmask;           // per 16-vertex group, keep bits | clear bits << 16 (null: recomputed)
+  uint32_t *have;            // edge cache, per group: rows held | rows stored since << 16 (null: no cache)
   uint32_t num_tiles;
   int aligned;               // the label, pointer and value arrays start on 16-byte boundaries
   int consume;               // sync: labels of queued vertices are cleared
@@ -381,6 +383,13 @@ __device__ __forceinline__ void gen_finish(const GenArgs &a, uint32_t *s_last) {
   if (a.parts) plan_cta(a.ptr, a.queue, a.ctl, a.parts, a.max_parts, a.cap);
 }
 
+// Rows that the passes since the last generate have stored in the edge cache are
+// held from now on.
+__device__ __forceinline__ void gen_have(const GenArgs &a, uint32_t v0) {
+  const uint32_t h = a.have[v0 / kGenVPerLane];
+  if (h >> 16) a.have[v0 / kGenVPerLane] = (h | h >> 16) & 0xffffu;
+}
+
 __device__ __forceinline__ uint32_t gen_v0(uint32_t tile) {
   return tile * kGenTile + (threadIdx.x >> 5) * (32 * kGenRounds) + (threadIdx.x & 31) * kGenVPerLane;
 }
@@ -411,6 +420,7 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_count(GenArg
     next = GenLabels();
     if (tile + 1 < t1) gen_labels(a, gen_v0(tile + 1), gen_full(a, gen_v0(tile + 1)), next);
     if (v0 < a.n) {
+      if (a.have) gen_have(a, v0);
       gen_select<SEL>(a, v0, full, L);
       if (a.gmask) {
         if (!a.edge_limit) gen_clear(a, v0, full, L);
@@ -580,6 +590,12 @@ __global__ void __launch_bounds__(kGenPrThreads, 2) k_generate_count_pr(GenArgs 
   for (uint32_t tile = t0; tile < t1; ++tile) {
     double dl[kGenPrRounds];
     uint32_t deg[kGenPrRounds];
+    if (a.have && threadIdx.x % kGenVPerLane == 0)
+#pragma unroll
+      for (int r = 0; r < kGenPrRounds; ++r) {
+        const uint32_t v = tile * kGenTile + r * kGenPrThreads + threadIdx.x;
+        if (v < a.n) gen_have(a, v);
+      }
     gen_pr_select(a, tile, dl, deg);
     GenTotals x{0, 0};
 #pragma unroll
@@ -1273,6 +1289,72 @@ __device__ __forceinline__ void load_edge_host(const HostEdges &h, uint32_t e, u
   }
 }
 
+// Edge cache of a sync run: the edge buffers, which passes that read the host
+// copy leave unused, hold the first `edges` records of the graph at their own
+// positions.  A row that lies among them is stored as its first pass reads it
+// and read from there afterwards; `have` says which rows those are.  Sync runs
+// are bound by the host link: PageRank-sync on an Erdos-Renyi graph of 16 M
+// edges in memory 15.2 -> 8.4 ms, on R-MAT 2^20 with half the edges' room 14.1 ->
+// 11.7 ms, CC-sync on 32 M arcs (half) 1.66 -> 1.45 ms, SSSP-sync on 2^25
+// vertices (half) 18.0 -> 14.3 ms.
+struct EdgeCache {
+  uint32_t *buf;
+  uint8_t *wbuf;             // split form: the weight bytes
+  uint32_t *have;            // per 16 vertices: rows held | rows stored since the last generate << 16
+  uint32_t edges;
+};
+// Where a first pass finds a partition's records.
+constexpr int kSrcBuffer = 0;  // gathered (or streamed) into an edge buffer
+constexpr int kSrcHost = 1;    // in the host copy
+constexpr int kSrcCache = 2;   // in the edge cache or the host copy
+
+enum : uint32_t { kRowHost = 0, kRowStore = 1, kRowHeld = 2 };
+__device__ __forceinline__ uint32_t cache_row(const EdgeCache &c, uint32_t u, uint32_t off, uint32_t deg) {
+  if ((unsigned long long)off + deg > c.edges) return kRowHost;
+  return (c.have[u >> 4] >> (u & 15u)) & 1u ? kRowHeld : kRowStore;
+}
+// The row's first pass (one lane of it): held from the next generate on.
+__device__ __forceinline__ void cache_stored(const EdgeCache &c, uint32_t u) {
+  atomicOr(&c.have[u >> 4], 0x10000u << (u & 15u));
+}
+
+template <int W>
+__device__ __forceinline__ void load_edge_cached(const HostEdges &h, const EdgeCache &c, uint32_t how, uint32_t e,
+                                                 uint32_t pbits, uint32_t &dst, uint32_t &w) {
+  if (W == 1) {
+    uint32_t r, x = 0;
+    if (how == kRowHeld) {
+      r = c.buf[e];
+      if (h.split) x = c.wbuf[e];
+    } else {
+      r = *reinterpret_cast<const uint32_t *>(hc_at(h.ends, (size_t)e * 4));
+      if (h.split) x = *reinterpret_cast<const uint8_t *>(hc_at(h.w, e));
+      if (how == kRowStore) {
+        c.buf[e] = r;
+        if (h.split) c.wbuf[e] = (uint8_t)x;
+      }
+    }
+    if (pbits) { dst = r & ((1u << pbits) - 1u); w = r >> pbits; }
+    else { dst = r; w = x; }
+  } else {
+    uint2 ed;
+    if (how == kRowHeld) ed = reinterpret_cast<const uint2 *>(c.buf)[e];
+    else {
+      ed = *reinterpret_cast<const uint2 *>(hc_at(h.ends, (size_t)e * 8));
+      if (how == kRowStore) reinterpret_cast<uint2 *>(c.buf)[e] = ed;
+    }
+    dst = ed.x;
+    w = ed.y;
+  }
+}
+
+// What an edge needs of its source in a first pass: its value and, with the
+// cache, where its row is.
+template <class T>
+struct CachedRow { T val; uint32_t how; };
+template <class T, int SRC> struct RowOf { using V = T; };
+template <class T> struct RowOf<T, kSrcCache> { using V = CachedRow<T>; };
+
 struct RelaxArgs {
   const uint32_t *queue;
   const uint32_t *ptr;
@@ -1298,6 +1380,7 @@ struct RelaxArgs {
   const uint32_t *off;
   const uint8_t *wbuf;       // split form: the buffer's weight bytes (else null)
   HostEdges host;            // first passes that read the host copy themselves
+  EdgeCache cache;
 };
 
 constexpr int kRelaxThreads = 256;
@@ -1478,7 +1561,7 @@ __global__ void __launch_bounds__(kRelaxThreads) k_relax_tile(RelaxArgs a) {
 
 // Relaxes the kRelaxUnroll edges of a lane: all record loads, then all
 // destination values, then the compares and reductions.
-template <int ALGO, int W, bool HOST = false>
+template <int ALGO, int W, int SRC = kSrcBuffer>
 __device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&pos)[kRelaxUnroll],
                                            const uint32_t (&sv)[kRelaxUnroll], const bool (&ok)[kRelaxUnroll]) {
   uint32_t dst[kRelaxUnroll], w[kRelaxUnroll], cur[kRelaxUnroll];
@@ -1486,7 +1569,7 @@ __device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
     if (ok[q]) {
-      if (HOST) load_edge_host<W>(a.host, pos[q], a.pbits, dst[q], w[q]);
+      if (SRC == kSrcHost) load_edge_host<W>(a.host, pos[q], a.pbits, dst[q], w[q]);
       else load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w[q], a.wbuf);
     }
 #pragma unroll
@@ -1495,6 +1578,28 @@ __device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
     if (ok[q]) any |= relax_edge_seen<ALGO>(sv[q], dst[q], w[q], cur[q], a.value, a.nxt);
+  return any;
+}
+
+// The same with the edge cache.
+template <int ALGO, int W, int SRC>
+__device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&pos)[kRelaxUnroll],
+                                           const CachedRow<uint32_t> (&sv)[kRelaxUnroll],
+                                           const bool (&ok)[kRelaxUnroll]) {
+  uint32_t dst[kRelaxUnroll], w[kRelaxUnroll], cur[kRelaxUnroll];
+  bool go[kRelaxUnroll];
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) load_edge_cached<W>(a.host, a.cache, sv[q].how, pos[q], a.pbits, dst[q], w[q]);
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q) {
+    go[q] = ok[q] && can_push<ALGO>(sv[q].val);  // a row is stored whole whether or not it pushes
+    if (go[q]) cur[q] = a.value[dst[q]];
+  }
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (go[q]) any |= relax_edge_seen<ALGO>(sv[q].val, dst[q], w[q], cur[q], a.value, a.nxt);
   return any;
 }
 
@@ -1513,7 +1618,7 @@ constexpr int kWarpsPerCta = kRelaxThreads / 32;
 
 // Counters of a CTA whose warps finish independently.
 struct CtaTally {
-  unsigned long long edges, srcs;
+  unsigned long long edges, srcs, host;
   uint32_t any, done;
   int skip;
 };
@@ -1528,6 +1633,7 @@ __device__ __forceinline__ bool iter_begin(const Args &a, CtaTally &t) {
     t.skip = skip;
     t.edges = 0;
     t.srcs = 0;
+    t.host = 0;
     t.any = 0;
     t.done = 0;
     if (blockIdx.x == 0) {
@@ -1543,11 +1649,13 @@ __device__ __forceinline__ bool iter_begin(const Args &a, CtaTally &t) {
 
 // End of a warp's share; the CTA's last warp publishes.
 __device__ __forceinline__ void warp_publish(CtaTally &t, Ctl *ctl, uint32_t slot, int lane, bool any,
-                                             unsigned long long edges, unsigned long long srcs) {
+                                             unsigned long long edges, unsigned long long srcs,
+                                             unsigned long long host = 0) {
   const bool warp_any = __any_sync(0xffffffffu, any);
   if (lane == 0) {
     if (edges) atomicAdd(&t.edges, edges);
     if (srcs) atomicAdd(&t.srcs, srcs);
+    if (host) atomicAdd(&t.host, host);
     if (warp_any) atomicOr(&t.any, 1u);
     __threadfence_block();
     if (atomicAdd(&t.done, 1u) == kWarpsPerCta - 1) {
@@ -1555,6 +1663,7 @@ __device__ __forceinline__ void warp_publish(CtaTally &t, Ctl *ctl, uint32_t slo
       if (t.any) atomicAdd(&ctl->upd[slot], 1u);
       if (t.edges) atomicAdd(&ctl->relaxed_edges, t.edges);
       if (t.srcs) atomicAdd(&ctl->relaxed_sources, t.srcs);
+      if (t.host) atomicAdd(&ctl->host_edges, t.host);
     }
   }
 }
@@ -1674,7 +1783,7 @@ __device__ __forceinline__ uint32_t unit_clip(unsigned long long start, uint32_t
   return a < hi ? (uint32_t)(hi - a) : 0u;
 }
 
-// With HOST the records are read over the host link by the pass itself (a
+// With kSrcHost the records are read over the host link by the pass itself (a
 // partition that is relaxed once: every sync pass), at edge off[u] + j of the
 // host copy, so nothing is written to an edge buffer and read back, and the
 // relaxation hides behind the link.  Bound by the link (211 GB/s by DMA):
@@ -1682,25 +1791,28 @@ __device__ __forceinline__ uint32_t unit_clip(unsigned long long start, uint32_t
 // before: 1.45 + 0.78 ms partly overlapped, now 1.43), PageRank-sync's query on
 // R-MAT 2^20 went from 21.1 to 16.1 ms.  The windows of a tile start on
 // multiples of 32 edges there (warp_expand's align): without it each one
-// touches two 128-byte lines and CC's passes take 1.65 ms.
-template <int ALGO, int W, bool HOST>
+// touches two 128-byte lines and CC's passes take 1.65 ms.  kSrcCache: see
+// EdgeCache.
+template <int ALGO, int W, int SRC>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_all(RelaxArgs a,
                                                                                   unsigned long long units,
                                                                                   unsigned long long per_warp) {
   chain_wait();
   __shared__ CtaTally s_tally;
-  __shared__ WarpExpand<uint32_t> s_exp[kWarpsPerCta];
+  constexpr bool kHost = SRC != kSrcBuffer, kCache = SRC == kSrcCache;
+  using V = typename RowOf<uint32_t, SRC>::V;
+  __shared__ WarpExpand<V> s_exp[kWarpsPerCta];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   iter_begin<false>(a, s_tally);
   bool any_update = false;
-  unsigned long long my_edges = 0, my_srcs = 0;
+  unsigned long long my_edges = 0, my_srcs = 0, my_host = 0;
   const unsigned long long t0 = per_warp * (blockIdx.x * kWarpsPerCta + wid);
   const unsigned long long t1 = min(units, t0 + per_warp);
   if (t0 < t1) {
     const uint32_t first = warp_find_unit<kRelaxHeader>(a.ptr, a.from, a.size, a.edge_from, t0, lane);
     for (uint32_t i0 = first; i0 < a.size; i0 += 32) {
       const uint32_t idx = i0 + lane;
-      uint32_t d = 0, boff = 0, val = 0;
+      uint32_t d = 0, boff = 0, val = 0, how = kRowHost;
       bool past = true, head = false;
       if (idx < a.size) {
         const uint32_t p0 = a.ptr[a.from + idx], p1 = a.ptr[a.from + idx + 1];
@@ -1711,18 +1823,34 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_a
         d = unit_clip<kRelaxHeader>(start, p1 - p0, t0, t1, &lo, &head);
         if (d || head) {
           val = a.value[u];
-          if (!can_push<ALGO>(val)) { d = 0; head = false; }
-          boff = (HOST ? a.off[u] : a.streamed ? a.off[u] - a.stream_base : p0 - a.edge_from) + lo;
+          boff = (kHost ? a.off[u] : a.streamed ? a.off[u] - a.stream_base : p0 - a.edge_from) + lo;
+          if (kCache) {
+            how = cache_row(a.cache, u, boff - lo, p1 - p0);
+            if (head && how == kRowStore) cache_stored(a.cache, u);
+          }
+          if (!can_push<ALGO>(val)) {
+            head = false;
+            if (!kCache) d = 0;
+          }
         }
       }
       my_srcs += __popc(__ballot_sync(0xffffffffu, head));
-      my_edges += warp_expand(s_exp[wid], lane, d, boff, val,
-                              [&](const uint32_t (&pos)[kRelaxUnroll], const uint32_t (&sv)[kRelaxUnroll],
-                                  const bool (&ok)[kRelaxUnroll]) { any_update |= relax_lane<ALGO, W, HOST>(a, pos, sv, ok); }, HOST);
+      V row;
+      if constexpr (kCache) {
+        row.val = val;
+        row.how = how;
+        my_host += __reduce_add_sync(0xffffffffu, how != kRowHeld ? d : 0u);
+      } else {
+        row = val;
+      }
+      my_edges += warp_expand(s_exp[wid], lane, d, boff, row,
+                              [&](const uint32_t (&pos)[kRelaxUnroll], const V (&sv)[kRelaxUnroll],
+                                  const bool (&ok)[kRelaxUnroll]) { any_update |= relax_lane<ALGO, W, SRC>(a, pos, sv, ok); },
+                              kHost);
       if (__any_sync(0xffffffffu, past)) break;
     }
   }
-  warp_publish(s_tally, a.ctl, (a.base + a.iter) & 3u, lane, any_update, my_edges, my_srcs);
+  warp_publish(s_tally, a.ctl, (a.base + a.iter) & 3u, lane, any_update, my_edges, my_srcs, my_host);
 }
 
 // Chunk list of inner iteration `iter`: one warp per item.
@@ -1879,6 +2007,7 @@ struct PrArgs {
   double acc;
   double damping;
   HostEdges host;
+  EdgeCache cache;
 };
 
 __device__ __forceinline__ double ld_relaxed_f64(const double *p) {
@@ -1889,19 +2018,31 @@ __device__ __forceinline__ double ld_relaxed_f64(const double *p) {
 
 // Adds each edge's push to its destination's residual: the records of
 // kRelaxUnroll edges of a lane are loaded before their (non-returning) adds.
-template <int W, bool HOST>
+template <int W, int SRC>
 __device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[kRelaxUnroll],
                                         const double (&push)[kRelaxUnroll], const bool (&ok)[kRelaxUnroll]) {
   uint32_t dst[kRelaxUnroll], w;
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
     if (ok[q]) {
-      if (HOST) load_edge_host<W>(a.host, pos[q], a.pbits, dst[q], w);
+      if (SRC == kSrcHost) load_edge_host<W>(a.host, pos[q], a.pbits, dst[q], w);
       else load_edge<W>(a.buf, pos[q], a.pbits, dst[q], w);
     }
 #pragma unroll
   for (int q = 0; q < kRelaxUnroll; ++q)
     if (ok[q]) atomicAdd(&a.delta[dst[q]], push[q]);
+}
+template <int W, int SRC>
+__device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[kRelaxUnroll],
+                                        const CachedRow<double> (&row)[kRelaxUnroll],
+                                        const bool (&ok)[kRelaxUnroll]) {
+  uint32_t dst[kRelaxUnroll], w;
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) load_edge_cached<W>(a.host, a.cache, row[q].how, pos[q], a.pbits, dst[q], w);
+#pragma unroll
+  for (int q = 0; q < kRelaxUnroll; ++q)
+    if (ok[q]) atomicAdd(&a.delta[dst[q]], row[q].val);
 }
 
 // Pushes of one inner iteration, the work cut by edges as in k_relax_all:
@@ -1910,12 +2051,14 @@ __device__ __forceinline__ void pr_lane(const PrArgs &a, const uint32_t (&pos)[k
 // not active again) has written.  PageRank's later rounds queue a few tens of
 // thousands of long rows, which left most of the chip idle when each CTA took
 // 256 of them and found its edges' owners by binary search.
-template <int W, bool HOST>
+template <int W, int SRC>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(PrArgs a, unsigned long long units,
                                                                                unsigned long long per_warp) {
   chain_wait();
   __shared__ CtaTally s_tally;
-  __shared__ WarpExpand<double> s_exp[kWarpsPerCta];
+  constexpr bool kHost = SRC != kSrcBuffer, kCache = SRC == kSrcCache;
+  using V = typename RowOf<double, SRC>::V;
+  __shared__ WarpExpand<V> s_exp[kWarpsPerCta];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t slot = (a.base + a.iter) & 3u;
   if (a.iter > 1) {  // k_pr_claim began the iteration and counted its sources
@@ -1925,14 +2068,14 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(
   } else {
     iter_begin<false>(a, s_tally);
   }
-  unsigned long long my_edges = 0, my_srcs = 0;
+  unsigned long long my_edges = 0, my_srcs = 0, my_host = 0;
   const unsigned long long t0 = per_warp * (blockIdx.x * kWarpsPerCta + wid);
   const unsigned long long t1 = min(units, t0 + per_warp);
   if (t0 < t1) {
     const uint32_t first = warp_find_unit<kRelaxHeader>(a.ptr, a.from, a.size, a.edge_from, t0, lane);
     for (uint32_t i0 = first; i0 < a.size; i0 += 32) {
       const uint32_t idx = i0 + lane;
-      uint32_t d = 0, boff = 0;
+      uint32_t d = 0, boff = 0, how = kRowHost;
       double push = 0.0;
       bool past = true, head = false;
       if (idx < a.size) {
@@ -1943,17 +2086,33 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(
         past = start >= t1;
         uint32_t lo;
         d = unit_clip<kRelaxHeader>(start, p1 - p0, t0, t1, &lo, &head);
-        if (push == 0.0) d = 0;
-        if (d) boff = (HOST ? a.off[a.queue[i]] : a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from) + lo;
+        if (push == 0.0 && !kCache) d = 0;
+        if (d || (kCache && head)) {
+          boff = (kHost ? a.off[a.queue[i]] : a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from) + lo;
+          if (kCache) {
+            const uint32_t u = a.queue[i];
+            how = cache_row(a.cache, u, boff - lo, p1 - p0);
+            if (head && how == kRowStore) cache_stored(a.cache, u);
+          }
+        }
       }
       if (a.iter == 1) my_srcs += __popc(__ballot_sync(0xffffffffu, head));
-      my_edges += warp_expand(s_exp[wid], lane, d, boff, push,
-                              [&](const uint32_t (&pos)[kRelaxUnroll], const double (&pv)[kRelaxUnroll],
-                                  const bool (&ok)[kRelaxUnroll]) { pr_lane<W, HOST>(a, pos, pv, ok); }, HOST);
+      V row;
+      if constexpr (kCache) {
+        row.val = push;
+        row.how = how;
+        my_host += __reduce_add_sync(0xffffffffu, how != kRowHeld ? d : 0u);
+      } else {
+        row = push;
+      }
+      my_edges += warp_expand(s_exp[wid], lane, d, boff, row,
+                              [&](const uint32_t (&pos)[kRelaxUnroll], const V (&rv)[kRelaxUnroll],
+                                  const bool (&ok)[kRelaxUnroll]) { pr_lane<W, SRC>(a, pos, rv, ok); },
+                              kHost);
       if (__any_sync(0xffffffffu, past)) break;
     }
   }
-  warp_publish(s_tally, a.ctl, slot, lane, my_srcs != 0, my_edges, my_srcs);
+  warp_publish(s_tally, a.ctl, slot, lane, my_srcs != 0, my_edges, my_srcs, my_host);
 }
 
 // Async inner iterations > 1 of a partition without long rows: one launch in
@@ -1990,7 +2149,7 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_warp
     my_srcs += __popc(__ballot_sync(0xffffffffu, d > 0));
     my_edges += warp_expand(s_exp[wid], lane, d, boff, push,
                             [&](const uint32_t (&pos)[kRelaxUnroll], const double (&pv)[kRelaxUnroll],
-                                const bool (&ok)[kRelaxUnroll]) { pr_lane<W, false>(a, pos, pv, ok); });
+                                const bool (&ok)[kRelaxUnroll]) { pr_lane<W, kSrcBuffer>(a, pos, pv, ok); });
   }
   warp_publish(s_tally, a.ctl, (a.base + a.iter) & 3u, lane, my_srcs != 0, my_edges, my_srcs);
 }

@@ -147,3 +147,42 @@ def test_async_iterations_polled(gpu, orc, inner_batch, max_inner):
         assert len(rec) == st["partitions"] and int(rec["inner_iterations"].sum()) == st["inner_iterations"]
         if max_inner:
             assert int(rec["inner_iterations"].max()) <= max_inner
+
+
+@pytest.mark.parametrize("form", [f[0] for f in FORMS])
+@pytest.mark.parametrize("share", [0.0, 0.3, 0.8])
+def test_sync_edge_cache(gpu, orc, form, share):
+    """Sync runs keep the rows that fit the edge buffers: without a budget
+    every record crosses the link once however often its vertex is queued, with
+    one the rest is read again; the trace's bytes add up to the run's."""
+    import ctypes as C
+    opts = dict(dict(FORMS)[form])
+    flags = getattr(gpu, opts.pop("flags"), 0) if "flags" in opts else 0
+    g = gpu.Graph.rmat(13, 11, seed=31, weighted=True, wmax=200)
+    budget = int(36.3 * g.n + 160 * 1024 + share * 8 * g.m) if share else 0
+    eng = gpu.Engine(g, budget_bytes=budget, flags=flags, **opts)
+    src = int(g.pick_sources(1, seed=5)[0])
+    deg = g.out_degree()
+    for algo in ("cc", "sssp", "sswp", "pr"):
+        e = g.edges if algo in ("sssp", "sswp") else np.ascontiguousarray(g.ends)
+        eng.trace_enable(True)
+        vals, st = eng.run(algo, "sync", src)
+        if algo != "pr":
+            ref = orc.run(algo, g.node_pointer, e, src)
+            assert np.array_equal(vals, ref), algo
+        cnt = C.c_uint64()
+        gpu.check(gpu.lib().sgw_trace_count(eng.h, C.byref(cnt)), "trace")
+        rec = np.zeros(cnt.value, gpu.TRACE_REC)
+        gpu.check(gpu.lib().sgw_trace_read(eng.h, rec.ctypes.data, cnt.value, C.byref(cnt)), "trace")
+        assert int(rec["bytes_h2d"].sum()) == st["h2d_bytes"]
+        eng.trace_enable(False)
+        again, st2 = eng.run(algo, "sync", src)  # nothing is carried from run to run
+        assert st2["h2d_bytes"] == st["h2d_bytes"] or share
+        if algo != "pr":
+            assert np.array_equal(again, ref)
+        per_edge = {"packed": 4, "chunks": 4, "records": 8, "in_place": 8}.get(form) or (5 if algo in ("sssp", "sswp") else 4)
+        assert st["h2d_bytes"] <= st["active_edges"] * per_edge
+        if not share:
+            once = g.m if algo in ("cc", "pr") else int(deg[ref != (4294967294 if algo == "sssp" else 0)].sum())
+            assert st["h2d_bytes"] == once * per_edge, algo
+            assert st["active_edges"] > once, algo  # vertices were queued again
