@@ -330,10 +330,12 @@ __device__ __forceinline__ void b_bfs_relax(const BState &s, WarpExpand<BRow> *e
 // whichever wins), so non-returning reductions suffice and the lane bits are
 // right.  In a small frontier, bound by latency, a query whose distance has
 // improved again since the frontier phase is left to the next iteration, which
-// it is in anyway, so the number of iterations does not hang on timing; in a
-// large one its fresh distance is used, which saves a fifth of the time.
+// it is in anyway: next bits are set before distances are lowered and read
+// after them, so no distance travels two edges in one iteration and the number
+// of iterations does not hang on timing.  In a large one a fresh distance is
+// used at once, which saves a fifth of the time.
 constexpr int kBGroup = 2;
-constexpr uint32_t kBLarge = 65536;  // work units
+constexpr uint32_t kBLarge = 32768;  // work units
 
 template <int W, int L>
 __device__ __forceinline__ void b_sssp_relax(const BState &s, WarpExpand<BRow> *exp, unsigned long long total) {
@@ -385,7 +387,10 @@ __device__ __forceinline__ void b_sssp_relax(const BState &s, WarpExpand<BRow> *
                   du = make_uint4(kBInf, kBInf, kBInf, kBInf);
                   if (on & 15u) {
                     du = __ldcg(reinterpret_cast<const uint4 *>(dist + (size_t)ru * L));
-                    if (!large) on &= ~(__ldcg(reinterpret_cast<const uint32_t *>(&s.mask[ru].next) + h) >> (4 * c));
+                    if (!large) {
+                      __threadfence();  // a distance improved in this iteration comes after its next bit
+                      on &= ~(__ldcg(reinterpret_cast<const uint32_t *>(&s.mask[ru].next) + h) >> (4 * c));
+                    }
                     if (!(on & 1u)) du.x = kBInf;
                     if (!(on & 2u)) du.y = kBInf;
                     if (!(on & 4u)) du.z = kBInf;
@@ -410,6 +415,10 @@ __device__ __forceinline__ void b_sssp_relax(const BState &s, WarpExpand<BRow> *
                 m |= __shfl_xor_sync(0xffffffffu, m, 2);
                 m |= __shfl_xor_sync(0xffffffffu, m, 4);
                 if (c == 0 && m) atomicOr(&s.mask[dst[q]].next, (unsigned long long)m << (32 * h));
+                if (!large) {  // uniform: the bits before the distances
+                  __threadfence();
+                  __syncwarp();
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                   if ((imp >> i) & 1u) atomicMin(dist + (size_t)dst[q] * L + i, cand[i]);
