@@ -4,7 +4,7 @@ Times candidate settings of the engine options that shape the kernels
 (tile_degree_max: sources above it leave the CTA tile for the chunk list;
 chunk_edges: edges per chunk-list item; gather_ctas: gather grid) on a short
 sample of the actual workload, greedily one option at a time, and returns the
-fastest.  For batched queries it tunes the edges per work item.  Nothing here
+fastest.  For batched queries it tunes the fewest edges of a warp's share.  Nothing here
 changes results: every candidate computes the same fixpoint.
 """
 from __future__ import annotations
@@ -15,7 +15,7 @@ from . import native as N
 
 ENGINE_SPACE = {
     "tile_degree_max": (64, 128, 256, 512, 1024),
-    "chunk_edges": (256, 512, 1024, 2048),
+    "chunk_edges": (128, 256, 512, 1024, 2048),
     "gather_ctas_per_sm": (1, 2, 3, 4),
 }
 
@@ -45,7 +45,7 @@ def tune_engine(g, budget, algo="sssp", mode="async", sources=None, policy="plai
     """Greedy coordinate search; returns (best option dict, trials)."""
     if sources is None:
         sources = g.pick_sources(2, seed=11)
-    best = {"tile_degree_max": 256, "chunk_edges": 1024, "gather_ctas_per_sm": 2}
+    best = {"tile_degree_max": 128, "chunk_edges": 256, "gather_ctas_per_sm": 2}
     if num_buffers:
         best["num_buffers"] = num_buffers
     trials = []

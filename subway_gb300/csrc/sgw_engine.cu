@@ -424,6 +424,13 @@ int read_ctl(sgw_engine *e) {
 // followed by the partition table, the chunk list and the edge buffers.
 enum Family { FAM_INT = 0, FAM_PR = 1 };
 
+// Where a row is long enough for the chunk list, and the list's pieces.  Later
+// inner iterations are short and bound by the longest warp: with 128 / 256
+// against 256 / 1024 SSSP-async in memory on R-MAT 2^16 takes 333 us (388),
+// SSWP-async on 1.3 M vertices 1.60 ms (1.67), one-query SSSP on 2^21 3.60 ms
+// (3.64), learned SSSP-async on 2^25 24.3 ms (24.5); 64 / 128 gains only the first.
+constexpr uint32_t kTileDegreeMax = 128, kChunkEdges = 256;
+
 constexpr uint32_t kGenMaxRuns = 2048;  // CTAs of a generate
 
 struct Layout {
@@ -1518,8 +1525,8 @@ void sgw_engine_opts_default(sgw_engine_opts *o) {
   o->device = 0;
   o->flags = 0;
   o->inner_batch = 8;
-  o->tile_degree_max = 256;
-  o->chunk_edges = 1024;
+  o->tile_degree_max = kTileDegreeMax;
+  o->chunk_edges = kChunkEdges;
   o->sched_inner = 3;
   o->sched_active_permille = 1;
   o->sched_flags = SGW_SCHED_CAP_COMPACT;
@@ -1606,8 +1613,8 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   sgw_engine_opts_default(&o);
   if (opts_in) o = *opts_in;
   if (o.inner_batch == 0) o.inner_batch = 8;
-  if (o.tile_degree_max == 0) o.tile_degree_max = 256;
-  if (o.chunk_edges == 0) o.chunk_edges = 1024;
+  if (o.tile_degree_max == 0) o.tile_degree_max = kTileDegreeMax;
+  if (o.chunk_edges == 0) o.chunk_edges = kChunkEdges;
   if (o.chunk_edges % 32) return fail(SGW_EINVAL, "chunk_edges must be a multiple of 32");
   if (g->weighted && (((uintptr_t)g->edges) & 7u)) return fail(SGW_EINVAL, "edges must be 8-byte aligned");
   if (g->n >= 0x80000000u) return fail(SGW_ERANGE, "vertex count %u above 2^31", g->n);
