@@ -87,7 +87,6 @@ struct sgw_engine {
   uint64_t hub_iters = 0;        // single-vertex partitions relaxed (counted on the host)
   uint32_t *d_queue = nullptr, *d_ptr = nullptr;
   uint32_t *d_gmask = nullptr;             // generate: keep | clear bits per 16-vertex group
-  uint32_t *d_have = nullptr;              // edge cache: rows held, per 16-vertex group
   EdgeCache cache{};                       // of the current run (have null: none)
   unsigned long long *d_tagg = nullptr;    // generate: per-tile totals
   GenTotals *d_runs = nullptr;             // and those of each CTA's run of tiles
@@ -434,27 +433,41 @@ constexpr uint32_t kTileDegreeMax = 128, kChunkEdges = 256;
 constexpr uint32_t kGenMaxRuns = 2048;  // CTAs of a generate
 
 struct Layout {
-  size_t off, obase, tagg, runs, ctl, mlp, sel, gmask, have, hct;  // common
+  size_t off, obase, tagg, runs, ctl, mlp, sel, gmask, hct;  // common
   size_t value, l1, l2, queue, ptr, delta, qpush;     // family
   size_t parts, ranges, rstat, wl, buf[kMaxBuf], total;
   uint64_t cap;
   uint32_t max_parts, wl_cap;
 };
 
+// Tiles whose totals a generate under an edge limit keeps (without one: none).
+uint32_t limit_tiles(const sgw_engine *e) { return e->edge_limit ? e->num_tiles : 0; }
+
+// Most items that a chunk list for `cap` edges can hold: a row of d > tdm edges
+// makes ceil(d / chunk), which is below d / tdm where chunk >= 2 tdm.
+uint64_t chunk_items(uint64_t cap, uint32_t chunk, uint32_t tdm) {
+  tdm = std::max<uint32_t>(tdm, 1);
+  return cap / tdm + (chunk >= 2ull * tdm ? 0 : cap / chunk) + 2;
+}
+
 Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
-                   uint32_t num_tiles, uint64_t cap, uint32_t chunk, uint32_t tdm, bool wide) {
+                   uint32_t limit_tiles, uint64_t cap, uint32_t chunk, uint32_t tdm, bool wide) {
   Layout L{};
   size_t p = 0;
   auto take = [&](size_t bytes) { size_t at = p; p += align_up(bytes, 256); return at; };
   L.off = take(4ull * (n + 1));
   L.obase = take(wide ? 8ull * ((n >> kOffGroupLog2) + 2) : 0);
-  L.tagg = take(8ull * num_tiles);
+  const uint32_t num_tiles = (n + kGenTile - 1) / kGenTile;
   L.runs = take(sizeof(GenTotals) * std::min(num_tiles, kGenMaxRuns));
   L.ctl = take(sizeof(Ctl));
   L.mlp = take(sizeof(__nv_bfloat16) * kMlpParams);
   L.sel = take(sizeof(unsigned long long) * kSelBins);
   L.gmask = take(4ull * ((n + kGenVPerLane - 1) / kGenVPerLane));
   L.hct = take(2ull * kMaxHostChunks * sizeof(unsigned long long));
+  // the regions up to here lie alike in both families.  PageRank keeps the tile
+  // totals' space in any case: residuals 512 bytes lower had their hottest
+  // sectors on other L2 slices, and PageRank-async on 2^17 took 3.21 instead of 2.83 ms
+  L.tagg = take(8ull * (fam == FAM_PR ? num_tiles : limit_tiles));
   if (fam == FAM_INT) {
     L.value = take(4ull * n);
     L.l1 = take(n);
@@ -469,14 +482,11 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
   L.cap = cap;
   L.max_parts = (uint32_t)std::min<uint64_t>(2ull * ((uint64_t)m / std::max<uint64_t>(cap, 1) + 1) + 2,
                                              0x7fffffffull);
-  L.wl_cap = (uint32_t)std::min<uint64_t>(cap / chunk + cap / std::max<uint32_t>(tdm, 1) + 64, 0x7fffffffull);
+  L.wl_cap = (uint32_t)std::min<uint64_t>(chunk_items(cap, chunk, tdm), 0x7fffffffull);
   L.parts = take(sizeof(Part) * (size_t)L.max_parts);
   L.ranges = take(sizeof(RangeInfo) * (size_t)L.max_parts);
   L.rstat = take(sizeof(RangeStat) * (size_t)L.max_parts);
-  L.wl = take(sizeof(WorkItem) * (size_t)L.wl_cap);
-  // behind the vertex state, whose addresses matter: shifting the residuals by
-  // 32 KB moved their hottest sectors to other L2 slices and PageRank-async on 2^17 by 12%
-  L.have = take(4ull * ((n + kGenVPerLane - 1) / kGenVPerLane));
+  L.wl = take(fam == FAM_INT ? sizeof(WorkItem) * (size_t)L.wl_cap : 0);  // PageRank has no chunk list
   for (uint32_t b = 0; b < kMaxBuf; ++b) L.buf[b] = b < nbuf ? take(cap * esz) : L.buf[0];
   L.total = p;
   return L;
@@ -484,9 +494,9 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
 
 // Largest edge-buffer capacity whose layout fits `bytes` (0 if none does).
 uint64_t fit_cap(int fam, const sgw_engine_opts &o, uint32_t n, uint64_t m, uint32_t esz,
-                 uint32_t nbuf, uint32_t num_tiles, uint64_t bytes, bool wide) {
+                 uint32_t nbuf, uint32_t limit_tiles, uint64_t bytes, bool wide) {
   auto total = [&](uint64_t cap) {
-    return (uint64_t)make_layout(fam, n, m, esz, nbuf, num_tiles, cap, o.chunk_edges, o.tile_degree_max, wide).total;
+    return (uint64_t)make_layout(fam, n, m, esz, nbuf, limit_tiles, cap, o.chunk_edges, o.tile_degree_max, wide).total;
   };
   // max_partition_size <= DIST_INFINITY, and no larger than the whole graph
   const uint64_t hi_cap = std::min<uint64_t>(std::max<uint64_t>(m, 64), 4294967294ull);
@@ -494,7 +504,7 @@ uint64_t fit_cap(int fam, const sgw_engine_opts &o, uint32_t n, uint64_t m, uint
   // the buffers grow as cap.  Below the minimum nothing fits; above it the
   // size grows monotonically, so bisect for the largest cap that fits.
   const double table = 2.0 * m * (sizeof(Part) + sizeof(RangeInfo) + sizeof(RangeStat));
-  const double per_edge = (double)nbuf * esz + 16.0 / o.chunk_edges + 16.0 / o.tile_degree_max;
+  const double per_edge = (double)nbuf * esz + 16.0 * chunk_items(1u << 20, o.chunk_edges, o.tile_degree_max) / (1u << 20);
   uint64_t lo = std::max<uint64_t>(64, (uint64_t)std::sqrt(table / per_edge));
   lo = std::min(lo, hi_cap);
   if (total(lo) > bytes) return 0;
@@ -508,7 +518,7 @@ uint64_t fit_cap(int fam, const sgw_engine_opts &o, uint32_t n, uint64_t m, uint
 }
 
 int carve(sgw_engine *e, int fam, uint64_t cap) {
-  const Layout L = make_layout(fam, e->n, e->m, e->rec_bytes, e->nbuf, e->num_tiles, cap,
+  const Layout L = make_layout(fam, e->n, e->m, e->rec_bytes, e->nbuf, limit_tiles(e), cap,
                                e->opts.chunk_edges, e->opts.tile_degree_max, e->wide);
   if (L.total > e->arena_bytes) return fail(SGW_EBUDGET, "layout exceeds the arena");
   char *b = e->d_arena;
@@ -518,7 +528,6 @@ int carve(sgw_engine *e, int fam, uint64_t cap) {
   e->d_runs = (GenTotals *)(b + L.runs);
   e->d_ctl = (Ctl *)(b + L.ctl);
   e->d_gmask = (uint32_t *)(b + L.gmask);
-  e->d_have = (uint32_t *)(b + L.have);
   e->d_hct = (unsigned long long *)(b + L.hct);
   e->d_value = (uint32_t *)(b + L.value);
   e->d_l1 = fam == FAM_INT ? (uint8_t *)(b + L.l1) : nullptr;
@@ -1133,6 +1142,9 @@ bool sync_from_host(const sgw_engine *e) {
          !(e->opts.flags & (SGW_OPT_SCALAR_GATHER | SGW_OPT_CTA_TILES | SGW_OPT_NO_OVERLAP));
 }
 
+// Its held and stored bits, one word per 16 vertices, at the start of the buffers.
+size_t have_bytes(const sgw_engine *e) { return 4ull * ((e->n + kGenVPerLane - 1) / kGenVPerLane); }
+
 // The edge cache of a plain sync run that may queue a vertex more than once
 // (BFS levels do not): the edge buffers hold the graph's first records, as many
 // as fit, instead of partitions.  A vertex beyond a buffer is streamed through
@@ -1143,11 +1155,12 @@ void cache_setup(sgw_engine *e, bool run_loop) {
   for (const RangeInfo &r : e->ranges)
     if (r.e1 - r.e0 > e->cap) return;
   const uint64_t space = (uint64_t)(e->d_arena + e->arena_bytes - (char *)e->d_buf[0]);
-  const uint64_t edges = std::min<uint64_t>(e->m, (space - std::min<uint64_t>(space, 256)) / run_rec(e));
+  const uint64_t have = align_up(have_bytes(e), 256);
+  const uint64_t edges = std::min<uint64_t>(e->m, (space - std::min<uint64_t>(space, have + 256)) / run_rec(e));
   if (edges == 0) return;
-  e->cache.buf = e->d_buf[0];
-  e->cache.wbuf = e->use_w ? (uint8_t *)e->d_buf[0] + 4ull * edges : nullptr;
-  e->cache.have = e->d_have;
+  e->cache.have = e->d_buf[0];
+  e->cache.buf = (uint32_t *)((char *)e->d_buf[0] + have);
+  e->cache.wbuf = e->use_w ? (uint8_t *)e->cache.buf + 4ull * edges : nullptr;
   e->cache.edges = (uint32_t)edges;
 }
 
@@ -1207,7 +1220,7 @@ int state_init(sgw_engine *e, const sgw_run_params *p, bool take_labels) {
   CK(cudaGetLastError());
   CK(cudaMemsetAsync(e->d_ctl, 0, sizeof(Ctl), e->s_comp));
   cache_setup(e, take_labels);
-  if (e->cache.have) CK(cudaMemsetAsync(e->d_have, 0, 4ull * ((e->n + kGenVPerLane - 1) / kGenVPerLane), e->s_comp));
+  if (e->cache.have) CK(cudaMemsetAsync(e->cache.have, 0, have_bytes(e), e->s_comp));
   e->stats.launches += 1;
   const bool async = p->mode == SGW_ASYNC;
   const int consume = !async || take_labels ? 1 : 0;
@@ -1700,13 +1713,13 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   const uint64_t mfull = std::max<uint64_t>(e->m, 64);
   size_t need = 0;
   for (int fam = 0; fam < 2; ++fam)
-    need = std::max(need, make_layout(fam, e->n, e->m, esz, e->nbuf, e->num_tiles, mfull,
+    need = std::max(need, make_layout(fam, e->n, e->m, esz, e->nbuf, limit_tiles(e), mfull,
                                       o.chunk_edges, o.tile_degree_max, e->wide).total);
   uint64_t budget = o.budget_bytes;
   if (budget == 0) {
     // Subway's rule: 0.9 * (totalGlobalMem - 32 n) bytes of edges
     // (shared/subgraph.cu:24), here on top of the engine's own vertex state.
-    const Layout L0 = make_layout(FAM_PR, e->n, e->m, esz, e->nbuf, e->num_tiles, mfull,
+    const Layout L0 = make_layout(FAM_PR, e->n, e->m, esz, e->nbuf, limit_tiles(e), mfull,
                                   o.chunk_edges, o.tile_degree_max, e->wide);
     const double state = (double)L0.total - (double)e->nbuf * mfull * esz;  // all but the buffers
     double edges_bytes = 0.9 * ((double)prop.totalGlobalMem - 32.0 * e->n);
@@ -1714,13 +1727,13 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   }
   const size_t arena = (size_t)std::min<uint64_t>(budget, need);
   for (int fam = 0; fam < 2; ++fam) {
-    e->cap_fam[fam] = fit_cap(fam, o, e->n, e->m, esz, e->nbuf, e->num_tiles, arena, e->wide);
+    e->cap_fam[fam] = fit_cap(fam, o, e->n, e->m, esz, e->nbuf, limit_tiles(e), arena, e->wide);
     // split form: the weight bytes start at 4 * cap past a 256-byte aligned
     // buffer; a multiple of 4 keeps them 16-byte aligned for vector stores
     if (e->split && e->cap_fam[fam] > 16) e->cap_fam[fam] &= ~3ull;
   }
   if (e->cap_fam[FAM_INT] == 0) {
-    const Layout L0 = make_layout(FAM_INT, e->n, e->m, esz, e->nbuf, e->num_tiles, 4096,
+    const Layout L0 = make_layout(FAM_INT, e->n, e->m, esz, e->nbuf, limit_tiles(e), 4096,
                                   o.chunk_edges, o.tile_degree_max, e->wide);
     delete e;
     return fail(SGW_EBUDGET, "budget %llu B < vertex state and minimum edge buffers (about %zu B)",
@@ -1737,7 +1750,7 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   uint32_t parts_host = kCtlParts;
   for (int fam = 0; fam < 2; ++fam)
     if (e->cap_fam[fam])
-      parts_host = std::max(parts_host, make_layout(fam, e->n, e->m, esz, e->nbuf, e->num_tiles,
+      parts_host = std::max(parts_host, make_layout(fam, e->n, e->m, esz, e->nbuf, limit_tiles(e),
                                                     e->cap_fam[fam], o.chunk_edges, o.tile_degree_max, e->wide).max_parts);
 
   int st = SGW_OK;

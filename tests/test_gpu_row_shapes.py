@@ -186,3 +186,24 @@ def test_sync_edge_cache(gpu, orc, form, share):
             once = g.m if algo in ("cc", "pr") else int(deg[ref != (4294967294 if algo == "sssp" else 0)].sum())
             assert st["h2d_bytes"] == once * per_edge, algo
             assert st["active_edges"] > once, algo  # vertices were queued again
+
+
+@pytest.mark.parametrize("extra", [0, 2048, 6144, 8192, 20000])
+def test_sync_cache_bits_in_small_buffers(gpu, orc, extra):
+    """The edge cache's bits (n / 4 bytes) share the edge buffers: from the
+    smallest accepted budget, whose buffers do not hold them, across the line."""
+    g = gpu.Graph.er(30011, 60000, seed=9, weighted=True, wmax=60)
+    lo, hi = 18 * g.n, 18 * g.n + (1 << 20)  # refused, accepted
+    while hi - lo > 64:
+        mid = (lo + hi) // 2
+        try:
+            gpu.Engine(g, budget_bytes=mid).close()
+            hi = mid
+        except gpu.SgwError:
+            lo = mid
+    eng = gpu.Engine(g, budget_bytes=hi + extra)
+    src = int(g.pick_sources(1, seed=5)[0])
+    for algo in ("cc", "sssp"):
+        e = g.edges if algo == "sssp" else np.ascontiguousarray(g.ends)
+        vals, _ = eng.run(algo, "sync", src)
+        assert np.array_equal(vals, orc.run(algo, g.node_pointer, e, src)), algo
