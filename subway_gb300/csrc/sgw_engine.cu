@@ -2223,8 +2223,6 @@ extern "C" int sgw_generate_noalloc(uint8_t *d_label1, uint8_t *d_label2,
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Ctl *ctl = reinterpret_cast<Ctl *>(scratch + kNaCtlOff);
-  // the previous call's counters are not trusted: clear the control block
-  CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), s));
   GenArgs a;
   a.n = n;
   a.l1 = d_label1;
@@ -2247,8 +2245,7 @@ extern "C" int sgw_generate_noalloc(uint8_t *d_label1, uint8_t *d_label2,
   const uint32_t grid = cut_tiles(a, sms, kGenCtas);
   k_generate_count<false><<<grid, kGenThreads, 0, s>>>(a);
   CK(cudaGetLastError());
-  k_generate_write<false><<<grid, kGenThreads, 0, s>>>(a);
-  CK(cudaGetLastError());
+  CK(chain(k_generate_write<false>, grid, kGenThreads, s, a));
   Ctl h;
   CK(cudaMemcpyAsync(&h, ctl, offsetof(Ctl, num_parts), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));

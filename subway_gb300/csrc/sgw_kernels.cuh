@@ -437,14 +437,16 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_count(GenArg
     }
   }
   maxd = __reduce_max_sync(0xffffffffu, maxd);
-  if (lane == 0 && maxd) atomicMax(&a.ctl->degree_max, maxd);
+  if (lane == 0 && maxd && a.gmask) atomicMax(&a.ctl->degree_max, maxd);
   sum = gen_block_sum<kGenThreads>(sum, s_sum);
   if (threadIdx.x == 0) a.runs[blockIdx.x] = sum;
 }
 
-// Write pass: the group's keep bits from the count pass (MASKS) or selected
-// again, the node pointers of groups that queue a vertex, and the queue /
-// pointer entries.
+// Write pass: the group's keep bits from the count pass (MASKS: the engine's
+// generate) or selected again (a caller's arrays, where there is no room for the
+// bits, no plan to make and no counter to ready: 77 us for 16.8 M vertices, 86
+// with a memset of the control block and the last CTA's turn), the node pointers
+// of groups that queue a vertex, and the queue / pointer entries.
 template <bool MASKS>
 __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_write(GenArgs a) {
   chain_wait();
@@ -543,7 +545,7 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas) k_generate_write(GenArg
   }
   // past the last tile: the totals, unless a tile was beyond the limit
   if (t1 == a.num_tiles && !cut && tid == 0) gen_report(a, before);
-  gen_finish(a, &s_last);
+  if (MASKS) gen_finish(a, &s_last);
 }
 
 // PageRank's two passes (prePrefix PR overload, shared/subgraph_generator.cu:
