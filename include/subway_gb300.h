@@ -170,6 +170,9 @@ void sgw_graph_free(sgw_graph *g);
  * from the split copy.  Otherwise the flag is ignored (a transfer copy is
  * made, pageable with SGW_OPT_PAGEABLE_COPY).  The drop-in apps set both. */
 #define SGW_OPT_GRAPH_IN_PLACE 0x200u
+/* sgw_batch: the work units of 64 edges that graphs of about 2^35 edges and
+ * more take by themselves (see sgw_batch_unit_edges), on any graph. */
+#define SGW_OPT_BATCH_WIDE_UNITS 0x400u
 /* sched_flags: the learned policy's inner cap also covers compacted ranges */
 #define SGW_SCHED_CAP_COMPACT 0x1u
 /* sched_flags: transfer active vertices that cannot push, as the reference's
@@ -503,6 +506,10 @@ int sgw_batch_run_u16(sgw_batch *b, int algo, const uint32_t *sources, uint32_t 
  * SGW_ETIMEOUT when the kernel gave up and the device stayed usable; the
  * batch object can be used again afterwards. */
 int sgw_batch_check_wait_timeout(sgw_batch *b, uint64_t wait_ns);
+/* Edges of one work unit of a batch over a graph of n vertices and m edges: a
+ * frontier's units are counted in 32 bits, 8 edges each where
+ * 2 n + m / 8 < 2^32, else 64. */
+uint32_t sgw_batch_unit_edges(uint32_t n, uint64_t m);
 /* The batch's pinned result buffer (lanes x n, lane-major), valid until the
  * next sgw_batch_run or sgw_batch_destroy. */
 int sgw_batch_results(const sgw_batch *b, const uint32_t **results);

@@ -80,15 +80,16 @@ __global__ void k_b_seed(const uint32_t *src, uint32_t nsrc, uint32_t *dist, BMa
 // ---- frontier phase ----------------------------------------------------------------
 // Every vertex whose `next` mask holds a query that is new to it joins the
 // frontier: its mask moves to cur, and it gets a row in (rows, unit).  A row is
-// 1 + ceil(degree / kBUnit) work units; `unit` is its first one.  A CTA takes
+// 1 + ceil(degree / unit edges) work units; `unit` is its first one.  A CTA takes
 // kBVerts vertices at a time and reserves their rows and units with one
 // 64-bit add, so both counts are prefixes in the same order and the relax
-// phase can cut the units into equal shares.
+// phase can cut the units into equal shares.  The units of a frontier that
+// holds every vertex have to stay below 2^32: see b_unit_log2.
 //
 // Loads that follow writes made earlier in the same launch (the persistent
 // form runs every phase in one kernel) go through L2 (__ldcg): L1 and the
 // read-only path are not kept coherent within a kernel.
-constexpr uint32_t kBUnit = 8;    // edges
+constexpr uint32_t kBUnitLog2 = 3, kBWideUnitLog2 = 6;  // edges of a work unit: 8, or 64
 constexpr int kBPer = 4;          // vertices per thread
 constexpr uint32_t kBVerts = kBThreads * kBPer;
 
@@ -101,6 +102,7 @@ struct BState {
   BMask *mask;
   uint32_t *rows, *unit;         // frontier rows: vertex, first work unit
   uint32_t min_units;            // fewest units in a warp's share
+  uint32_t unit_log2;            // edges of a work unit
 };
 
 struct BFrontierSmem {
@@ -159,7 +161,7 @@ __device__ __forceinline__ void b_frontier(const BState &s, BFrontierSmem &sm, u
         ++act;
         const uint32_t deg = s.off[v + 1] - s.off[v];
         if (deg) {
-          units[k] = 1 + (deg + kBUnit - 1) / kBUnit;
+          units[k] = 2 + ((deg - 1) >> s.unit_log2);
           mine += units[k];
           ++rows;
         }
@@ -255,7 +257,8 @@ __device__ __forceinline__ void b_rows(const BState &s, unsigned long long total
         if (!past) {
           u = __ldcg(&s.rows[i]);
           const uint32_t deg = s.off[u + 1] - s.off[u];
-          const unsigned long long x = t0 > first ? (t0 - first) * kBUnit : 0, y = t1 > first ? (t1 - first) * kBUnit : 0;
+          const unsigned long long x = t0 > first ? (t0 - first) << s.unit_log2 : 0,
+                                   y = t1 > first ? (t1 - first) << s.unit_log2 : 0;
           const unsigned long long end = min(y, (unsigned long long)deg);
           if (x < end) {
             d = (uint32_t)(end - x);
@@ -618,6 +621,7 @@ struct sgw_batch {
   uint64_t m = 0;
   uint32_t lanes = 64;            // 32 or 64 distance columns
   uint32_t min_units = 0;         // option: fewest work units of a warp's share (0: by algorithm)
+  uint32_t unit_log2 = kBUnitLog2;
   char *d_arena = nullptr;
   size_t arena_bytes = 0;
   uint32_t *d_off = nullptr, *d_edges = nullptr, *d_dist = nullptr, *d_stage = nullptr;
@@ -641,6 +645,16 @@ namespace {
 
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
+// Edges of a work unit, as a power of two.  A frontier's units are counted in
+// the low 32 bits of a counter whose high word counts its rows, and a row of d
+// edges has 1 + ceil(d / unit) of them, so a frontier of n vertices and m edges
+// has at most 2 n + m / unit: 8 edges where that is below 2^32, 64 on larger
+// graphs (156 n bytes of state and 4 m of edges fit 288 GB only with fewer than
+// 2^32 of those).
+uint32_t b_unit_log2(uint64_t n, uint64_t m) {
+  return 2 * n + (m >> kBUnitLog2) < (uint64_t(1) << 32) ? kBUnitLog2 : kBWideUnitLog2;
+}
+
 BState state_of(const sgw_batch *b, bool sssp) {
   BState s;
   s.n = b->n;
@@ -656,6 +670,7 @@ BState state_of(const sgw_batch *b, bool sssp) {
   // a warp's share is at least 128 edges of BFS (one round of its loads) and 16 of
   // SSSP (two of its groups): a small frontier is spread over as many warps
   s.min_units = b->min_units ? b->min_units : sssp ? 2u : 16u;
+  s.unit_log2 = b->unit_log2;
   return s;
 }
 
@@ -775,7 +790,8 @@ int sgw_batch_create(const sgw_graph *g, const sgw_engine_opts *opts, uint32_t l
   b->n = g->n;
   b->m = g->m;
   b->lanes = lanes;
-  b->min_units = o.chunk_edges ? std::max<uint32_t>(1, o.chunk_edges / kBUnit) : 0;
+  b->unit_log2 = (o.flags & SGW_OPT_BATCH_WIDE_UNITS) ? kBWideUnitLog2 : b_unit_log2(g->n, g->m);
+  b->min_units = o.chunk_edges ? std::max<uint32_t>(1, o.chunk_edges >> b->unit_log2) : 0;
   if ((o.flags & SGW_OPT_BATCH_PERSISTENT) && (o.flags & SGW_OPT_BATCH_GRAPH)) {
     delete b;
     return sgw::fail(SGW_EINVAL, "SGW_OPT_BATCH_PERSISTENT and SGW_OPT_BATCH_GRAPH exclude each other");
@@ -886,6 +902,8 @@ int sgw_batch_results(const sgw_batch *b, const uint32_t **results) {
   *results = b->h_out;
   return SGW_OK;
 }
+
+uint32_t sgw_batch_unit_edges(uint32_t n, uint64_t m) { return 1u << b_unit_log2(n, m); }
 
 int sgw_batch_device_bytes(const sgw_batch *b, uint64_t *bytes) {
   if (!b || !bytes) return sgw::fail(SGW_EINVAL, "null argument");

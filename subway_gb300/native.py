@@ -28,6 +28,7 @@ OPT_BATCH_PERSISTENT = 0x40
 OPT_BATCH_GRAPH = 0x80
 OPT_PAGEABLE_COPY = 0x100
 OPT_GRAPH_IN_PLACE = 0x200
+OPT_BATCH_WIDE_UNITS = 0x400
 SCHED_CAP_COMPACT = 0x1
 SCHED_KEEP_IDLE = 0x2
 ALGOS = {"bfs": BFS, "sssp": SSSP, "sswp": SSWP, "cc": CC, "pr": PR}
@@ -120,6 +121,7 @@ _PROTOS = {
     "sgw_engine_dma_rate": (C.c_int, [_P, C.POINTER(C.c_double)]),
     "sgw_batch_create": (C.c_int, [_P, C.POINTER(EngineOpts), C.c_uint32, C.POINTER(_P)]),
     "sgw_batch_destroy": (C.c_int, [_P]),
+    "sgw_batch_unit_edges": (C.c_uint32, [C.c_uint32, C.c_uint64]),
     "sgw_batch_device_bytes": (C.c_int, [_P, _u64p]),
     "sgw_batch_run": (C.c_int, [_P, C.c_int, _P, C.c_uint32, _P, _P]),
     "sgw_batch_results": (C.c_int, [_P, C.POINTER(_P)]),
