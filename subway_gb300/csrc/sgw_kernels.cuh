@@ -1756,7 +1756,7 @@ constexpr uint32_t kRelaxMinUnits = 256;  // per warp: about one tile
 // Last source i in [0, size) that starts at or before unit t; every lane
 // returns it.  Source i starts at unit ptr[from + i] - edge_from + H * i.
 template <uint32_t H>
-__device__ __forceinline__ uint32_t warp_find_unit(const uint32_t *__restrict__ ptr, uint32_t from, uint32_t size,
+__device__ __forceinline__ uint32_t warp_find_unit(const uint32_t *ptr, uint32_t from, uint32_t size,
                                                    uint32_t edge_from, unsigned long long t, int lane) {
   uint32_t lo = 0, hi = size;
   auto le = [&](uint32_t i) {
@@ -2231,10 +2231,9 @@ struct RangeStat {           // one global iteration of one range
 // One warp per range: locate the range's queue segment, form the five
 // features, evaluate the network (or, with no weights, predict that the
 // current active edge fraction persists).
-__global__ void k_range_stats(const RangeInfo *__restrict__ ranges, uint32_t num_ranges,
-                              const uint32_t *__restrict__ queue, const uint32_t *__restrict__ ptr,
-                              const Ctl *__restrict__ ctl, RangeStat *st,
-                              const __nv_bfloat16 *__restrict__ w, uint32_t iter, uint32_t cap) {
+__global__ void k_range_stats(const RangeInfo *ranges, uint32_t num_ranges, const uint32_t *queue,
+                              const uint32_t *ptr, const Ctl *ctl, RangeStat *st, const __nv_bfloat16 *w,
+                              uint32_t iter, uint32_t cap) {
   chain_wait();
   chain_open();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -18,6 +18,10 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // once, where they wait in turn; only the short kernels do that, since blocks
 // waiting beside a wide relaxation keep the registers that the next gather's
 // blocks need (PageRank-async 3.0 against 2.8 ms).
+// Such a kernel's inputs change while it runs, up to its wait: no parameter is
+// `__restrict__`, and __ldg is for arrays that no kernel of the stream writes
+// (node pointers, the host chunk table); both would allow a load before the
+// wait.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
