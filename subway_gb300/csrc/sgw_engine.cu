@@ -104,6 +104,7 @@ struct sgw_engine {
   uint64_t cap = 0;  // edges per buffer
   uint32_t nbuf = 2;
   uint32_t max_parts = 0, wl_cap = 0, num_tiles = 0;
+  bool pr_place = true;                    // PageRank's residuals lie at kPrPlace
 
   // host side
   volatile unsigned long long *h_poll = nullptr;  // mapped: progress of the running partition
@@ -450,8 +451,20 @@ uint64_t chunk_items(uint64_t cap, uint32_t chunk, uint32_t tdm) {
   return cap / tdm + (chunk >= 2ull * tdm ? 0 : cap / chunk) + 2;
 }
 
+// Where PageRank's residuals start, modulo 2 KB of the arena.  The first 64
+// residuals fill 512 bytes, and an R-MAT graph's pushes go to the low ids above
+// all: started in the upper half of a kilobyte they spread over more L2 slices
+// than in the lower half.  Measured on 16 R-MAT graphs (2^13 .. 2^21 vertices,
+// async and sync), at 512 against the better of 0 and 256: faster on every one,
+// by 0.4 to 15% (2^16 vertices 3.02 and 2.61 ms, 2^17 4.43 and 3.80, 200 017
+// 5.50 and 4.70); 768 equals 512, and so does the other kilobyte of two but for
+// 200 017 (5.6).  Erdos-Renyi graphs take the same time anywhere.
+constexpr size_t kPrPlace = 512;
+
+// place: PageRank's residuals at kPrPlace (a budget that the up to 2 KB before
+// them would exceed goes without).
 Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
-                   uint32_t limit_tiles, uint64_t cap, uint32_t chunk, uint32_t tdm, bool wide) {
+                   uint32_t limit_tiles, uint64_t cap, uint32_t chunk, uint32_t tdm, bool wide, bool place) {
   Layout L{};
   size_t p = 0;
   auto take = [&](size_t bytes) { size_t at = p; p += align_up(bytes, 256); return at; };
@@ -464,16 +477,15 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
   L.sel = take(sizeof(unsigned long long) * kSelBins);
   L.gmask = take(4ull * ((n + kGenVPerLane - 1) / kGenVPerLane));
   L.hct = take(2ull * kMaxHostChunks * sizeof(unsigned long long));
-  // the regions up to here lie alike in both families.  PageRank keeps the tile
-  // totals' space in any case: residuals 512 bytes lower had their hottest
-  // sectors on other L2 slices, and PageRank-async on 2^17 took 3.21 instead of 2.83 ms
-  L.tagg = take(8ull * (fam == FAM_PR ? num_tiles : limit_tiles));
+  // the regions up to here lie alike in both families
+  L.tagg = take(8ull * limit_tiles);
   if (fam == FAM_INT) {
     L.value = take(4ull * n);
     L.l1 = take(n);
     L.l2 = take(n);
   } else {
     L.value = take(8ull * n);
+    if (place) p += (kPrPlace - p) & 2047u;
     L.delta = take(8ull * n);
   }
   L.queue = take(4ull * n);
@@ -494,9 +506,10 @@ Layout make_layout(int fam, uint32_t n, uint64_t m, uint32_t esz, uint32_t nbuf,
 
 // Largest edge-buffer capacity whose layout fits `bytes` (0 if none does).
 uint64_t fit_cap(int fam, const sgw_engine_opts &o, uint32_t n, uint64_t m, uint32_t esz,
-                 uint32_t nbuf, uint32_t limit_tiles, uint64_t bytes, bool wide) {
+                 uint32_t nbuf, uint32_t limit_tiles, uint64_t bytes, bool wide, bool place) {
   auto total = [&](uint64_t cap) {
-    return (uint64_t)make_layout(fam, n, m, esz, nbuf, limit_tiles, cap, o.chunk_edges, o.tile_degree_max, wide).total;
+    return (uint64_t)make_layout(fam, n, m, esz, nbuf, limit_tiles, cap, o.chunk_edges, o.tile_degree_max, wide,
+                                 place).total;
   };
   // max_partition_size <= DIST_INFINITY, and no larger than the whole graph
   const uint64_t hi_cap = std::min<uint64_t>(std::max<uint64_t>(m, 64), 4294967294ull);
@@ -519,7 +532,7 @@ uint64_t fit_cap(int fam, const sgw_engine_opts &o, uint32_t n, uint64_t m, uint
 
 int carve(sgw_engine *e, int fam, uint64_t cap) {
   const Layout L = make_layout(fam, e->n, e->m, e->rec_bytes, e->nbuf, limit_tiles(e), cap,
-                               e->opts.chunk_edges, e->opts.tile_degree_max, e->wide);
+                               e->opts.chunk_edges, e->opts.tile_degree_max, e->wide, e->pr_place);
   if (L.total > e->arena_bytes) return fail(SGW_EBUDGET, "layout exceeds the arena");
   char *b = e->d_arena;
   e->d_off = (uint32_t *)(b + L.off);
@@ -1714,27 +1727,31 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   size_t need = 0;
   for (int fam = 0; fam < 2; ++fam)
     need = std::max(need, make_layout(fam, e->n, e->m, esz, e->nbuf, limit_tiles(e), mfull,
-                                      o.chunk_edges, o.tile_degree_max, e->wide).total);
+                                      o.chunk_edges, o.tile_degree_max, e->wide, true).total);
   uint64_t budget = o.budget_bytes;
   if (budget == 0) {
     // Subway's rule: 0.9 * (totalGlobalMem - 32 n) bytes of edges
     // (shared/subgraph.cu:24), here on top of the engine's own vertex state.
     const Layout L0 = make_layout(FAM_PR, e->n, e->m, esz, e->nbuf, limit_tiles(e), mfull,
-                                  o.chunk_edges, o.tile_degree_max, e->wide);
+                                  o.chunk_edges, o.tile_degree_max, e->wide, true);
     const double state = (double)L0.total - (double)e->nbuf * mfull * esz;  // all but the buffers
     double edges_bytes = 0.9 * ((double)prop.totalGlobalMem - 32.0 * e->n);
     budget = (uint64_t)(state + std::max(0.0, edges_bytes));
   }
   const size_t arena = (size_t)std::min<uint64_t>(budget, need);
   for (int fam = 0; fam < 2; ++fam) {
-    e->cap_fam[fam] = fit_cap(fam, o, e->n, e->m, esz, e->nbuf, limit_tiles(e), arena, e->wide);
+    e->cap_fam[fam] = fit_cap(fam, o, e->n, e->m, esz, e->nbuf, limit_tiles(e), arena, e->wide, true);
+    if (fam == FAM_PR && e->cap_fam[fam] == 0) {
+      e->pr_place = false;
+      e->cap_fam[fam] = fit_cap(fam, o, e->n, e->m, esz, e->nbuf, limit_tiles(e), arena, e->wide, false);
+    }
     // split form: the weight bytes start at 4 * cap past a 256-byte aligned
     // buffer; a multiple of 4 keeps them 16-byte aligned for vector stores
     if (e->split && e->cap_fam[fam] > 16) e->cap_fam[fam] &= ~3ull;
   }
   if (e->cap_fam[FAM_INT] == 0) {
     const Layout L0 = make_layout(FAM_INT, e->n, e->m, esz, e->nbuf, limit_tiles(e), 4096,
-                                  o.chunk_edges, o.tile_degree_max, e->wide);
+                                  o.chunk_edges, o.tile_degree_max, e->wide, true);
     delete e;
     return fail(SGW_EBUDGET, "budget %llu B < vertex state and minimum edge buffers (about %zu B)",
                 (unsigned long long)budget, L0.total);
@@ -1751,7 +1768,8 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   for (int fam = 0; fam < 2; ++fam)
     if (e->cap_fam[fam])
       parts_host = std::max(parts_host, make_layout(fam, e->n, e->m, esz, e->nbuf, limit_tiles(e),
-                                                    e->cap_fam[fam], o.chunk_edges, o.tile_degree_max, e->wide).max_parts);
+                                                    e->cap_fam[fam], o.chunk_edges, o.tile_degree_max, e->wide,
+                                                    e->pr_place).max_parts);
 
   int st = SGW_OK;
   auto cleanup = [&](int s) { sgw_engine_destroy(e); return s; };
