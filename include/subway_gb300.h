@@ -188,7 +188,8 @@ typedef struct sgw_engine_opts {
   uint32_t flags;          /* SGW_OPT_*                                       */
   uint32_t inner_batch;    /* async inner iterations launched ahead, at most 3 */
   uint32_t tile_degree_max;/* sources above this degree go to the chunk list  */
-  uint32_t chunk_edges;    /* edges per chunk-list item (multiple of 32)      */
+  uint32_t chunk_edges;    /* edges per chunk-list item (multiple of 32), 0 = 256;
+                              sgw_batch reads it otherwise                    */
   uint32_t gather_ctas;    /* CTAs of the gather kernel, 0 = 2 per SM (3 per SM
                               under the learned policy)                      */
   uint32_t num_buffers;    /* device edge buffers sharing the budget, 0 = 2
@@ -470,7 +471,8 @@ int sgw_range_trace_read(const sgw_engine *e, sgw_range_rec *out, uint64_t capac
  * are bit-exact with single-source runs.
  * opts: budget_bytes (admission: SGW_EBUDGET if the graph, lanes x n
  * distances and the work lists do not fit), device, chunk_edges (fewest edges
- * that one warp's share of an iteration holds; 0: chosen by the algorithm),
+ * that one warp's share of an iteration holds, also above the share that the
+ * algorithm would take; 0, the default: chosen by the algorithm),
  * flags (SGW_OPT_NO_PACK). */
 typedef struct sgw_batch sgw_batch;
 typedef struct sgw_batch_stats {

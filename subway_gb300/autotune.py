@@ -71,7 +71,8 @@ def engine_opts(best: dict, device=0) -> dict:
     return o
 
 
-def tune_batch(g, algo="bfs", lanes=64, device=0, candidates=(64, 128, 256, 512, 1024), seed=3):
+def tune_batch(g, algo="bfs", lanes=64, device=0, candidates=(0, 64, 128, 256, 512, 1024), seed=3):
+    """Fastest chunk_edges of a batch (0: the batch's own choice) and the trials."""
     rng = np.random.default_rng(seed)
     src = rng.integers(0, g.n, lanes).astype(np.uint32)
     res = []

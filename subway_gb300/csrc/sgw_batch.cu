@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(kBThreads) k_b_frontier(BState s, uint32_t *ct
 }
 
 // ---- relax phase -------------------------------------------------------------------
-// The frontier's work units are cut into equal shares of at most `share`; a warp
+// The frontier's work units are cut into equal shares of at most `share` (at
+// least min_units, if the caller sets more than that); a warp
 // finds a share's first row with a 32-way search and goes through its rows 32
 // at a time, the first and the last clipped to the share.  (One warp per row or
 // per piece of 256 edges left most warps waiting at the end of an iteration for

@@ -1552,7 +1552,7 @@ void sgw_engine_opts_default(sgw_engine_opts *o) {
   o->flags = 0;
   o->inner_batch = 8;
   o->tile_degree_max = kTileDegreeMax;
-  o->chunk_edges = kChunkEdges;
+  o->chunk_edges = 0;  // the engine's or the batch's own
   o->sched_inner = 3;
   o->sched_active_permille = 1;
   o->sched_flags = SGW_SCHED_CAP_COMPACT;
