@@ -186,7 +186,8 @@ typedef struct sgw_engine_opts {
   uint64_t budget_bytes;
   int32_t device;          /* CUDA device ordinal (--device)                  */
   uint32_t flags;          /* SGW_OPT_*                                       */
-  uint32_t inner_batch;    /* async inner iterations launched ahead, at most 3 */
+  uint32_t inner_batch;    /* async inner iterations launched ahead of the last
+                              that is known to have begun, 0 = 3              */
   uint32_t tile_degree_max;/* sources above this degree go to the chunk list  */
   uint32_t chunk_edges;    /* edges per chunk-list item (multiple of 32), 0 = 256;
                               sgw_batch reads it otherwise                    */

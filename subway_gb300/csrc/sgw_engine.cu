@@ -431,6 +431,7 @@ enum Family { FAM_INT = 0, FAM_PR = 1 };
 // (3.64), learned SSSP-async on 2^25 24.3 ms (24.5); 64 / 128 gains only the first.
 constexpr uint32_t kTileDegreeMax = 128, kChunkEdges = 256;
 
+constexpr uint32_t kPollAhead = 3;      // opts.inner_batch by default
 constexpr uint32_t kGenMaxRuns = 2048;  // CTAs of a generate
 
 struct Layout {
@@ -1076,16 +1077,14 @@ int poll_wait(sgw_engine *e, uint64_t begun, uint64_t *iter, bool *done) {
 }
 
 // Relaxation of one resident partition: sync = one pass; async = inner
-// iterations until no relaxation improves (or max_inner), at most kPollAhead
-// of them launched beyond the last that is known to have begun, so that a
-// partition costs at most that many idle launches (batches of eight wasted a
-// third of them).  Returns when the partition is done.  The learned policy
+// iterations until no relaxation improves (or max_inner), at most
+// opts.inner_batch of them launched beyond the last that is known to have
+// begun, so that a partition costs at most that many idle launches (batches of
+// eight wasted a third of them; kPollAhead is the default).  Returns when the partition is done.  The learned policy
 // needs that wait: letting the host run ahead put more gathers beside each
 // relaxation and made both slower (RMAT-24 SSSP-async: 12.2 against 17.0
 // GTEPS).  iters_out: iterations that did work, counted on the device.
 // first: no partition of this global iteration has been relaxed before.
-constexpr uint32_t kPollAhead = 3;
-
 int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool first) {
   const bool async = e->params.mode == SGW_ASYNC;
   const bool tiles = (e->opts.flags & SGW_OPT_CTA_TILES) != 0;
@@ -1112,7 +1111,7 @@ int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_o
   }
   uint32_t max_inner = e->params.max_inner ? e->params.max_inner : 0xffffffffu;
   if (e->range_inner_cap) max_inner = std::min(max_inner, e->range_inner_cap);
-  const uint64_t ahead = std::min<uint64_t>(std::max<uint32_t>(1, e->opts.inner_batch), kPollAhead);
+  const uint64_t ahead = std::min(e->opts.inner_batch, 1024u);  // a stream queues about as many launches
   e->poll_tag = (e->poll_tag + 1) & 0xffffu;
   const uint64_t total0 = e->iters_known;
   uint64_t launched = 0, begun = 1;
@@ -1550,7 +1549,7 @@ void sgw_engine_opts_default(sgw_engine_opts *o) {
   o->budget_bytes = 0;
   o->device = 0;
   o->flags = 0;
-  o->inner_batch = 8;
+  o->inner_batch = kPollAhead;
   o->tile_degree_max = kTileDegreeMax;
   o->chunk_edges = 0;  // the engine's or the batch's own
   o->sched_inner = 3;
@@ -1638,7 +1637,7 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
   sgw_engine_opts o;
   sgw_engine_opts_default(&o);
   if (opts_in) o = *opts_in;
-  if (o.inner_batch == 0) o.inner_batch = 8;
+  if (o.inner_batch == 0) o.inner_batch = kPollAhead;
   if (o.tile_degree_max == 0) o.tile_degree_max = kTileDegreeMax;
   if (o.chunk_edges == 0) o.chunk_edges = kChunkEdges;
   if (o.chunk_edges % 32) return fail(SGW_EINVAL, "chunk_edges must be a multiple of 32");
