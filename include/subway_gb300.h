@@ -293,7 +293,10 @@ typedef struct sgw_run_stats {
 /* One whole application run: the init loops, the first generate, the
  * global-iteration / partition / inner-iteration loops and the final value
  * read-back of subway/<algo>-<mode>.cu (e.g. subway/sssp-async.cu:38-127).
- * out_values: host buffer of n uint32 (float for PR).  stats may be NULL. */
+ * out_values: host buffer of n uint32 (float for PR).  stats may be NULL.
+ * Async runs poll a word of host memory for the progress of each partition:
+ * a busy wait of some tens of microseconds, then one that yields its core to
+ * other threads, or sleeps under cudaDeviceScheduleBlockingSync. */
 int sgw_run(sgw_engine *e, const sgw_run_params *p, void *out_values,
             sgw_run_stats *stats);
 

@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <memory>
 #include <thread>
 #include <vector>
@@ -110,6 +111,7 @@ struct sgw_engine {
   volatile unsigned long long *h_poll = nullptr;  // mapped: progress of the running partition
   unsigned long long *d_poll = nullptr;
   uint32_t poll_tag = 0;
+  bool wait_blocks = false;                // cudaDeviceScheduleBlockingSync is set
   uint32_t iter_base = 0;                  // inner iterations launched so far in the run
   uint64_t iters_known = 0;                // inner iterations that did work, at the last read-back
   Ctl *h_ctl = nullptr;
@@ -1057,8 +1059,11 @@ int process_hub(sgw_engine *e, const Part &q, uint32_t b) {
 // Waits until the running partition reports an iteration later than `begun` (or
 // that it has converged) and returns the report.  The host polls mapped memory:
 // waiting for a copy of the control block instead left the GPU idle for about
-// 12 us per partition.
+// 12 us per partition.  After kPollSpins polls (some tens of microseconds) it
+// offers its core to other threads between two of them, and sleeps where the
+// device's schedule flag asks for waits that block.
 int poll_wait(sgw_engine *e, uint64_t begun, uint64_t *iter, bool *done) {
+  constexpr uint64_t kPollSpins = 16384;
   for (uint64_t spin = 1;; ++spin) {
     const unsigned long long x = *e->h_poll;
     if ((uint32_t)(x >> 48) == e->poll_tag) {
@@ -1066,7 +1071,10 @@ int poll_wait(sgw_engine *e, uint64_t begun, uint64_t *iter, bool *done) {
       *done = x & 1u;
       if (*iter > begun || *done) return SGW_OK;
     }
-    if (spin % 65536 == 0) {  // nothing for a while: a failed launch reports here
+    if (spin < kPollSpins) continue;
+    if (e->wait_blocks) std::this_thread::sleep_for(std::chrono::microseconds(20));
+    else std::this_thread::yield();
+    if (spin % 1024 == 0) {  // nothing for a while: a failed launch reports here
       const cudaError_t q = cudaStreamQuery(e->s_comp);
       if (q == cudaSuccess && *e->h_poll == x)
         return fail(SGW_ECUDA, "a partition's inner iterations ended without a report");
@@ -1716,6 +1724,10 @@ int sgw_engine_create(const sgw_graph *g, const sgw_engine_opts *opts_in, sgw_en
     e->nbuf = o.num_buffers;
   }
   e->num_tiles = (uint32_t)((g->n + kGenTile - 1) / kGenTile);
+  unsigned dev_flags = 0;
+  if (cudaGetDeviceFlags(&dev_flags) == cudaSuccess)
+    e->wait_blocks = (dev_flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
+  cudaGetLastError();
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, o.device) != cudaSuccess) { delete e; return fail(SGW_ECUDA, "device properties"); }
   e->num_sms = prop.multiProcessorCount;
