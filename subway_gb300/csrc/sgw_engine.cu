@@ -155,6 +155,7 @@ struct sgw_engine {
   // cleared the labels of what it queued, so a partition processed before any
   // other of its global iteration has none left to clear.
   bool labels_partial = false, labels_taken = false;
+  std::vector<char> part_done;             // step API: processed since the last generate
   uint32_t gitr = 0;  // current global iteration (1-based once processing)
   sgw_run_stats stats{};
   bool trace_on = false;
@@ -414,6 +415,8 @@ int read_ctl(sgw_engine *e) {
   CK(cudaStreamSynchronize(e->s_comp));
   e->iters_known = e->h_ctl->iters_total;
   e->stats.inner_iterations = (uint64_t)e->h_ctl->iters_total + e->hub_iters;
+  e->stats.relaxed_edges = e->h_ctl->relaxed_edges;
+  e->stats.relaxed_sources = e->h_ctl->relaxed_sources;
   return check_ctl_error(e);
 }
 
@@ -703,6 +706,7 @@ int launch_generate(sgw_engine *e, int consume, bool plan) {
   e->parts_valid = false;
   e->labels_partial = false;
   e->labels_taken = consume != 0;
+  e->part_done.clear();
   return SGW_OK;
 }
 
@@ -1010,13 +1014,13 @@ int launch_flat(sgw_engine *e, uint32_t b, uint32_t count) {
 
 // A single vertex whose edges exceed one buffer: claim it once, then stream
 // and relax its edges piece by piece (one inner iteration).
-int process_hub(sgw_engine *e, const Part &q, uint32_t b) {
+int process_hub(sgw_engine *e, const Part &q, uint32_t b, bool again = false) {
   const bool async = e->params.mode == SGW_ASYNC;
   const bool pr = e->params.algo == SGW_PR;
   const uint32_t u = q.first_vertex;
   if (pr) k_pr_hub_claim<<<1, 1, 0, e->s_comp>>>(q.from, e->d_qpush, e->d_ctl);
   else k_hub_claim<<<1, 1, 0, e->s_comp>>>(u, e->d_value, e->d_l1, e->d_l2, e->d_ctl,
-                                          !async ? 0 : e->labels_partial ? 1 : 2);
+                                          !async ? 0 : e->labels_partial || again ? 1 : 2);
   CK(cudaGetLastError());
   const uint64_t deg = q.edge_count;
   const uint64_t hoff = np_at(e->g, u);
@@ -1093,10 +1097,14 @@ int poll_wait(sgw_engine *e, uint64_t begun, uint64_t *iter, bool *done) {
 // relaxation and made both slower (RMAT-24 SSSP-async: 12.2 against 17.0
 // GTEPS).  iters_out: iterations that did work, counted on the device.
 // first: no partition of this global iteration has been relaxed before.
-int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool first) {
+// again: this one has been (the step API allows it), so only the sources
+// labelled since then are active.
+int process_resident(sgw_engine *e, const Part &q, uint32_t b, uint32_t *iters_out, bool first,
+                     bool again = false) {
   const bool async = e->params.mode == SGW_ASYNC;
   const bool tiles = (e->opts.flags & SGW_OPT_CTA_TILES) != 0;
-  const bool all = !tiles && !(async && e->labels_partial);  // the first pass relaxes every queued source
+  // the first pass relaxes every queued source
+  const bool all = !tiles && !(async && (e->labels_partial || again));
   size_t slot = 0;
   if (!async) {
     TRY(prof_begin(e, K_RELAX, e->s_comp, &slot));
@@ -1998,11 +2006,14 @@ int sgw_process_partition(sgw_engine *e, uint32_t i, uint32_t *inner_iterations)
   CK(cudaSetDevice(e->device));
   const Part &q = e->h_parts[i];
   uint32_t iters = 1;
+  e->part_done.resize(e->num_parts);
+  const bool again = e->part_done[i] != 0;
+  e->part_done[i] = 1;
   if (is_hub(e, q)) {
-    TRY(process_hub(e, q, 0));
+    TRY(process_hub(e, q, 0, again));
   } else {
     TRY(enqueue_gather(e, i, e->s_comp));
-    TRY(process_resident(e, q, i % e->nbuf, &iters, false));
+    TRY(process_resident(e, q, i % e->nbuf, &iters, false, again));
   }
   CK(cudaStreamSynchronize(e->s_comp));
   TRY(read_ctl(e));
