@@ -2088,7 +2088,7 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_pr_all(
         past = start >= t1;
         uint32_t lo;
         d = unit_clip<kRelaxHeader>(start, p1 - p0, t0, t1, &lo, &head);
-        if (push == 0.0 && !kCache) d = 0;
+        if (a.iter > 1 && push == 0.0) d = 0;  // not claimed
         if (d || (kCache && head)) {
           boff = (kHost ? a.off[a.queue[i]] : a.streamed ? a.off[a.queue[i]] - a.stream_base : p0 - a.edge_from) + lo;
           if (kCache) {
