@@ -419,7 +419,8 @@ def run_ours(a, dist):
     # kernel classes: the gather kernel, the whole-range DMA copies, the
     # relaxation and the generate step (algorithmic bytes per launch)
     esz = transfer_record_bytes(g.n, weighted, a.no_pack)
-    gbytes = sum(s["gather_bytes"] for s in steps)
+    # (sync passes read the host copy themselves: no gather launches, their time in ms_relax)
+    gbytes = sum(s["gather_bytes"] for s in steps if s["gather_launches"])
     sbytes = sum(s["h2d_bytes"] - s["gather_bytes"] for s in steps)
     relax_bytes = sum(s["relaxed_sources"] * 17 + s["relaxed_edges"] * (esz + 4) for s in steps)
     gen_bytes = sum(s["generate_launches"] * 2 * g.n + s["active_vertices"] * 16 for s in steps)
@@ -539,7 +540,7 @@ def run_profile(a, dist):
             "warm": {k: w[k] for k in keys},
             "run": {k: st[k] for k in keys + ("ms_gather", "ms_relax", "ms_generate", "ms_device", "relaxed_edges",
                                               "relaxed_sources", "active_vertices", "gather_bytes", "h2d_bytes")},
-            "algorithmic_bytes": {"gather": st["gather_bytes"],
+            "algorithmic_bytes": {"gather": st["gather_bytes"] if st["gather_launches"] else 0,
                                   "relax": st["relaxed_sources"] * 17 + st["relaxed_edges"] * (esz + 4),
                                   "generate": st["generate_launches"] * 2 * g.n + st["active_vertices"] * 16},
             "record_bytes": esz}

@@ -274,18 +274,23 @@ typedef struct sgw_run_stats {
                                    not the initial one (Graph500 m_reached)     */
   double ms_device;             /* CUDA-event time of the processing loop       */
   double ms_generate;           /* SGW_OPT_PROFILE: per kernel class totals     */
-  double ms_partition;
+  double ms_partition;          /* plans on their own (sgw_partition) and the
+                                   learned policy's range statistics; a plain
+                                   run plans in the generate launches           */
   double ms_gather;             /* the gather kernel (k_gather_v) alone         */
-  double ms_relax;
+  double ms_relax;              /* with the host reads of the passes that make
+                                   them (sync runs)                             */
   uint64_t launches;            /* kernels launched by the run                  */
   uint64_t gather_launches;
   uint64_t relax_launches;
   uint64_t generate_launches;
   uint64_t relaxed_edges;       /* edges expanded by the relaxation kernels     */
   uint64_t relaxed_sources;     /* sources whose edges were expanded            */
-  uint64_t gather_bytes;        /* host bytes the gather kernel read (the same
-                                   count is written to HBM); h2d_bytes minus
-                                   this is what DMA copies moved                */
+  uint64_t gather_bytes;        /* host bytes that kernels read: the gather (the
+                                   same count is written to HBM), or, in sync
+                                   runs with gather_launches 0, the relaxation
+                                   passes themselves; h2d_bytes minus this is
+                                   what DMA copies moved                        */
   double ms_stream;             /* SGW_OPT_PROFILE: DMA copies of whole ranges
                                    and of split-vertex pieces                   */
 } sgw_run_stats;
@@ -348,7 +353,8 @@ typedef struct sgw_trace_rec {
   uint64_t iteration_active_nodes;/* queued vertices of the whole iteration   */
   uint64_t iteration_active_edges;
   uint64_t bytes_h2d;             /* bytes read from host for the partition   */
-  uint32_t transfer;              /* 0 compacted gather, 1 range stream, 2 split vertex */
+  uint32_t transfer;              /* 0 active edges alone (gathered, or read by a
+                                     sync pass itself), 1 range stream, 2 split vertex */
   uint32_t reserved;
 } sgw_trace_rec;
 

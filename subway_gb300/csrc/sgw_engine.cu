@@ -1199,7 +1199,10 @@ int process_from_host(sgw_engine *e, const Part &q) {
   TRY(launch_relax(e, q, 0, 1, false, true, e->cache.have ? kSrcCache : kSrcHost));
   e->iter_base += 1;
   TRY(prof_end(e, e->s_comp, slot));
-  if (!e->cache.have) e->stats.h2d_bytes += q.edge_count * run_rec(e);  // else counted on the device
+  if (!e->cache.have) {  // else counted on the device
+    e->stats.h2d_bytes += q.edge_count * run_rec(e);
+    e->stats.gather_bytes += q.edge_count * run_rec(e);
+  }
   return SGW_OK;
 }
 
@@ -2196,6 +2199,7 @@ int sgw_run(sgw_engine *e, const sgw_run_params *p, void *out_values, sgw_run_st
   e->stats.relaxed_edges = e->h_ctl->relaxed_edges;
   e->stats.relaxed_sources = e->h_ctl->relaxed_sources;
   e->stats.h2d_bytes += e->h_ctl->host_edges * run_rec(e);
+  e->stats.gather_bytes += e->h_ctl->host_edges * run_rec(e);
   e->stats.inner_iterations = (uint64_t)e->h_ctl->iters_total + e->hub_iters;
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, e->ev_t0, e->ev_t1));
