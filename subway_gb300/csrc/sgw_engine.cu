@@ -906,7 +906,8 @@ int launch_relax_pass(sgw_engine *e, const Part &q, uint32_t b, uint32_t iter, u
   }
   const uint32_t g1 = grid_for(e, q.size, kRelaxThreads);
   if (e->opts.flags & SGW_OPT_CTA_TILES) k_relax_tile<ALGO, ASYNC, W><<<g1, kRelaxThreads, 0, e->s_comp>>>(a);
-  else CK(chain(k_relax_warp<ALGO, ASYNC, W>, g1, kRelaxThreads, e->s_comp, a));
+  else if constexpr (ASYNC) CK(chain(k_relax_warp<ALGO, W>, g1, kRelaxThreads, e->s_comp, a));
+  else return fail(SGW_ESTATE, "a sync pass relaxes every queued source");
   CK(cudaGetLastError());
   e->stats.launches += 1;
   e->stats.relax_launches += 1;

@@ -1605,7 +1605,8 @@ __device__ __forceinline__ bool relax_lane(const RelaxArgs &a, const uint32_t (&
   return any;
 }
 
-// Warp-tile form of k_relax_tile: each warp takes 32 partition sources at a
+// Warp-tile form of k_relax_tile for async inner iterations (sync passes take
+// k_relax_all): each warp takes 32 partition sources at a
 // time and expands their edges on its own (warp_expand), so
 // warps never wait on each other: a warp that runs out of tiles adds its counters
 // to the CTA's in shared memory and leaves, and the last warp of the CTA to
@@ -1670,14 +1671,14 @@ __device__ __forceinline__ void warp_publish(CtaTally &t, Ctl *ctl, uint32_t slo
   }
 }
 
-template <int ALGO, bool ASYNC, int W>
+template <int ALGO, int W>
 __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_warp(RelaxArgs a) {
   chain_wait();
   __shared__ CtaTally s_tally;
   __shared__ WarpExpand<uint32_t> s_exp[kWarpsPerCta];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t slot = (a.base + a.iter) & 3u;
-  if (!iter_begin<ASYNC>(a, s_tally)) return;
+  if (!iter_begin<true>(a, s_tally)) return;
   bool any_update = false;
   unsigned long long my_edges = 0, my_srcs = 0;
   const uint32_t ntiles = (a.size + 31u) / 32u;
@@ -1688,12 +1689,8 @@ __global__ void __launch_bounds__(kRelaxThreads, SGW_RELAX_MIN_BLOCKS) k_relax_w
     if (idx < a.size) {
       const uint32_t i = a.from + idx;
       const uint32_t u = a.queue[i];
-      bool act = true;
-      if (ASYNC) {
-        act = a.cur[u] != 0;
-        if (act) a.cur[u] = 0;
-      }
-      if (act) {
+      if (a.cur[u]) {
+        a.cur[u] = 0;
         val = a.value[u];
         if (can_push<ALGO>(val)) {
           const uint32_t p0 = a.ptr[i];
