@@ -509,11 +509,13 @@ def run_ours(a, dist):
 
 # ---- one run for a profiler ------------------------------------------------------------
 def run_profile(a, dist):
-    """What an ncu capture of one run needs: the launch counts of the warm-up
-    run (ncu -s) and of the measured run (ncu -c) per kernel class, and the
-    measured run's algorithmic bytes to compare with the captured DRAM bytes.
-    Per generate step the integer family launches k_generate_count, _scan and
-    _write; per relaxation pass k_relax_warp and k_relax_chunks."""
+    """What an ncu capture of a warm-up and a measured run needs: the launch
+    counts per kernel class and the algorithmic bytes of each, to compare with
+    the captured DRAM bytes.  Async launch counts vary from run to run (the host
+    keeps a few iterations launched ahead), so a capture takes both runs whole.
+    A generate step is k_generate_count and k_generate_write; a first relaxation
+    pass k_relax_all, later ones k_relax_warp and, where a queued row is long,
+    k_relax_chunks."""
     import numpy as np
 
     from subway_gb300 import native as N
@@ -535,14 +537,18 @@ def run_profile(a, dist):
     in_place = e.host_copy_bytes() == 0
     esz = (8 if weighted else 4) if in_place else transfer_record_bytes(g.n, weighted, a.no_pack)
     keys = ("gather_launches", "relax_launches", "generate_launches", "launches")
+
+    def algorithmic(s):
+        return {"gather": s["gather_bytes"] if s["gather_launches"] else 0,
+                "relax": s["relaxed_sources"] * 17 + s["relaxed_edges"] * (esz + 4),
+                "generate": s["generate_launches"] * 2 * g.n + s["active_vertices"] * 16}
+
     return {"profile_run": policy, "engine": a.profile_engine, "records_in_place": in_place,
             "workload": workload_config(a)["workload"],
             "warm": {k: w[k] for k in keys},
             "run": {k: st[k] for k in keys + ("ms_gather", "ms_relax", "ms_generate", "ms_device", "relaxed_edges",
                                               "relaxed_sources", "active_vertices", "gather_bytes", "h2d_bytes")},
-            "algorithmic_bytes": {"gather": st["gather_bytes"] if st["gather_launches"] else 0,
-                                  "relax": st["relaxed_sources"] * 17 + st["relaxed_edges"] * (esz + 4),
-                                  "generate": st["generate_launches"] * 2 * g.n + st["active_vertices"] * 16},
+            "algorithmic_bytes_warm": algorithmic(w), "algorithmic_bytes": algorithmic(st),
             "record_bytes": esz}
 
 
