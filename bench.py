@@ -239,16 +239,16 @@ def probe_link(N, dev):
     return h.value, d.value
 
 
-# DRAM bytes (read + write) per algorithmic byte of each kernel class, from
-# one-kernel-class ncu captures over one measured RMAT-24 / 1 GB run
+# DRAM bytes (read + write) per algorithmic byte of each kernel class, from an
+# ncu capture over two RMAT-24 / 1 GB runs
 # (profiles/dram_per_class_rmat24_sssp_async_1gb.md; ncu empties the caches
 # before each launch, so these are cold-cache figures).  A full-size launch's
 # traffic is the ratio times its algorithmic bytes: an estimate, not a count.
-DRAM_PER_ALGO_BYTE = {"gather": 0.73, "relax": 1.06, "generate": 2.23}
+DRAM_PER_ALGO_BYTE = {"gather": 0.68, "relax": 1.06, "generate": 2.24}
 # Host-link bytes (L2 sectors filled from host memory) per algorithmic byte of
-# the gather, from a one-kernel capture over every gather of one measured
-# RMAT-24 / 1 GB run (profiles/k_gather_v_rmat24_sssp_async_1gb.md).
-LINK_PER_ALGO_BYTE = {"gather": 1.063}
+# the gather, from a one-kernel capture over every gather of two RMAT-24 / 1 GB
+# runs (profiles/k_gather_v_rmat24_sssp_async_1gb.md).
+LINK_PER_ALGO_BYTE = {"gather": 1.060}
 
 
 def run_ours(a, dist):

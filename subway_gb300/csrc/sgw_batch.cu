@@ -759,9 +759,12 @@ constexpr unsigned long long kBarrierWaitNs = 2000000000ull;
 int batch_run(sgw_batch *b, int algo, const uint32_t *sources, uint32_t nsrc, void *out, uint32_t answer_bytes,
               sgw_batch_stats *stats, bool persistent, uint32_t extra_blocks, unsigned long long wait_ns);
 
-// Default form per algorithm, measured on R-MAT 22-26 with 64 queries: the
-// persistent kernel runs SSSP batches 2-9% faster than the graph loop and BFS
-// batches within 4% either way, so SSSP takes it and BFS keeps the graph.
+// Default form per algorithm, measured with 7, 32 and 64 queries on R-MAT 14 to
+// 24.  SSSP, 64 queries, persistent against graph: 1.76 and 1.84 ms on 2^18,
+// 5.55 and 6.15 on 2^20, 22.0 and 25.0 on 2^22, 86.6 and 101 on 2^24; below 2^17
+// the graph is ahead (0.75 and 0.71 ms on 2^16, 0.43 and 0.42 on 2^14).  BFS: 0.29
+// and 0.25 ms on 2^18, 0.59 and 0.44 on 2^20, 7.5 and 5.5 on 2^24, equal on 2^14.
+// So SSSP takes the persistent kernel and BFS the graph.
 bool use_persistent(const sgw_batch *b, int algo) {
   return b->form == 1 || (b->form == 0 && algo == SGW_SSSP);
 }

@@ -143,7 +143,7 @@ struct GenArgs {
   int sel_mode = 0;
   int algo = 0;
   const uint32_t *value = nullptr;
-  // Partition plan, made by the last tile to finish (null: none)
+  // Partition plan, made by the write pass's last CTA (null: none)
   Part *parts = nullptr;
   uint32_t max_parts = 0;
   unsigned long long cap = 0;
@@ -280,7 +280,7 @@ __device__ __forceinline__ void gen_select(const GenArgs &a, uint32_t v0, bool f
 }
 
 // Clears the labels of the lane's vertices in L.clearmask (16-byte stores of
-// the words read by gen_lane when the group is whole).
+// the words that gen_labels read when the group is whole).
 __device__ __forceinline__ void gen_clear(const GenArgs &a, uint32_t v0, bool full, const GenLane &L) {
   if (!L.clearmask) return;
   uint32_t cw[4];
